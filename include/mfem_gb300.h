@@ -83,18 +83,18 @@ enum { MFEM_PRECISION_FP64 = 0, MFEM_PRECISION_MIXED = 1 };
  * with a 9-vector energy only: Stable-Neohookean, Neohookean) ------------ */
 enum { MFEM_FORMULATION_MIXED_STRETCH = 0, MFEM_FORMULATION_STRETCH = 1 };
 
-/* How the PCG runs.  PERSISTENT: one cooperative (co-resident,
- * grid-synchronised) launch per solve; SPLIT: two launches per iteration
- * with a host check for convergence every few iterations (same arithmetic
- * and bitwise the same results as PERSISTENT: Eigen's PCG iteration).
- * FUSED: the single-reduction form of the same PCG (Chronopoulos and Gear,
- * 1989), one launch per iteration; equal to the others in exact arithmetic,
- * not bitwise.  AUTO: the batch picks FUSED when its PCG tiles (256 rows
- * each) fill at least two per SM or fit in a few blocks, SPLIT in between,
- * where the system sits in L2 and FUSED's extra gathers per neighbour set
- * the pace (a 30^3 cube: 117 tiles, SPLIT 20% faster; a 60^3 cube: 873
- * tiles, FUSED faster; a 200-tet beam: one tile, FUSED's single launch per
- * iteration faster). */
+/* How the PCG runs.  PERSISTENT: one cooperative (co-resident) launch per
+ * solve; SPLIT: two launches per iteration (same arithmetic and bitwise the
+ * same results as PERSISTENT: Eigen's PCG iteration).  FUSED: the
+ * single-reduction form of the same PCG (Chronopoulos and Gear, 1989), one
+ * launch per iteration; equal to the others in exact arithmetic, not bitwise.
+ * AUTO: the batch picks the form: FUSED when its PCG tiles (256 rows each)
+ * fill at least two per SM, or are at most four (but not for one FP64 scene),
+ * SPLIT in between.  A batch of PERSISTENT, or of AUTO where it picked SPLIT
+ * or at most four tiles, runs each solve as one launch with the matrix
+ * resident in shared memory if that fits (up to two tiles per SM; FP64 up to
+ * 128 rows per SM), with the results of the picked form's launches, bitwise;
+ * mfem_gpu_batch_step_n runs FUSED batches that way too. */
 enum { MFEM_PCG_KERNEL_PERSISTENT = 0, MFEM_PCG_KERNEL_SPLIT = 1, MFEM_PCG_KERNEL_FUSED = 2,
        MFEM_PCG_KERNEL_AUTO = 3 };
 

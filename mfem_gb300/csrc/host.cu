@@ -30,6 +30,7 @@
 
 #include "../../include/mfem_gb300.h"
 #include "kernels.cuh"
+#include "resident.cuh"
 
 using namespace mfem_gpu;
 
@@ -556,6 +557,15 @@ struct mfem_batch {
   int fem = 0;     // every scene uses the standard-FEM variable
   int jacobi = 1;  // no scene uses the 3x3 block-Jacobi preconditioner
   int coop_grid = 0;  // blocks of the persistent PCG (all co-resident)
+  bool auto_form = false;  // the scenes left the PCG form to the batch
+  // the resident solve (k_resident.cu) of the batch's form, planned on first
+  // use: 0 not planned yet, 1 planned, -1 the batch does not fit
+  int cgr_state = 0;
+  char* cgr_mem = nullptr;
+  CgrArgs cgr_args{};
+  int cgr_blocks = 0, cgr_nthreads = 0;
+  size_t cgr_smem_bytes = 0;
+  bool loop_resident = false;  // the PCG loop graph's body starts with the resident solve
   int pstride = 0;  // tiles per partials quantity
   // instrumentation
   bool profiling = false;
@@ -802,6 +812,7 @@ int sync_counters(mfem_batch* b) {
     b->k_launches[MFEM_K_CG_LOOP] += 1 + bodies;  // k_cg_enter and one k_cg_continue a body
     if (b->loop_fused) {
       b->k_launches[MFEM_K_CGF_ITER] += bodies * b->cg_loop_len;
+      if (b->loop_resident) b->k_launches[MFEM_K_CG_SOLVE] += bodies;
     } else {
       b->k_launches[MFEM_K_CG_SPMV] += bodies * b->cg_loop_len;
       b->k_launches[MFEM_K_CG_UPDATE] += bodies * b->cg_loop_len;
@@ -874,6 +885,156 @@ int worst_status(const SceneScalars& sc) {
   return MFEM_OK;
 }
 
+// ------------------------------------------------- resident PCG plan ---
+// Blocks of the resident solve for the whole batch (resident.cuh).  FP32: a
+// reduction tile of eight slices each (39k tets, 34 tiles: 6.5 us an
+// iteration, against 7.9 / 8.2 / 14.7 us with 4 / 2 / 1 slices, whose halos
+// overlap more and whose exchange has more records).  FP64: as few slices as
+// leave every block an SM of its own, for the multiplication's 64-cycle
+// instructions (5,400 tets: 11.9 / 11.9 / 16.0 us with 1 / 2 / 4).  Above one
+// block an SM, two share it, each with half the shared memory (320k tets, 263
+// tiles: 17.2 us against 26.5 us for the launches).  False: the batch does not
+// fit, or its form has no resident kernel.
+bool cgr_plan(mfem_batch* b) {
+  if (b->cgr_state != 0) return b->cgr_state > 0;
+  b->cgr_state = -1;
+  const bool fused = b->pcg_kernel == MFEM_PCG_KERNEL_FUSED;
+  const bool fp64 = b->fp64 != 0;
+  if (b->minres || (fused && fp64)) return false;
+  int dev = 0, sms = 0, coop = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
+    return false;
+  const int n = (int)b->scenes.size();
+  auto count = [&](int spb) {
+    long c = 0;
+    for (mfem_scene* s : b->scenes) c += ((s->M.nf + 31) / 32 + spb - 1) / spb;
+    return c;
+  };
+  int spb = fp64 ? 1 : kCgrTile;
+  while (fp64 && spb < kCgrMaxSpb64 && count(spb) > sms) spb *= 2;
+  const bool two = count(spb) > sms;
+  if (count(spb) > 2 * sms) return false;
+  const size_t budget = two ? kCgrSmemTwo : kCgrSmemOne;
+  std::vector<CgrBlock> blocks;
+  std::vector<int> h_col;
+  std::vector<uint16_t> lidx;
+  size_t rows = 0, smem = 0;
+  int nrec = 0;
+  for (int i = 0; i < n; ++i) {
+    const HostMesh& M = b->scenes[i]->M;
+    if (M.nf == 0) return false;
+    const int ns = (M.nf + 31) / 32, nblk = (ns + spb - 1) / spb;
+    const bool tile = spb == kCgrTile || nblk == 1;
+    if (!tile && (ns + kCgrTile - 1) / kCgrTile > kCgrMaxSliceTiles) return false;
+    std::vector<int> local(M.nf, -1);
+    for (int k = 0; k < nblk; ++k) {
+      CgrBlock B{};
+      B.scene = i;
+      B.slice0 = k * spb;
+      B.nsl = std::min(spb, ns - B.slice0);
+      B.hoff = (int)h_col.size();
+      B.loff = (int)lidx.size();
+      B.rec0 = nrec;
+      B.nrec = tile ? nblk : ns;
+      B.rec = tile ? k : B.slice0;
+      B.row0 = (int)rows;
+      B.nblk = nblk;
+      B.tile = tile ? 1 : 0;
+      const int r0 = 32 * B.slice0, own = 32 * B.nsl, r1 = std::min(M.nf, r0 + own);
+      // every slot's column as an index into the block's rows, then its halo
+      for (int q = M.slice_off[B.slice0]; q < M.slice_off[B.slice0 + B.nsl]; ++q) {
+        const int c = M.ell_col[q];
+        if (c >= r0 && c < r1) {
+          lidx.push_back((uint16_t)(c - r0));
+          continue;
+        }
+        if (local[c] < 0) {
+          local[c] = (int)h_col.size() - B.hoff;
+          h_col.push_back(c);
+        }
+        lidx.push_back((uint16_t)std::min(own + local[c], 65535));
+      }
+      B.nh = (int)h_col.size() - B.hoff;
+      for (int j = B.hoff; j < (int)h_col.size(); ++j) local[h_col[j]] = -1;
+      if (own + B.nh > 65535) return false;
+      // the slots that fit, the same number for each slice
+      auto slots = [&](int kres) {
+        size_t t = 0;
+        for (int s = B.slice0; s < B.slice0 + B.nsl; ++s)
+          t += std::min(kres, (M.slice_off[s + 1] - M.slice_off[s]) / 32);
+        return t;
+      };
+      int kres = kMaxRowBlocks + 1;
+      while (kres >= 0 && cgr_smem(fp64, fused, b->jacobi, slots(kres), own, B.nh) > budget) --kres;
+      if (kres < 0) return false;
+      B.kres = kres;
+      smem = std::max(smem, cgr_smem(fp64, fused, b->jacobi, slots(kres), own, B.nh));
+      blocks.push_back(B);
+    }
+    nrec += tile ? nblk : ns;
+    rows += M.nf;
+  }
+  // blocks that can have an SM each are kept from sharing one
+  if (!two) smem = std::max(smem, kCgrSmemTwo + 8 * 1024);
+  const int threads = cgr_threads(fp64, spb);
+  if ((long)cgr_blocks_per_sm(fp64, fused, b->jacobi, threads, smem) * sms < (long)blocks.size()) return false;
+  const size_t pub = rows * (fp64 ? 3 : 1);
+  CgrArgs& a = b->cgr_args;
+  auto lay = [&](Arena& A) {
+    a.blocks = A.take<CgrBlock>(blocks.size());
+    a.h_col = A.take<int>(std::max<size_t>(h_col.size(), 1));
+    a.lidx = A.take<uint16_t>(std::max<size_t>(lidx.size(), 1));
+    a.recs = A.take<uint4>(6 * (size_t)nrec);
+    a.pub = A.take<uint4>(2 * pub);
+    a.seq = A.take<unsigned int>(n);
+  };
+  Arena dry;
+  lay(dry);
+  if (cudaMalloc(&b->cgr_mem, dry.used) != cudaSuccess) {
+    cudaGetLastError();
+    b->cgr_mem = nullptr;
+    return false;
+  }
+  Arena real;
+  real.base = b->cgr_mem;
+  lay(real);
+  a.nrec_total = nrec;
+  a.pub_stride = pub;
+  a.sds = b->d_sds;
+  a.ctrs = b->d_ctr;
+  a.max_iters = 1 << 30;
+  const std::vector<unsigned int> seq(n, 1u);  // records start with tag 0
+  auto up = [&](const void* dst, const void* src, size_t bytes) {
+    return bytes == 0 || cudaMemcpyAsync(const_cast<void*>(dst), src, bytes, cudaMemcpyHostToDevice, b->stream) == cudaSuccess;
+  };
+  const bool ok = cudaMemsetAsync(b->cgr_mem, 0, dry.used, b->stream) == cudaSuccess &&
+                  up(a.blocks, blocks.data(), sizeof(CgrBlock) * blocks.size()) &&
+                  up(a.h_col, h_col.data(), sizeof(int) * h_col.size()) &&
+                  up(a.lidx, lidx.data(), sizeof(uint16_t) * lidx.size()) &&
+                  up(a.seq, seq.data(), sizeof(unsigned int) * n) &&
+                  cudaStreamSynchronize(b->stream) == cudaSuccess;
+  if (!ok) {
+    cudaGetLastError();
+    cudaFree(b->cgr_mem);
+    b->cgr_mem = nullptr;
+    return false;
+  }
+  b->cgr_blocks = (int)blocks.size();
+  b->cgr_nthreads = threads;
+  b->cgr_smem_bytes = smem;
+  b->cgr_state = 1;
+  return true;
+}
+
+cudaError_t cgr_launch(mfem_batch* b, int max_iters) {
+  CgrArgs a = b->cgr_args;
+  a.max_iters = max_iters;
+  return launch_cgr(a, b->fp64 != 0, b->pcg_kernel == MFEM_PCG_KERNEL_FUSED, b->jacobi != 0, b->cgr_blocks,
+                    b->cgr_nthreads, b->cgr_smem_bytes, b->stream);
+}
+
 // PCG iterations after k_cg_init: one cooperative launch for the whole solve,
 // or SpMV/update launch pairs in chunks with a host check of the active
 // count after each chunk.
@@ -912,8 +1073,11 @@ int capture_cg_graph(mfem_batch* b, const Launch& Lcg, bool fused, cudaGraphExec
 // capture_cg_graph) followed by k_cg_continue, which sets it again from the
 // batch's counters.  A solve ends within one chunk of its last iteration,
 // with no host round trip.
-int capture_cg_loop(mfem_batch* b, const Launch& Lcg, bool fused, cudaGraphExec_t* out) {
-  const int len = fused ? 8 : kCgReplace;
+// resident: the body is the resident solve, which ends when a stop of the
+// recursion is to be verified, and the three launches of k_cgf_iter that
+// verify it.
+int capture_cg_loop(mfem_batch* b, const Launch& Lcg, bool fused, bool resident, cudaGraphExec_t* out) {
+  const int len = resident ? 3 : fused ? 8 : kCgReplace;
   const int max_launch = b->max_cg + (fused && !b->fp64 ? 9 : 0);
   const int max_bodies = (max_launch + len - 1) / len + 1;
   cudaGraph_t g = nullptr;
@@ -950,6 +1114,8 @@ int capture_cg_loop(mfem_batch* b, const Launch& Lcg, bool fused, cudaGraphExec_
   if ((e = cudaStreamBeginCaptureToGraph(b->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
       cudaSuccess)
     return fail(e);
+  cudaError_t er = cudaSuccess;
+  if (resident) er = cgr_launch(b, 1 << 30);
   for (int k = 0; k < len; ++k) {
     if (fused) {
       launch_cgf_iter(Lcg, b->cgf_shape);
@@ -962,19 +1128,27 @@ int capture_cg_loop(mfem_batch* b, const Launch& Lcg, bool fused, cudaGraphExec_
   launch_cg_continue(Lcg, h, max_bodies);
   cudaGraph_t cap = body;
   e = cudaStreamEndCapture(b->stream, &cap);
+  if (e == cudaSuccess) e = er;
   if (e != cudaSuccess) return fail(e);
   e = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   CUDA_OR(e, MFEM_ERR_CUDA);
   b->cg_loop_len = len;
   b->loop_fused = fused;
+  b->loop_resident = resident;
   return MFEM_OK;
 }
 
 int run_pcg_graph(mfem_batch* b, const Launch& Lcg, bool fused) {
   const int len = fused ? 8 : kCgReplace;
   if (b->cg_loop_on && !b->cg_loop) {
-    if (capture_cg_loop(b, Lcg, fused, &b->cg_loop) != MFEM_OK) {
+    const bool resident = fused && b->auto_form && cgr_plan(b);
+    int rc = capture_cg_loop(b, Lcg, fused, resident, &b->cg_loop);
+    if (rc != MFEM_OK && resident) {
+      cudaGetLastError();
+      rc = capture_cg_loop(b, Lcg, fused, false, &b->cg_loop);
+    }
+    if (rc != MFEM_OK) {
       // conditional nodes unavailable: chunks with host checks instead
       cudaGetLastError();
       b->cg_loop = nullptr;
@@ -1033,6 +1207,17 @@ int run_pcg(mfem_batch* b, const Launch& Lcg) {
     } else {
       launch_cg_init(Lcg);
     }
+  }
+  // the whole solve in one launch where the batch fits.  With profiling on,
+  // a batch that chose its form itself runs that form's launches instead
+  // (the same results), so that every kernel carries its own event pair.
+  if ((b->pcg_kernel == MFEM_PCG_KERNEL_PERSISTENT ||
+       (b->pcg_kernel == MFEM_PCG_KERNEL_SPLIT && b->auto_form && !b->profiling)) &&
+      cgr_plan(b)) {
+    cudaError_t e;
+    { KTimer t(b, MFEM_K_CG_SOLVE); e = cgr_launch(b, 1 << 30); }
+    CUDA_OR(e, MFEM_ERR_CUDA);
+    return MFEM_OK;
   }
   if (b->pcg_kernel == MFEM_PCG_KERNEL_PERSISTENT) {
     cudaError_t e;
@@ -1203,6 +1388,9 @@ int batch_step_impl(mfem_batch* b, mfem_step_stats* stats) {
 
 int upload_sds(mfem_batch* b);
 
+// PCG iterations of one tick when they run as one resident launch.
+constexpr int kTickResident = 64;
+
 // One tick of the ticked multi-step form as a CUDA graph over the current
 // tables: every kernel of a Newton iteration once, each acting on the
 // scenes in its phase, with tick_pcg PCG iterations and one line-search
@@ -1216,17 +1404,21 @@ int capture_tick_graph(mfem_batch* b, cudaGraphExec_t* out) {
   Lls.variant = b->var_ls;
   const Launch Lcg = make_launch(b, TB_CG);
   cudaGraph_t g = nullptr;
+  const bool resident = cgr_plan(b);
+  cudaError_t er = cudaSuccess;
   CUDA_OR(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), MFEM_ERR_CUDA);
   launch_elem_update(Lel, nullptr);
   launch_assemble(make_launch(b, TB_ROW));
   launch_cgf_scale(Lcg);
   launch_cgf_init(Lcg);
-  for (int k = 0; k < b->tick_pcg; ++k) launch_cgf_iter(Lcg, b->cgf_shape);
+  if (resident) er = cgr_launch(b, kTickResident);
+  for (int k = 0; k < (resident ? 3 : b->tick_pcg); ++k) launch_cgf_iter(Lcg, b->cgf_shape);
   launch_local_solve(Llo);
   launch_ls_energy(Lls);
   launch_apply(Lev);
   launch_step_turn(Lev);
-  const cudaError_t ec = cudaStreamEndCapture(b->stream, &g);
+  cudaError_t ec = cudaStreamEndCapture(b->stream, &g);
+  if (ec == cudaSuccess) ec = er;
   if (ec != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
     CUDA_OR(ec, MFEM_ERR_CUDA);
@@ -1735,6 +1927,8 @@ int batch_autotune(mfem_batch* b) {
   std::vector<SceneDev> tsd = b->h_sds;
   for (SceneDev& d : tsd) {
     d.cg_tol = 0.0;
+    d.cg_tolx = make_float2(0.f, 0.f);
+    d.cg_itolx = make_float2(0.f, 0.f);
     d.max_cg = 1 << 30;
   }
   CUDA_OR(cudaMemcpyAsync(b->d_sds, tsd.data(), sizeof(SceneDev) * n, cudaMemcpyHostToDevice, b->stream),
@@ -1897,9 +2091,11 @@ int batch_build(mfem_scene* const* scenes, int n, mfem_batch** out) {
     CUDA_OR(cudaGetDevice(&dev), MFEM_ERR_CUDA);
     CUDA_OR(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), MFEM_ERR_CUDA);
   }
+  b->auto_form = b->pcg_kernel == MFEM_PCG_KERNEL_AUTO;
   if (b->pcg_kernel == MFEM_PCG_KERNEL_AUTO)
-    b->pcg_kernel = (b->ntiles[TB_CG] >= 2 * sms || b->ntiles[TB_CG] <= 4) ? MFEM_PCG_KERNEL_FUSED
-                                                                          : MFEM_PCG_KERNEL_SPLIT;
+    b->pcg_kernel = (b->ntiles[TB_CG] >= 2 * sms || (b->ntiles[TB_CG] <= 4 && !(b->fp64 && n == 1)))
+                        ? MFEM_PCG_KERNEL_FUSED
+                        : MFEM_PCG_KERNEL_SPLIT;
   if (b->pcg_kernel == MFEM_PCG_KERNEL_PERSISTENT) {
     const int per_sm = cg_solve_blocks_per_sm(b->fp64);
     if (per_sm <= 0) return MFEM_ERR_CUDA;
@@ -1963,6 +2159,7 @@ void batch_free(mfem_batch* b) {
   if (!b) return;
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->dmem) cudaFree(b->dmem);
+  if (b->cgr_mem) cudaFree(b->cgr_mem);
   if (b->h_ctr) cudaFreeHost(b->h_ctr);
   if (b->h_ctr_pipe) cudaFreeHost(b->h_ctr_pipe);
   if (b->cg_graph) cudaGraphExecDestroy(b->cg_graph);
@@ -2013,6 +2210,9 @@ int scene_init_device(mfem_scene* s) {
   D.newton_tol = s->cfg.newton_tol;
   D.res_tol = s->cfg.newton_residual_tolerance;
   D.cg_tol = s->cfg.iterative_solver_tolerance;
+  D.cg_tolx = split_df(D.cg_tol);
+  // (below FP32's range the tolerance counts as 0: the solve never meets it)
+  D.cg_itolx = D.cg_tol > 1e-37 ? split_df(1.0 / D.cg_tol) : make_float2(0.f, 0.f);
   D.max_newton = s->cfg.max_newton_iterations;
   D.max_ls = s->cfg.max_linesearch_iterations;
   D.max_cg = s->cfg.max_iterative_solver_iters;

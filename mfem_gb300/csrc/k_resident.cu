@@ -1,0 +1,989 @@
+// PCG solves in one launch with the matrix resident in shared memory.
+//
+// A system of up to some ten thousand block rows has a matrix of at most
+// 34 MB: it fits the SMs' shared memory together, or at worst the L2, and an
+// iteration moves almost nothing.  What one launch per half iteration
+// (k_cg_spmv, k_cg_update) or per iteration (k_cgf_iter) then costs is the
+// chain of latencies: launch boundaries, a row's slots walked one after
+// another (column -> gather -> FMA), tile tickets, a serial finalizer.  Here
+// each block owns up to eight 32-row slices for the whole solve and
+//   * copies its slices' blocks to shared memory once, as nine planes of 32
+//     lanes per slot, and keeps its rows' vectors in registers;
+//   * knows its halo, the distinct columns outside its rows (built by the
+//     host), and once per iteration fetches one vector at them, all columns
+//     in flight together, updates its copy of the multiplied vector with the
+//     owner's own operations, and multiplies out of shared memory;
+//   * exchanges data through L2 without fences, flags or atomics: a row's
+//     vector and a block's partial sums are 16-byte records whose last word
+//     is the exchange's sequence number, written and read as single 128-bit
+//     accesses, so a reader polls the record itself.  Every block sums all
+//     partials in the same fixed order and takes the same decisions.
+// The arithmetic, the order of every sum included, is that of the launches
+// it replaces (pcg.cuh), so the results are bitwise the same.
+//
+// A record is overwritten only after everybody has read it: partials and the
+// single-reduction form's vector alternate between two buffers by the
+// exchange's parity, and a block writes exchange k + 2 only after it has read
+// k + 1 from every block, which each wrote after reading k; the two-reduction
+// form's vector has a second exchange between its reading and its writing.
+// Sequence numbers go on from launch to launch (CgrArgs::seq).
+//
+// Every wait is bounded: after kCgrTimeoutNs the block raises ctrs->error and
+// leaves, as do the others when they see the flag or time out themselves; the
+// host reports MFEM_ERR_TIMEOUT.  The launch is cooperative: all blocks are
+// co-resident, the exchange needs them all.
+#include "pcg.cuh"
+#include "resident.cuh"
+
+namespace mfem_gpu {
+
+namespace {
+
+constexpr unsigned long long kCgrTimeoutNs = 2000000000ull;
+constexpr unsigned int kCgrMaxPolls = 1u << 24;
+
+__device__ __forceinline__ uint4 ld_rec(const uint4* p) {
+  unsigned long long a, b;
+  asm volatile(
+      "{\n\t.reg .b128 q;\n\t"
+      "ld.relaxed.gpu.global.b128 q, [%2];\n\t"
+      "mov.b128 {%0, %1}, q;\n\t}"
+      : "=l"(a), "=l"(b)
+      : "l"(p)
+      : "memory");
+  return make_uint4((unsigned)a, (unsigned)(a >> 32), (unsigned)b, (unsigned)(b >> 32));
+}
+__device__ __forceinline__ void st_rec(uint4* p, uint4 v) {
+  const unsigned long long a = (unsigned long long)v.x | ((unsigned long long)v.y << 32);
+  const unsigned long long b = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
+  asm volatile(
+      "{\n\t.reg .b128 q;\n\t"
+      "mov.b128 q, {%1, %2};\n\t"
+      "st.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p),
+      "l"(a), "l"(b)
+      : "memory");
+}
+__device__ __forceinline__ uint4 rec_of(df64 v, unsigned tag) {
+  return make_uint4(__float_as_uint(v.hi), __float_as_uint(v.lo), 0u, tag);
+}
+__device__ __forceinline__ uint4 rec_of(double v, unsigned tag) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return make_uint4((unsigned)b, (unsigned)(b >> 32), 0u, tag);
+}
+template <typename E> __device__ __forceinline__ E rec_val(uint4 v);
+template <> __device__ __forceinline__ df64 rec_val<df64>(uint4 v) {
+  return df64(__uint_as_float(v.x), __uint_as_float(v.y));
+}
+template <> __device__ __forceinline__ double rec_val<double>(uint4 v) {
+  return __longlong_as_double((long long)((unsigned long long)v.x | ((unsigned long long)v.y << 32)));
+}
+
+__device__ __forceinline__ unsigned long long cgr_now() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Whether a wait of the calling warp has run out, or another block has raised
+// the error flag; every 64th poll (n counts them, t0 is set on the first
+// call).  Warp-uniform.
+__device__ __noinline__ bool wait_over(unsigned n, unsigned long long* t0, BatchCounters* ctrs) {
+  const unsigned long long now = cgr_now();
+  if (*t0 == 0) *t0 = now;
+  bool over = *(volatile int*)&ctrs->error != 0;
+  if (now - *t0 > kCgrTimeoutNs || n > kCgrMaxPolls) {
+    atomicExch(&ctrs->error, 1);
+    over = true;
+  }
+  return __any_sync(0xffffffffu, over);
+}
+
+// Loads N records a lane and polls until all of them carry the tag, the whole
+// warp in step (a lane that stopped polling early would leave the warp
+// diverged for the shuffles that follow).  want: the records the lane needs;
+// the others' values are not looked at.  False: the wait ran out.
+template <int N, typename Ptr>
+__device__ __forceinline__ bool poll_recs(uint4 (&v)[N], const Ptr& at, const bool (&want)[N], unsigned tag,
+                                          BatchCounters* ctrs) {
+  unsigned long long t0 = 0;
+#pragma unroll 1
+  for (unsigned n = 1;; ++n) {
+    bool good = true;
+#pragma unroll
+    for (int q = 0; q < N; ++q) good = good && (!want[q] || v[q].w == tag);
+    if (__all_sync(0xffffffffu, good)) return true;
+    if ((n & 63u) == 0 && wait_over(n, &t0, ctrs)) return false;
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+      if (want[q]) v[q] = ld_rec(at(q));
+  }
+}
+
+__device__ __forceinline__ df64 shfl_to(df64 v, int lane) {
+  return df64(__shfl_sync(0xffffffffu, v.hi, lane), __shfl_sync(0xffffffffu, v.lo, lane));
+}
+__device__ __forceinline__ double shfl_to(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
+template <typename E, int NQ, int kFrom>
+__device__ __forceinline__ void tree(E (&v)[NQ]) {
+#pragma unroll
+  for (int off = kFrom; off > 0; off >>= 1)
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) v[q] = radd(v[q], shfl_down(v[q], off));
+}
+
+struct CgrShared {
+  double part[2][3][kCgrMaxSlices];      // the block's slice sums
+  double tp[2][3][kCgrMaxSliceTiles];    // tile sums (slice records)
+  double red[2][3][8];                   // warp sums of the tiles
+};
+
+// Sums over the scene's rows, the same in every thread of every block.  v
+// holds each lane's values in the lead warps (one per slice, `sl` its number
+// in the block); the order is that of tile_partials and scene_sums: a tree
+// over a slice's 32 rows, a tree over the 8 slices of a tile, each thread over
+// tiles i, i + 256, .., a tree over 32 such sums, a tree over 8.  (Their
+// trees over absent entries only add zeros.)  A block of eight slices sends
+// its tile's sum, a smaller one its slices' sums, a scene of one block
+// nothing.  `ahead` runs once the other blocks' sums have come in, before the
+// last of the adding: loads issued there are under way meanwhile.  False: a
+// wait ran out.
+template <typename E, int NQ, typename F>
+__device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B, CgrShared& S, bool lead, int sl,
+                                            unsigned seq, E (&v)[NQ], const F& ahead) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int par = seq & 1;
+  const bool tiles = B.tile != 0;
+  uint4* rec = A.recs + (size_t)(par * 3) * A.nrec_total + B.rec0;
+  if (lead) tree<E, NQ, 16>(v);
+  if (tiles) {
+    if (lead && lane == 0)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.part[par][q][sl], v[q]);
+    __syncthreads();
+    if (B.nblk == 1) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[q] = lane < B.nsl ? Slot<E>::sget(&S.part[par][q][lane]) : E(0);
+      tree<E, NQ, 4>(v);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[q] = shfl_to(v[q], 0);
+      ahead();
+      return true;
+    }
+    if (warp < NQ) {
+      E a[1] = {lane < B.nsl ? Slot<E>::sget(&S.part[par][warp][lane]) : E(0)};
+      tree<E, 1, 4>(a);
+      if (lane == 0) st_rec(rec + (size_t)warp * A.nrec_total + B.rec, rec_of(a[0], seq));
+    }
+  } else if (lead && lane == 0) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) st_rec(rec + (size_t)q * A.nrec_total + B.rec + sl, rec_of(v[q], seq));
+  }
+  const int n = B.nrec;
+  // the sums of record i (0 for lanes without one), the warp in step
+  auto fetch = [&](int i, E (&a)[NQ]) -> bool {
+    uint4 w[NQ];
+    bool want[NQ];
+    const uint4* src = rec + min(i, n - 1);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      want[q] = i < n;
+      w[q] = ld_rec(src + (size_t)q * A.nrec_total);
+    }
+    const bool ok = poll_recs<NQ>(w, [&](int q) { return src + (size_t)q * A.nrec_total; }, want, seq, A.ctrs);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) a[q] = i < n ? rec_val<E>(w[q]) : E(0);
+    return ok;
+  };
+  if (n <= 32) {
+    // every warp for itself, no block barrier
+    E a[NQ];
+    if (!fetch(lane, a)) return false;
+    ahead();
+    if (tiles) {
+      tree<E, NQ, 16>(a);
+    } else {
+      tree<E, NQ, 4>(a);  // tiles' sums in lanes 0, 8, 16, 24
+#pragma unroll
+      for (int off = 16; off >= 8; off >>= 1)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) a[q] = radd(a[q], shfl_down(a[q], off));
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) v[q] = shfl_to(a[q], 0);
+    return true;
+  }
+  E s[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) s[q] = E(0);
+  int nt = n;
+  if (!tiles) {
+    nt = (n + kCgrTile - 1) / kCgrTile;
+    for (int i0 = 32 * warp; i0 < n; i0 += (int)blockDim.x) {
+      const int i = i0 + lane;
+      E a[NQ];
+      if (!fetch(i, a)) return false;
+      tree<E, NQ, 4>(a);
+      if ((lane & 7) == 0 && i < n)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.tp[par][q][i >> 3], a[q]);
+    }
+    __syncthreads();
+    ahead();
+    if (nt <= 32) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) s[q] = lane < nt ? Slot<E>::sget(&S.tp[par][q][lane]) : E(0);
+      tree<E, NQ, 16>(s);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[q] = shfl_to(s[q], 0);
+      return true;
+    }
+    if (warp < 8)
+      for (int i = threadIdx.x; i < nt; i += 256)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) s[q] = radd(s[q], Slot<E>::sget(&S.tp[par][q][i]));
+  } else if (warp < 8) {
+    for (int i0 = 32 * warp; i0 < n; i0 += 256) {
+      E a[NQ];
+      if (!fetch(i0 + lane, a)) return false;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) s[q] = radd(s[q], a[q]);
+    }
+  }
+  if (warp < 8) {
+    tree<E, NQ, 16>(s);
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.red[par][q][warp], s[q]);
+  }
+  __syncthreads();
+  if (tiles) ahead();
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) v[q] = lane < 8 ? Slot<E>::sget(&S.red[par][q][lane]) : E(0);
+  tree<E, NQ, 4>(v);
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) v[q] = shfl_to(v[q], 0);
+  return true;
+}
+
+// The block's slices in shared memory: nine planes (row-major 3x3 entries) of
+// 32 lanes per resident slot, and each slot's local column indices.
+template <typename Real> struct CgrMatrix {
+  const Real* mat;       // this warp's slice: + 288 k + 32 e + lane
+  const uint16_t* li;    // + 32 k + lane
+  int res, len;          // resident and all slots of the slice
+  const Real* gell;      // the slice in the packed global layout (pairs from 5 soff)
+  const uint16_t* gli;
+  int soff;
+};
+
+template <typename Real>
+__device__ __forceinline__ CgrMatrix<Real> cgr_load_matrix(const CgrArgs& A, const CgrBlock& B, const SceneDev& sd,
+                                                           int sl, unsigned char* smem, unsigned char** rest) {
+  using P = typename std::conditional<sizeof(Real) == 4, float2, double2>::type;
+  const int soff0 = sd.slice_off[B.slice0];
+  int slots = 0;
+  for (int s = 0; s < B.nsl; ++s)
+    slots += min(B.kres, (sd.slice_off[B.slice0 + s + 1] - sd.slice_off[B.slice0 + s]) >> 5);
+  Real* mat = reinterpret_cast<Real*>(smem);
+  uint16_t* li = reinterpret_cast<uint16_t*>(mat + (size_t)slots * 288);
+  *rest = reinterpret_cast<unsigned char*>(li + (size_t)slots * 32);
+  CgrMatrix<Real> M{};
+  int at = 0;
+  for (int s = 0; s < B.nsl; ++s) {
+    const int soff = sd.slice_off[B.slice0 + s], len = (sd.slice_off[B.slice0 + s + 1] - soff) >> 5;
+    const int res = min(B.kres, len);
+    const P* src = static_cast<const P*>(sd.ell) + 5 * (size_t)soff;
+    Real* dst = mat + (size_t)at * 288;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < res * 160; i += blockDim.x) {
+      const P v = src[i];
+      const int k = i / 160, w = (i - 160 * k) >> 5, l = i & 31;
+      Real* d = dst + 288 * k + l;
+      if (w == 0) {
+        d[0] = v.y;
+      } else {
+        d[32 * (2 * w - 1)] = v.x;
+        d[32 * (2 * w)] = v.y;
+      }
+    }
+    const uint16_t* gl = A.lidx + B.loff + (soff - soff0);
+    for (int i = threadIdx.x; i < res * 32; i += blockDim.x) li[32 * at + i] = gl[i];
+    if (s == sl) {
+      M.mat = dst;
+      M.li = li + 32 * at;
+      M.res = res;
+      M.len = len;
+      M.gell = static_cast<const Real*>(sd.ell);
+      M.gli = gl;
+      M.soff = soff;
+    }
+    at += res;
+  }
+  return M;
+}
+
+// acc += (row of A) u, slots in order; u: float4 per local index.
+__device__ __forceinline__ void cgr_multiply(const CgrMatrix<float>& M, const float4* u, float (&acc)[3]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 4
+  for (int k = 0; k < M.res; ++k) {
+    const float4 p = u[M.li[32 * k + lane]];
+    const float* m = M.mat + 288 * k + lane;
+    acc[0] = fma(m[64], p.z, fma(m[32], p.y, fma(m[0], p.x, acc[0])));
+    acc[1] = fma(m[160], p.z, fma(m[128], p.y, fma(m[96], p.x, acc[1])));
+    acc[2] = fma(m[256], p.z, fma(m[224], p.y, fma(m[192], p.x, acc[2])));
+  }
+#pragma unroll 2
+  for (int k = M.res; k < M.len; ++k) {
+    const size_t q = ell_pair(M.soff, k, lane, 0);
+    const float2 w0 = ld_pair<false>(M.gell, q), w1 = ld_pair<false>(M.gell, q + 32),
+                 w2 = ld_pair<false>(M.gell, q + 64), w3 = ld_pair<false>(M.gell, q + 96),
+                 w4 = ld_pair<false>(M.gell, q + 128);
+    const float4 p4 = u[M.gli[32 * k + lane]];
+    const float p[3] = {p4.x, p4.y, p4.z};
+    ell_block_fma(w0, w1, w2, w3, w4, p, acc[0], acc[1], acc[2]);
+  }
+}
+// One component of the row in FP64 (three warps a slice: the FP64 pipe issues
+// a warp instruction every 64 cycles, so a row's 9 products a slot in one
+// thread are the iteration's longest chain); u: three doubles per local index.
+__device__ __forceinline__ void cgr_multiply(const CgrMatrix<double>& M, const double* u, int comp, double& acc) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 4
+  for (int k = 0; k < M.res; ++k) {
+    const double* p = u + 3 * (int)M.li[32 * k + lane];
+    const double* m = M.mat + 288 * k + 96 * comp + lane;
+    acc = fma(m[64], p[2], fma(m[32], p[1], fma(m[0], p[0], acc)));
+  }
+  for (int k = M.res; k < M.len; ++k) {
+    const double* p = u + 3 * (int)M.gli[32 * k + lane];
+    const double a0 = M.gell[ell_entry(M.soff, k, lane, 3 * comp)],
+                 a1 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 1)],
+                 a2 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 2)];
+    acc = fma(a2, p[2], fma(a1, p[1], fma(a0, p[0], acc)));
+  }
+}
+
+// A solve that ended on a wait that ran out: later launches use other tags.
+__device__ __forceinline__ void cgr_abort(const CgrArgs& A, const CgrBlock& B) {
+  if ((threadIdx.x & 31) == 0) atomicAdd(A.seq + B.scene, 0x100000u);
+}
+
+constexpr int kHaloRegs = 4;  // halo columns a thread keeps in registers
+
+// ------------------------------------------------ two-reduction form ---
+// Eigen's iteration, as k_cg_spmv, k_cg_update and k_cg_replace run it:
+//   p = z + beta p;  Ap;  (p, Ap) -> alpha;  x += alpha p;  r -= alpha Ap;
+//   z = D^-1 r;  (r, r), (r, z) -> the stopping test and beta;
+// the exchanged vector is z, and each block keeps p at its halo.  In FP64 a
+// row is three threads' (one component each), and the lead thread (component
+// 0) forms the row's share of the inner products in component order.
+template <typename Real, int kThreads, int kMinBlocks>
+__global__ void __launch_bounds__(kThreads, kMinBlocks) k_cgr_split(const CgrArgs A) {
+  using E = typename Ext<Real>::T;
+  constexpr bool k64 = sizeof(Real) == 8;
+  constexpr int NC = k64 ? 1 : 3;
+  extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
+  __shared__ CgrShared S;
+  const CgrBlock B = A.blocks[blockIdx.x];
+  const SceneDev& sd = A.sds[B.scene];
+  SceneScalars* sc = sd.sc;
+  if (!sc->cg_active) return;
+  unsigned seq = __ldcg(A.seq + B.scene);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int sl = k64 ? warp / 3 : warp, comp = k64 ? warp % 3 : 0;
+  const bool roww = sl < B.nsl, lead = roww && comp == 0;
+  const int row = 32 * (B.slice0 + sl) + lane;
+  const bool live = roww && row < sd.nf;
+  const int own = 32 * B.nsl, mine = 32 * sl + lane;
+  unsigned char* rest;
+  const CgrMatrix<Real> M = cgr_load_matrix<Real>(A, B, sd, sl, cgr_smem_raw, &rest);
+  Real* vec = reinterpret_cast<Real*>(rest);                    // FP32: 4 per entry, FP64: 3
+  double* ex = reinterpret_cast<double*>(vec + 3 * (size_t)(own + B.nh));  // FP64: r, z of the rows
+  (void)ex;
+  // the first halo columns of each thread, and their records under way
+  int hc[kHaloRegs];
+  bool hw[kHaloRegs];
+  uint4 hv[kHaloRegs];
+#pragma unroll
+  for (int j = 0; j < kHaloRegs; ++j) {
+    const int h = threadIdx.x + j * kThreads;
+    hw[j] = h < B.nh;
+    hc[j] = hw[j] ? A.h_col[B.hoff + h] : 0;
+    if (!k64 && hw[j])
+      hv[j] = *reinterpret_cast<const uint4*>(static_cast<const float*>(sd.cg_z) + 4 * (size_t)hc[j]);
+  }
+  auto halo_ahead = [&]() {
+    if constexpr (!k64) {
+#pragma unroll
+      for (int j = 0; j < kHaloRegs; ++j)
+        if (hw[j]) hv[j] = ld_rec(A.pub + B.row0 + hc[j]);
+    }
+  };
+  auto nothing = []() {};
+
+  const size_t k4 = 4 * (size_t)row;
+  Real r[NC], z[NC], p[NC], x[NC], acc[NC], dv[k64 ? 3 : 9];
+  X3 xe = zero_x3();
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    r[c] = live ? static_cast<const Real*>(sd.cg_r)[k4 + comp + c] : Real(0);
+    z[c] = live ? static_cast<const Real*>(sd.cg_z)[k4 + comp + c] : Real(0);
+    p[c] = x[c] = acc[c] = Real(0);
+  }
+  if constexpr (k64) {
+    // the component's row of the preconditioner
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      dv[c] = !live ? 0.0
+                    : sd.block_jacobi ? static_cast<const double*>(sd.dinv)[9 * (size_t)row + 3 * comp + c]
+                                      : (c == 0 ? static_cast<const double*>(sd.dinv)[k4 + comp] : 0.0);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 9; ++c)
+      dv[c] = !live ? 0.f
+                    : sd.block_jacobi ? static_cast<const float*>(sd.dinv)[9 * (size_t)row + c]
+                                      : (c < 3 ? static_cast<const float*>(sd.dinv)[k4 + c] : 0.f);
+  }
+  const bool block_jacobi = sd.block_jacobi != 0;
+  // apply_prec with the row's entries in registers
+  auto precond = [&](const float (&rv)[3], float (&zv)[3]) {
+    if constexpr (!k64) {
+      if (block_jacobi) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) zv[c] = fma(dv[3 * c + 2], rv[2], fma(dv[3 * c + 1], rv[1], dv[3 * c] * rv[0]));
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) zv[c] = dv[c] * rv[c];
+      }
+    }
+  };
+  E rz = sc_get<E>(&sc->rz), rz_prev = rz;
+  const E rr0 = sc_get<E>(&sc->cg_rhs_norm2);
+  E rr = rr0;
+  Real beta = Real(0);
+  E alphaE = E(0), betaE = E(0);
+  int it = 0, status = 0, cg_status = 0;
+  unsigned ztag = 0;
+
+  auto publish_z = [&](unsigned tag) {
+    if (!live || B.nblk == 1) return;
+    if constexpr (k64) {
+      st_rec(A.pub + 3 * (size_t)(B.row0 + row) + comp, rec_of(z[0], tag));
+    } else {
+      st_rec(A.pub + B.row0 + row,
+             make_uint4(__float_as_uint(z[0]), __float_as_uint(z[1]), __float_as_uint(z[2]), tag));
+    }
+  };
+
+  for (;;) {
+    const bool first = it == 0;
+    // ---- p = z + beta p: own rows, then the halo
+    if (roww) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) p[c] = first ? z[c] : fma(beta, p[c], z[c]);
+      if constexpr (k64) vec[3 * mine + comp] = p[0];
+      else reinterpret_cast<float4*>(vec)[mine] = make_float4(p[0], p[1], p[2], 0.f);
+    }
+    bool ok = true;
+    if constexpr (k64) {
+      const int nh3 = 3 * B.nh;
+      for (int h0 = 32 * warp; h0 < nh3; h0 += kThreads) {
+        const int h = h0 + lane;
+        const bool want[1] = {h < nh3};
+        const int col = want[0] ? __ldg(A.h_col + B.hoff + h / 3) : 0, c = h % 3;
+        double zc = 0.0;
+        if (first) {
+          if (want[0]) zc = static_cast<const double*>(sd.cg_z)[4 * (size_t)col + c];
+        } else {
+          const uint4* src = A.pub + 3 * (size_t)(B.row0 + col) + c;
+          uint4 v[1] = {ld_rec(src)};
+          ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, A.ctrs) && ok;
+          zc = rec_val<double>(v[0]);
+        }
+        if (want[0]) {
+          double* pd = vec + 3 * own + h;
+          *pd = first ? zc : fma(beta, *pd, zc);
+        }
+      }
+    } else {
+      float4* ph = reinterpret_cast<float4*>(vec) + own;
+      auto put = [&](int h, const uint4& v) {
+        const float z0 = __uint_as_float(v.x), z1 = __uint_as_float(v.y), z2 = __uint_as_float(v.z);
+        const float4 o = ph[h];
+        ph[h] = first ? make_float4(z0, z1, z2, 0.f)
+                      : make_float4(fma(beta, o.x, z0), fma(beta, o.y, z1), fma(beta, o.z, z2), 0.f);
+      };
+      if (!first)
+        ok = poll_recs<kHaloRegs>(hv, [&](int j) { return A.pub + B.row0 + hc[j]; }, hw, ztag, A.ctrs) && ok;
+#pragma unroll
+      for (int j = 0; j < kHaloRegs; ++j)
+        if (hw[j]) put(threadIdx.x + j * kThreads, hv[j]);
+      for (int h0 = 32 * warp + kHaloRegs * kThreads; h0 < B.nh; h0 += kThreads) {
+        const int h = h0 + lane;
+        const bool want[1] = {h < B.nh};
+        const int col = want[0] ? __ldg(A.h_col + B.hoff + h) : 0;
+        const uint4* src = first ? reinterpret_cast<const uint4*>(static_cast<const float*>(sd.cg_z) + 4 * (size_t)col)
+                                 : A.pub + B.row0 + col;
+        uint4 v[1] = {ld_rec(src)};
+        if (!first) ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, A.ctrs) && ok;
+        if (want[0]) put(h, v[0]);
+      }
+    }
+    if (!__syncthreads_and(ok)) {
+      cgr_abort(A, B);
+      return;
+    }
+    // ---- Ap, (p, Ap)
+    E d1[1] = {E(0)};
+    if (roww) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c] = Real(0);
+      if constexpr (k64) cgr_multiply(M, vec, comp, acc[0]);
+      else cgr_multiply(M, reinterpret_cast<const float4*>(vec), acc);
+    }
+    if constexpr (k64) {
+      if (roww) ex[96 * sl + 32 * comp + lane] = acc[0];
+      __syncthreads();
+      if (lead && live) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) d1[0] = acc_prod(d1[0], vec[3 * mine + c], ex[96 * sl + 32 * c + lane]);
+      }
+    } else if (live) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) d1[0] = acc_prod(d1[0], p[c], acc[c]);
+    }
+    if (!scene_total<E, 1>(A, B, S, lead, sl, seq, d1, nothing)) {
+      cgr_abort(A, B);
+      return;
+    }
+    ++seq;
+    alphaE = rz / d1[0];
+    const Real alpha = Real(to_step(alphaE));
+    // ---- x, r, z, (r, r), (r, z)
+    const bool replace = !k64 && (it + 1) % kCgReplace == 0;
+    E d2[2] = {E(0), E(0)};
+    if constexpr (k64) {
+      double* exr = ex;
+      double* exz = ex + 96 * B.nsl;
+      x[0] = fma(alpha, p[0], x[0]);
+      r[0] = fma(-alpha, acc[0], r[0]);
+      // the lead warps have read Ap of the exchange buffer by now only if
+      // they are past their sum: a barrier before it is reused
+      __syncthreads();
+      if (roww) exr[96 * sl + 32 * comp + lane] = r[0];
+      if (block_jacobi) {
+        __syncthreads();
+        if (roww) {
+          const double* q = exr + 96 * sl + lane;
+          z[0] = fma(dv[2], q[64], fma(dv[1], q[32], dv[0] * q[0]));
+        }
+      } else {
+        z[0] = dv[0] * r[0];
+      }
+      if (roww) exz[96 * sl + 32 * comp + lane] = z[0];
+      publish_z(seq);
+      __syncthreads();
+      if (lead && live) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double rc = exr[96 * sl + 32 * c + lane], zc = exz[96 * sl + 32 * c + lane];
+          d2[0] = acc_prod(d2[0], rc, rc);
+          d2[1] = acc_prod(d2[1], rc, zc);
+        }
+      }
+    } else if (live) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        xe.v[c] = xe.v[c] + two_prod(float(alpha), float(p[c]));
+        r[c] = fma(-alpha, acc[c], r[c]);
+        d2[0] = acc_prod(d2[0], r[c], r[c]);
+      }
+      if (replace) {
+        xe_store(sd.cg_xe, row, xe);
+        __threadfence();
+      }
+      float r3[3] = {float(r[0]), float(r[1]), float(r[2])}, z3[3];
+      precond(r3, z3);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        z[c] = z3[c];
+        d2[1] = acc_prod(d2[1], r[c], z[c]);
+      }
+      if (!replace) publish_z(seq);
+    }
+    if constexpr (!k64) {
+      if (replace) __syncthreads();  // every row's x_e is visible before the block's sums
+    }
+    if (!scene_total<E, 2>(A, B, S, lead, sl, seq, d2, halo_ahead)) {
+      cgr_abort(A, B);
+      return;
+    }
+    ztag = seq;
+    ++seq;
+    rr = d2[0];
+    bool stop = false;
+    if (cg_meets(sd, rr, rr0)) {
+      stop = true;
+    } else {
+      betaE = d2[1] / rz;
+      rz_prev = rz;
+      rz = d2[1];
+      it = it + 1;
+      if (it >= sd.max_cg) {
+        stop = true;
+        cg_status = 5;  // MFEM_ERR_CG_MAXITER
+      }
+    }
+    if (is_nan(rr)) {
+      stop = true;
+      status = 4;
+    }
+    if (stop) break;
+    if constexpr (!k64) {
+      if (replace) {
+        // ---- r = b - A x with x in df64 (k_cg_replace)
+        __syncwarp();
+        __threadfence();
+        E d3[2] = {E(0), E(0)};
+        if (live) {
+          df64 ax[3] = {df64(0.f), df64(0.f), df64(0.f)};
+#pragma unroll 4
+          for (int k = 0; k < M.len; ++k) {
+            const size_t q = ell_pair(M.soff, k, lane, 0);
+            const float* ell = static_cast<const float*>(sd.ell);
+            const float2 w0 = ld_pair<false>(ell, q), w1 = ld_pair<false>(ell, q + 32),
+                         w2 = ld_pair<false>(ell, q + 64), w3 = ld_pair<false>(ell, q + 96),
+                         w4 = ld_pair<false>(ell, q + 128);
+            const X3 xc = xe_load<true>(sd.cg_xe, pair_col(w0));
+            const float a[9] = {w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y, w4.x, w4.y};
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+              for (int j = 0; j < 3; ++j) {
+                const float aij = a[3 * i + j];
+                ax[i] = ax[i] + two_prod(aij, xc.v[j].hi) + df64(aij * xc.v[j].lo);
+              }
+          }
+          float b[3], r3[3], z3[3];
+          ld3<false>(static_cast<const float*>(sd.rhs) + k4, b);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) r3[c] = Ext<float>::to_real(df64(b[c]) - ax[c]);
+          precond(r3, z3);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            r[c] = r3[c];
+            z[c] = z3[c];
+            d3[0] = acc_prod(d3[0], r3[c], r3[c]);
+            d3[1] = acc_prod(d3[1], r3[c], z3[c]);
+          }
+          publish_z(seq);
+        }
+        if (!scene_total<E, 2>(A, B, S, lead, sl, seq, d3, halo_ahead)) {
+          cgr_abort(A, B);
+          return;
+        }
+        ztag = seq;
+        ++seq;
+        rr = d3[0];
+        if (cg_meets(sd, rr, rr0) || is_nan(rr)) {
+          if (is_nan(rr)) status = 4;
+          it = it - 1;  // as in Eigen, the iteration that meets the threshold is not counted
+          break;
+        }
+        betaE = d3[1] / rz_prev;
+        rz = d3[1];
+      }
+    }
+    beta = Real(to_step(betaE));
+  }
+  // ---- the solution and the scene's scalars
+  if (live) {
+    if constexpr (k64) {
+      static_cast<double*>(sd.cg_x)[k4 + comp] = x[0];
+    } else {
+      float xf[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) xf[c] = Ext<float>::to_real(xe.v[c]);
+      st3(static_cast<float*>(sd.cg_x) + k4, xf);
+      xe_store(sd.cg_xe, row, xe);
+    }
+  }
+  if (B.rec == 0 && threadIdx.x == 0) {
+    sc_put(&sc->alpha, alphaE);
+    sc_put(&sc->beta, betaE);
+    sc_put(&sc->rz, rz);
+    sc_put(&sc->rz_prev, rz_prev);
+    sc->cg_err = cg_rel(rr, rr0);
+    sc->cg_iter = it;
+    sc->cg_total += it;
+    if (status) sc->status = status;
+    if (cg_status) sc->cg_status = cg_status;
+    sc->cg_active = 0;
+    sc->nph = kPhLocal;
+    atomicSub(&A.ctrs->cg_active, 1);
+    A.seq[B.scene] = seq;
+  }
+}
+
+// --------------------------------------------- single-reduction form ---
+// The mixed path's Chronopoulos-Gear iteration as cgf_tile runs it, from the
+// state of the vectors of the current parity to the state after the last
+// iteration done: until the recursion's stop is to be verified (cgf_phase set:
+// the next launches of k_cgf_iter verify), or max_iters iterations.  The
+// exchanged vector is w; each block keeps r and s at its halo.
+template <bool kScaled>
+__global__ void __launch_bounds__(256, 1) k_cgr_fused(const CgrArgs A) {
+  constexpr int kThreads = 256;
+  extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
+  __shared__ CgrShared S;
+  const CgrBlock B = A.blocks[blockIdx.x];
+  const SceneDev& sd = A.sds[B.scene];
+  SceneScalars* sc = sd.sc;
+  if (!sc->cg_active || sc->cgf_phase) return;
+  unsigned seq = __ldcg(A.seq + B.scene);
+  const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+  const bool roww = sl < B.nsl;
+  const int row = 32 * (B.slice0 + sl) + lane;
+  const bool live = roww && row < sd.nf;
+  const int own = 32 * B.nsl, mine = 32 * sl + lane;
+  unsigned char* rest;
+  const CgrMatrix<float> M = cgr_load_matrix<float>(A, B, sd, sl, cgr_smem_raw, &rest);
+  float4* u4 = reinterpret_cast<float4*>(rest);         // u at the own rows and the halo
+  float4* sh = u4 + own + B.nh;                         // s at the halo
+  float4* rh = kScaled ? u4 + own : sh + B.nh;          // r at the halo (scaled: u itself)
+  float* Dh = reinterpret_cast<float*>(sh + 2 * B.nh);  // unscaled: M^-1 at the halo, 9 each
+  const int it0 = sc->cg_iter;
+  int it = it0;
+  const float* gr = static_cast<const float*>(sd.cgf_r[it & 1]);
+  const float* gw = static_cast<const float*>(sd.cgf_w[it & 1]);
+  const float* gs = static_cast<const float*>(sd.cgf_s[(it + 1) & 1]);
+  int hc[kHaloRegs];
+  bool hw[kHaloRegs];
+  uint4 hv[kHaloRegs];
+#pragma unroll
+  for (int j = 0; j < kHaloRegs; ++j) {
+    const int h = threadIdx.x + j * kThreads;
+    hw[j] = h < B.nh;
+    hc[j] = hw[j] ? A.h_col[B.hoff + h] : 0;
+    if (hw[j]) hv[j] = *reinterpret_cast<const uint4*>(gw + 4 * (size_t)hc[j]);
+  }
+  for (int h = threadIdx.x; h < B.nh; h += kThreads) {
+    const int col = A.h_col[B.hoff + h];
+    rh[h] = *reinterpret_cast<const float4*>(gr + 4 * (size_t)col);
+    sh[h] = *reinterpret_cast<const float4*>(gs + 4 * (size_t)col);
+    if (!kScaled) {
+      const float* dinv = static_cast<const float*>(sd.dinv);
+      if (sd.block_jacobi) {
+        for (int c = 0; c < 9; ++c) Dh[9 * h + c] = dinv[9 * (size_t)col + c];
+      } else {
+        for (int c = 0; c < 3; ++c) Dh[9 * h + c] = dinv[4 * (size_t)col + c];
+      }
+    }
+  }
+  const size_t k4 = 4 * (size_t)row;
+  float r[3] = {0.f, 0.f, 0.f}, w[3] = {0.f, 0.f, 0.f}, s[3] = {0.f, 0.f, 0.f}, p[3] = {0.f, 0.f, 0.f},
+        x[3] = {0.f, 0.f, 0.f}, u[3] = {0.f, 0.f, 0.f}, dv[3] = {1.f, 1.f, 1.f};
+  if (live) {
+    ld3<false>(gr + k4, r);
+    ld3<false>(gw + k4, w);
+    ld3<false>(gs + k4, s);
+    ld3<false>(static_cast<const float*>(sd.cg_p[0]) + k4, p);
+    ld3<false>(static_cast<const float*>(sd.cg_x) + k4, x);
+    if (kScaled) ld3<false>(static_cast<const float*>(sd.dinv) + k4, dv);
+    else ld3<false>(static_cast<const float*>(sd.cg_z) + k4, u);
+  }
+  df64 gamma = sc_get<df64>(&sc->cgf_gamma[0]), alphaE = sc_get<df64>(&sc->alpha), betaE = sc_get<df64>(&sc->beta);
+  const df64 rr0 = sc_get<df64>(&sc->cg_rhs_norm2);
+  float a = sc->alpha_f, b = sc->beta_f;
+  const int rounds = sc->cgf_rounds;
+  int phase = 0, status = 0, cg_status = 0;
+  df64 rr = rr0;
+  unsigned wtag = 0;
+  bool swapped = false;  // an iteration left the recursion without counting (phase set)
+
+  for (int n = 0;; ++n) {
+    const bool first = n == 0;
+    // ---- own rows: s, r, u, p, x of iteration it + 1
+    float rn[3], un[3];
+    if (live) {
+      float sv[3], uv[3];
+      if (kScaled) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          sv[c] = fma(b, s[c], w[c]);
+          un[c] = fma(-a, sv[c], r[c]);
+          rn[c] = un[c] / dv[c];
+          uv[c] = r[c];
+        }
+      } else {
+        cgf_next<float>(sd, row, r, w, s, a, b, sv, rn, un);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) uv[c] = u[c];
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        p[c] = fma(b, p[c], uv[c]);
+        x[c] = fma(a, p[c], x[c]);
+        s[c] = sv[c];
+        r[c] = kScaled ? un[c] : rn[c];
+        u[c] = un[c];
+      }
+      u4[mine] = make_float4(un[0], un[1], un[2], 0.f);
+    } else if (roww) {
+      u4[mine] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    // ---- the halo's s, r and u
+    const uint4* pw = A.pub + (size_t)(wtag & 1) * A.pub_stride + B.row0;
+    bool ok = true;
+    auto halo = [&](int h, const uint4& v) {
+      const float wc[3] = {__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z)};
+      const float4 so = sh[h], ro = rh[h];
+      const float sn[3] = {fma(b, so.x, wc[0]), fma(b, so.y, wc[1]), fma(b, so.z, wc[2])};
+      const float rc[3] = {fma(-a, sn[0], ro.x), fma(-a, sn[1], ro.y), fma(-a, sn[2], ro.z)};
+      sh[h] = make_float4(sn[0], sn[1], sn[2], 0.f);
+      rh[h] = make_float4(rc[0], rc[1], rc[2], 0.f);
+      if (!kScaled) {
+        float uc[3];
+        const float* D = Dh + 9 * h;
+        if (sd.block_jacobi) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) uc[c] = fma(D[3 * c + 2], rc[2], fma(D[3 * c + 1], rc[1], D[3 * c] * rc[0]));
+        } else {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) uc[c] = D[c] * rc[c];
+        }
+        u4[own + h] = make_float4(uc[0], uc[1], uc[2], 0.f);
+      }
+    };
+    if (!first) ok = poll_recs<kHaloRegs>(hv, [&](int j) { return pw + hc[j]; }, hw, wtag, A.ctrs) && ok;
+#pragma unroll
+    for (int j = 0; j < kHaloRegs; ++j)
+      if (hw[j]) halo(threadIdx.x + j * kThreads, hv[j]);
+    for (int h0 = 32 * sl + kHaloRegs * kThreads; h0 < B.nh; h0 += kThreads) {
+      const int h = h0 + lane;
+      const bool want[1] = {h < B.nh};
+      const int col = want[0] ? __ldg(A.h_col + B.hoff + h) : 0;
+      const uint4* src = first ? reinterpret_cast<const uint4*>(gw + 4 * (size_t)col) : pw + col;
+      uint4 v[1] = {ld_rec(src)};
+      if (!first) ok = poll_recs<1>(v, [&](int) { return src; }, want, wtag, A.ctrs) && ok;
+      if (want[0]) halo(h, v[0]);
+    }
+    if (!__syncthreads_and(ok)) {
+      cgr_abort(A, B);
+      return;
+    }
+    // ---- w = A u, (r, r), (r, u), (w, u)
+    df64 d[3] = {df64(0.f), df64(0.f), df64(0.f)};
+    if (roww) {
+      float acc[3] = {0.f, 0.f, 0.f};
+      cgr_multiply(M, u4, acc);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) w[c] = kScaled ? dv[c] * acc[c] : acc[c];
+      if (live) {
+        if (B.nblk > 1)
+          st_rec(A.pub + (size_t)(seq & 1) * A.pub_stride + B.row0 + row,
+                 make_uint4(__float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), seq));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          d[0] = acc_prod(d[0], rn[c], rn[c]);
+          d[1] = acc_prod(d[1], rn[c], un[c]);
+          d[2] = acc_prod(d[2], acc[c], un[c]);
+        }
+      }
+    }
+    if (!scene_total<df64, 3>(A, B, S, roww, sl, seq, d, [&]() {
+#pragma unroll
+          for (int j = 0; j < kHaloRegs; ++j)
+            if (hw[j]) hv[j] = ld_rec(A.pub + (size_t)(seq & 1) * A.pub_stride + B.row0 + hc[j]);
+        })) {
+      cgr_abort(A, B);
+      return;
+    }
+    wtag = seq;
+    ++seq;
+    // ---- cgf_verify_step, phase 0
+    rr = d[0];
+    if (is_nan(rr)) {
+      status = 4;
+      phase = 3;
+    } else if (cg_meets(sd, rr, rr0)) {
+      phase = rounds < kCgfRounds ? 1 : 3;
+    }
+    if (phase) {
+      swapped = true;
+      break;
+    }
+    cgf_steps(d[1], d[2], gamma, alphaE, &alphaE, &betaE);
+    gamma = d[1];
+    a = to_step(alphaE);
+    b = to_step(betaE);
+    it += 1;
+    if (it >= sd.max_cg) {
+      cg_status = 5;  // MFEM_ERR_CG_MAXITER
+      phase = 3;
+      break;
+    }
+    if (n + 1 >= A.max_iters) break;
+  }
+  // ---- the vectors as k_cgf_iter leaves them after iteration `last`
+  const int last = swapped ? it : it - 1;
+  if (live) {
+    st3(static_cast<float*>(sd.cgf_r[(last + 1) & 1]) + k4, r);
+    st3(static_cast<float*>(sd.cgf_w[(last + 1) & 1]) + k4, w);
+    st3(static_cast<float*>(sd.cgf_s[last & 1]) + k4, s);
+    st3(static_cast<float*>(sd.cg_p[0]) + k4, p);
+    st3(static_cast<float*>(sd.cg_x) + k4, x);
+    if (!kScaled) st3(static_cast<float*>(sd.cg_z) + k4, u);
+  }
+  if (B.rec == 0 && threadIdx.x == 0) {
+    sc->cg_err = cg_rel(rr, rr0);
+    sc_put(&sc->beta, betaE);
+    sc->beta_f = b;
+    sc_put(&sc->alpha, alphaE);
+    sc->alpha_f = a;
+    sc_put(&sc->cgf_gamma[0], gamma);
+    sc->cg_iter = it;
+    sc->cgf_phase = phase;
+    if (status) sc->status = status;
+    if (cg_status) sc->cg_status = cg_status;
+    A.seq[B.scene] = seq;
+  }
+}
+
+template <typename F> auto with_kernel(bool fp64, bool fused, bool jacobi, int threads, bool two, F&& f) {
+  if (fused) return jacobi ? f((const void*)k_cgr_fused<true>) : f((const void*)k_cgr_fused<false>);
+  if (fp64) return threads > 256 ? f((const void*)k_cgr_split<double, 384, 1>) : f((const void*)k_cgr_split<double, 256, 1>);
+  return two ? f((const void*)k_cgr_split<float, 256, 2>) : f((const void*)k_cgr_split<float, 256, 1>);
+}
+
+// Blocks of at most half an SM's shared memory come in pairs.
+bool cgr_pairs(size_t smem) { return smem <= kCgrSmemTwo; }
+
+}  // namespace
+
+int cgr_blocks_per_sm(bool fp64, bool fused, bool jacobi, int threads, size_t smem) {
+  return with_kernel(fp64, fused, jacobi, threads, cgr_pairs(smem), [&](const void* k) {
+    int nb = 0;
+    // the function's limit is shared by every batch: always the largest
+    if (smem > kCgrSmemOne ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgrSmemOne) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, smem) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return nb;
+  });
+}
+
+cudaError_t launch_cgr(const CgrArgs& args, bool fp64, bool fused, bool jacobi, int nblocks, int threads, size_t smem,
+                       cudaStream_t stream) {
+  return with_kernel(fp64, fused, jacobi, threads, cgr_pairs(smem), [&](const void* k) {
+    CgrArgs a = args;
+    void* params[] = {&a};
+    return cudaLaunchCooperativeKernel(k, dim3(nblocks), dim3(threads), params, smem, stream);
+  });
+}
+
+}  // namespace mfem_gpu

@@ -18,6 +18,7 @@
 #include "device_math.cuh"
 #include "kernels.cuh"
 #include "async_copy.cuh"
+#include "pcg.cuh"
 #include "reduce.cuh"
 
 namespace mfem_gpu {
@@ -36,123 +37,6 @@ __device__ __forceinline__ int rec_offset(int i, int j, int l, int m) {
     return start + (l == 0 ? m : (l == 1 ? 2 + m : 5));
   }
   return start + 6 + 9 * (j - i - 1) + 3 * l + m;
-}
-
-// Three components of a row of a 4-padded vector: one 16-byte access in
-// FP32, two in FP64.  kCo: the load bypasses L1 (data written by other
-// blocks earlier in the same launch).
-template <bool kCo>
-__device__ __forceinline__ void ld3(const float* p, float v[3]) {
-  const float4 t = kCo ? __ldcg(reinterpret_cast<const float4*>(p)) : *reinterpret_cast<const float4*>(p);
-  v[0] = t.x;
-  v[1] = t.y;
-  v[2] = t.z;
-}
-template <bool kCo>
-__device__ __forceinline__ void ld3(const double* p, double v[3]) {
-  const double2 a = kCo ? __ldcg(reinterpret_cast<const double2*>(p)) : *reinterpret_cast<const double2*>(p);
-  const double2 b = kCo ? __ldcg(reinterpret_cast<const double2*>(p) + 1) : reinterpret_cast<const double2*>(p)[1];
-  v[0] = a.x;
-  v[1] = a.y;
-  v[2] = b.x;
-}
-__device__ __forceinline__ void st3(float* p, const float v[3]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], 0.f);
-}
-__device__ __forceinline__ void st3(double* p, const double v[3]) {
-  reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
-  reinterpret_cast<double2*>(p)[1] = make_double2(v[2], 0.0);
-}
-
-// Loads of data that other blocks wrote earlier in the same launch: in the
-// persistent PCG (kCo) they bypass L1, which is not coherent across SMs;
-// between separate launches a plain load is fine.
-template <bool kCo, typename T> __device__ __forceinline__ T ldv(const T* p) {
-  if constexpr (kCo) return __ldcg(p);
-  else return *p;
-}
-
-// Pair w of a packed ELL slot; the column of pair 0 is stored as the
-// integer's bits in the first word.
-template <bool kCo>
-__device__ __forceinline__ float2 ld_pair(const float* ell, size_t pair) {
-  const float2* p = reinterpret_cast<const float2*>(ell) + pair;
-  return kCo ? __ldcg(p) : *p;
-}
-template <bool kCo>
-__device__ __forceinline__ double2 ld_pair(const double* ell, size_t pair) {
-  const double2* p = reinterpret_cast<const double2*>(ell) + pair;
-  return kCo ? __ldcg(p) : *p;
-}
-// L2 policies for the PCG's SpMV: the matrix is streamed once per iteration
-// (evict first, no L1 allocation, read-only path), while the vectors the
-// SpMV gathers at neighbouring rows are kept (evict last).  Without them the
-// 115 MB matrix stream of a 1M-tet scene pushes the 4 MB vectors out of L2.
-__device__ __forceinline__ unsigned long long l2_evict_first() {
-  unsigned long long p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ unsigned long long l2_evict_last() {
-  unsigned long long p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ float2 ld_stream(const float* ell, size_t pair, unsigned long long pol) {
-  float2 v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
-               : "=f"(v.x), "=f"(v.y) : "l"(reinterpret_cast<const float2*>(ell) + pair), "l"(pol));
-  return v;
-}
-__device__ __forceinline__ double2 ld_stream(const double* ell, size_t pair, unsigned long long pol) {
-  double2 v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
-               : "=d"(v.x), "=d"(v.y) : "l"(reinterpret_cast<const double2*>(ell) + pair), "l"(pol));
-  return v;
-}
-// Gather of a row's three components with the keep policy (between
-// launches only: the persistent form bypasses L1 instead).
-__device__ __forceinline__ void ld3_keep(const float* p, float v[3], unsigned long long pol) {
-  float4 t;
-  asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
-               : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "l"(p), "l"(pol));
-  v[0] = t.x;
-  v[1] = t.y;
-  v[2] = t.z;
-}
-__device__ __forceinline__ void ld3_keep(const double* p, double v[3], unsigned long long pol) {
-  double2 a, b;
-  asm volatile("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(a.x), "=d"(a.y) : "l"(p), "l"(pol));
-  asm volatile("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(b.x), "=d"(b.y) : "l"(p + 2), "l"(pol));
-  v[0] = a.x;
-  v[1] = a.y;
-  v[2] = b.x;
-}
-template <bool kCo, typename Real>
-__device__ __forceinline__ void ld3_gather(const Real* p, Real v[3], unsigned long long pol) {
-  if constexpr (kCo) ld3<true>(p, v);
-  else ld3_keep(p, v, pol);
-}
-
-__device__ __forceinline__ int pair_col(float2 w) { return __float_as_int(w.x); }
-__device__ __forceinline__ int pair_col(double2 w) { return (int)__double_as_longlong(w.x); }
-
-// x of the mixed-path PCG in df64: a row is 4 float pairs (32 bytes).
-struct X3 {
-  df64 v[3];
-};
-__device__ __forceinline__ X3 zero_x3() { return X3{{df64(0.f), df64(0.f), df64(0.f)}}; }
-template <bool kCo>
-__device__ __forceinline__ X3 xe_load(const void* base, int row) {
-  const float4* p = static_cast<const float4*>(base) + 2 * (size_t)row;
-  const float4 a = kCo ? __ldcg(p) : p[0];
-  const float4 b = kCo ? __ldcg(p + 1) : p[1];
-  return X3{{df64(a.x, a.y), df64(a.z, a.w), df64(b.x, b.y)}};
-}
-__device__ __forceinline__ void xe_store(void* base, int row, const X3& x) {
-  float4* p = static_cast<float4*>(base) + 2 * (size_t)row;
-  p[0] = make_float4(x.v[0].hi, x.v[0].lo, x.v[1].hi, x.v[1].lo);
-  p[1] = make_float4(x.v[2].hi, x.v[2].lo, 0.f, 0.f);
 }
 
 constexpr int kAsmWindow = 64;  // block slots per warp accumulated in shared memory per pass
@@ -380,27 +264,6 @@ __global__ void __launch_bounds__(256) k_assemble(const Tile* tiles, const Scene
   }
 }
 
-// ---------------------------------------------------------------- PCG ---
-// Products of two Reals carried exactly in Ext (TwoProduct in the mixed path).
-__device__ __forceinline__ df64 exact_prod(float a, float b) { return two_prod(a, b); }
-__device__ __forceinline__ double exact_prod(double a, double b) { return a * b; }
-
-// z = D^{-1} r for one row (Jacobi or 3x3 block Jacobi).
-template <typename Real>
-__device__ __forceinline__ void apply_prec(const SceneDev& sd, int row, const Real r[3], Real z[3]) {
-  const Real* dinv = static_cast<const Real*>(sd.dinv);
-  if (sd.block_jacobi) {
-    const Real* D = dinv + 9 * (size_t)row;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) z[c] = D[3 * c] * r[0] + D[3 * c + 1] * r[1] + D[3 * c + 2] * r[2];
-  } else {
-    Real d[3];
-    ld3<false>(dinv + 4 * (size_t)row, d);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) z[c] = d[c] * r[c];
-  }
-}
-
 // ------------------------------------------------------------- PCG ------
 // Every kernel writes tile partials; the last tile of a scene to finish
 // (atomic tickets, no thread waits) reduces them in a fixed order and sets
@@ -431,8 +294,8 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_init(const Tile* tiles, const
     if (sd.cg_xe) xe_store(sd.cg_xe, row, zero_x3());
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      dots[0] = dots[0] + exact_prod(r[c], r[c]);
-      dots[1] = dots[1] + exact_prod(r[c], z[c]);
+      dots[0] = acc_prod(dots[0], r[c], r[c]);
+      dots[1] = acc_prod(dots[1], r[c], z[c]);
     }
   }
   tile_partials<E, Real, 2, 0>(dots, nullptr, partials, pstride, 0, tix);
@@ -441,27 +304,22 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_init(const Tile* tiles, const
     E v[2];
     scene_sums<E, 2>(partials, pstride, 0, t0, tc, v);
     if (threadIdx.x == 0) {
-      const double rrs = to_double_any(v[0]), rzs = to_double_any(v[1]);
-      sc->cg_rhs_norm2 = rrs;
+      sc_put(&sc->cg_rhs_norm2, v[0]);
       sc->cg_iter = 0;
-      sc->beta = 0.0;
+      sc_put(&sc->beta, E(0));
       sc->beta_f = 0.0f;
-      sc->rz = rzs;
+      sc_put(&sc->rz, v[1]);
       sc->cg_err = 0.0;
-      if (rrs == 0.0) {
+      if (is_zero(v[0])) {
         sc->cg_active = 0;
         sc->nph = kPhLocal;
+      } else if (cg_meets(sd, v[0], v[0]) || sd.max_cg <= 0) {
+        sc->cg_active = 0;
+        sc->nph = kPhLocal;
+        sc->cg_err = 1.0;
       } else {
-        const double thr = fmax(sd.cg_tol * sd.cg_tol * rrs, DBL_MIN);
-        sc->cg_threshold = thr;
-        if (rrs < thr || sd.max_cg <= 0) {
-          sc->cg_active = 0;
-          sc->nph = kPhLocal;
-          sc->cg_err = 1.0;
-        } else {
-          sc->cg_active = 1;
-          atomicAdd(&ctrs->cg_active, 1);
-        }
+        sc->cg_active = 1;
+        atomicAdd(&ctrs->cg_active, 1);
       }
     }
   }
@@ -507,11 +365,9 @@ __device__ __forceinline__ void cg_spmv_tile(int tix, const Tile* tiles, const S
         Real pp[3];
         ld3_gather<kCo>(pin + 4 * (size_t)col, pp, pol_k);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) p[c] += beta * pp[c];
+        for (int c = 0; c < 3; ++c) p[c] = fma(beta, pp[c], p[c]);
       }
-      acc0 += w0.y * p[0] + w1.x * p[1] + w1.y * p[2];
-      acc1 += w2.x * p[0] + w2.y * p[1] + w3.x * p[2];
-      acc2 += w3.y * p[0] + w4.x * p[1] + w4.y * p[2];
+      ell_block_fma(w0, w1, w2, w3, w4, p, acc0, acc1, acc2);
     }
     const Real acc[3] = {acc0, acc1, acc2};
     Real p[3];
@@ -520,21 +376,21 @@ __device__ __forceinline__ void cg_spmv_tile(int tix, const Tile* tiles, const S
       Real pp[3];
       ld3<kCo>(pin + 4 * (size_t)row, pp);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) p[c] += beta * pp[c];
+      for (int c = 0; c < 3; ++c) p[c] = fma(beta, pp[c], p[c]);
     }
     st3(pout + 4 * (size_t)row, p);
     st3(Ap + 4 * (size_t)row, acc);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) pAp[0] = pAp[0] + exact_prod(p[c], acc[c]);
+    for (int c = 0; c < 3; ++c) pAp[0] = acc_prod(pAp[0], p[c], acc[c]);
   }
   tile_partials<E, Real, 1, 0>(pAp, nullptr, partials, pstride, 0, tix);
   if (last_tile(sd, TB_CG, tix)) {
     E s[1];
     scene_sums<E, 1>(partials, pstride, 0, sd.tile_first[TB_CG], sd.tile_count[TB_CG], s);
     if (threadIdx.x == 0) {
-      const double a = Fin<Real>::div(ldv<kCo>(&sc->rz), to_double_any(s[0]));
-      sc->alpha = a;
-      sc->alpha_f = float(a);
+      const E a = sc_get<E>(&sc->rz) / s[0];
+      sc_put(&sc->alpha, a);
+      sc->alpha_f = float(to_step(a));
     }
   }
 }
@@ -572,44 +428,44 @@ __device__ __forceinline__ void cg_update_tile(int tix, const Tile* tiles, const
       xe_store(sd.cg_xe, row, xe);
     } else {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) xv[c] += alpha * pv[c];
+      for (int c = 0; c < 3; ++c) xv[c] = fma(alpha, pv[c], xv[c]);
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      rv[c] -= alpha * av[c];
-      dots[0] = dots[0] + exact_prod(rv[c], rv[c]);
+      rv[c] = fma(-alpha, av[c], rv[c]);
+      dots[0] = acc_prod(dots[0], rv[c], rv[c]);
     }
     st3(x, xv);
     st3(r, rv);
     apply_prec<Real>(sd, row, rv, z);
     st3(static_cast<Real*>(sd.cg_z) + k, z);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) dots[1] = dots[1] + exact_prod(rv[c], z[c]);
+    for (int c = 0; c < 3; ++c) dots[1] = acc_prod(dots[1], rv[c], z[c]);
   }
   tile_partials<E, Real, 2, 0>(dots, nullptr, partials, pstride, 0, tix);
   if (last_tile(sd, TB_CG, tix)) {
     E v[2];
     scene_sums<E, 2>(partials, pstride, 0, sd.tile_first[TB_CG], sd.tile_count[TB_CG], v);
     if (threadIdx.x == 0) {
-      const double rrs = to_double_any(v[0]), rzs = to_double_any(v[1]);
-      sc->cg_err = Fin<Real>::sqrt_ratio(rrs, ldv<kCo>(&sc->cg_rhs_norm2));
+      const E rr0 = sc_get<E>(&sc->cg_rhs_norm2);
+      sc->cg_err = cg_rel(v[0], rr0);
       bool stop = false;
-      if (rrs < ldv<kCo>(&sc->cg_threshold)) {
+      if (cg_meets(sd, v[0], rr0)) {
         stop = true;
       } else {
-        const double rz_old = ldv<kCo>(&sc->rz);
-        const double b = Fin<Real>::div(rzs, rz_old);
-        sc->beta = b;
-        sc->beta_f = float(b);
-        sc->rz_prev = rz_old;
-        sc->rz = rzs;
+        const E rz_old = sc_get<E>(&sc->rz);
+        const E b = v[1] / rz_old;
+        sc_put(&sc->beta, b);
+        sc->beta_f = float(to_step(b));
+        sc_put(&sc->rz_prev, rz_old);
+        sc_put(&sc->rz, v[1]);
         sc->cg_iter = it + 1;
         if (it + 1 >= sd.max_cg) {
           stop = true;
           sc->cg_status = 5;  // MFEM_ERR_CG_MAXITER
         }
       }
-      if (!(rrs == rrs)) {
+      if (is_nan(v[0])) {
         stop = true;
         sc->status = 4;
       }
@@ -667,8 +523,8 @@ __device__ __forceinline__ void cg_replace_tile(int tix, const Tile* tiles, cons
     st3(static_cast<float*>(sd.cg_z) + 4 * (size_t)row, z);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      dots[0] = dots[0] + exact_prod(r[c], r[c]);
-      dots[1] = dots[1] + exact_prod(r[c], z[c]);
+      dots[0] = acc_prod(dots[0], r[c], r[c]);
+      dots[1] = acc_prod(dots[1], r[c], z[c]);
     }
   }
   tile_partials<df64, float, 2, 0>(dots, nullptr, partials, pstride, 0, tix);
@@ -676,10 +532,10 @@ __device__ __forceinline__ void cg_replace_tile(int tix, const Tile* tiles, cons
     df64 v[2];
     scene_sums<df64, 2>(partials, pstride, 0, sd.tile_first[TB_CG], sd.tile_count[TB_CG], v);
     if (threadIdx.x == 0) {
-      const double rrs = to_double_any(v[0]), rzs = to_double_any(v[1]);
-      sc->cg_err = Fin<float>::sqrt_ratio(rrs, ldv<kCo>(&sc->cg_rhs_norm2));
-      if (rrs < ldv<kCo>(&sc->cg_threshold) || !(rrs == rrs)) {
-        if (!(rrs == rrs)) sc->status = 4;
+      const df64 rr0 = sc_get<df64>(&sc->cg_rhs_norm2);
+      sc->cg_err = cg_rel(v[0], rr0);
+      if (cg_meets(sd, v[0], rr0) || is_nan(v[0])) {
+        if (is_nan(v[0])) sc->status = 4;
         // x_{cg_iter} meets the threshold: as in Eigen, that iteration is not counted
         const int done = ldv<kCo>(&sc->cg_iter) - 1;
         sc->cg_iter = done;
@@ -689,10 +545,10 @@ __device__ __forceinline__ void cg_replace_tile(int tix, const Tile* tiles, cons
         sc->nph = kPhLocal;
         atomicSub(&ctrs->cg_active, 1);
       } else {
-        const double b2 = Fin<float>::div(rzs, ldv<kCo>(&sc->rz_prev));
-        sc->beta = b2;
-        sc->beta_f = float(b2);
-        sc->rz = rzs;
+        const df64 b2 = v[1] / sc_get<df64>(&sc->rz_prev);
+        sc_put(&sc->beta, b2);
+        sc->beta_f = to_step(b2);
+        sc_put(&sc->rz, v[1]);
       }
     }
   }
@@ -732,33 +588,6 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_update(const Tile* tiles, con
 // iteration parity, so no row is overwritten while another block reads it).
 // In exact arithmetic the iterates are those of the two-reduction PCG.
 
-// acc += B u for one packed ELL slot (pairs (col, a00) (a01, a02) (a10, a11)
-// (a12, a20) (a21, a22)), as explicit FMA chains: every form of the fused
-// iteration (registers or staged through shared memory) rounds alike.
-template <typename P, typename Real>
-__device__ __forceinline__ void ell_block_fma(const P& w0, const P& w1, const P& w2, const P& w3, const P& w4,
-                                              const Real u[3], Real& a0, Real& a1, Real& a2) {
-  a0 = fma(w1.y, u[2], fma(w1.x, u[1], fma(w0.y, u[0], a0)));
-  a1 = fma(w3.x, u[2], fma(w2.y, u[1], fma(w2.x, u[0], a1)));
-  a2 = fma(w4.y, u[2], fma(w4.x, u[1], fma(w3.y, u[0], a2)));
-}
-
-// u_{i+1} of a row from r_i, w_i, s_{i-1}: the same operations, in the same
-// order, wherever a row's value is formed.
-template <typename Real>
-__device__ __forceinline__ void cgf_next(const SceneDev& sd, int row, const Real r[3], const Real w[3],
-                                         const Real sp[3], Real a, Real b, Real s[3], Real rn[3],
-                                         Real u[3]) {
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    s[c] = fma(b, sp[c], w[c]);
-    rn[c] = fma(-a, s[c], r[c]);
-  }
-  apply_prec<Real>(sd, row, rn, u);
-}
-
-__device__ __forceinline__ void cgf_verify_step(const SceneDev& sd, BatchCounters* ctrs, double rr, double g,
-                                                double d, double su, double ps, int it);
 
 // The three inner products of one tile as tile partials; the scene's last
 // tile reduces them and sets a, b of the next iteration and the stopping
@@ -775,57 +604,50 @@ __device__ __forceinline__ void cgf_finish(const SceneDev& sd, BatchCounters* ct
     E v[NQ];
     scene_sums<E, NQ>(partials, pstride, 0, sd.tile_first[TB_CG], sd.tile_count[TB_CG], v);
     if (threadIdx.x == 0) {
-      const double rr = to_double_any(v[0]), g = to_double_any(v[1]), d = to_double_any(v[2]);
-      const double su = NQ > 3 ? to_double_any(v[NQ > 3 ? 3 : 0]) : 0.0;
-      const double ps = NQ > 4 ? to_double_any(v[NQ > 4 ? 4 : 0]) : 0.0;
+      const E rr = v[0], g = v[1], d = v[2];
       if (kInit) {
-        sc->cg_rhs_norm2 = rr;
+        sc_put(&sc->cg_rhs_norm2, rr);
         sc->cg_iter = 0;
         sc->cg_err = 0.0;
         sc->cgf_phase = 0;
         sc->cgf_rounds = 0;
-        const double thr = fmax(sd.cg_tol * sd.cg_tol * rr, DBL_MIN);
-        sc->cg_threshold = thr;
-        if (rr == 0.0) {
+        if (is_zero(rr)) {
           sc->cg_active = 0;
-          sc->nph = kPhLocal;
-        } else if (rr < thr || sd.max_cg <= 0) {
+        } else if (cg_meets(sd, rr, rr) || sd.max_cg <= 0) {
           sc->cg_active = 0;
-          sc->nph = kPhLocal;
           sc->cg_err = 1.0;
         } else {
           sc->cg_active = 1;
           atomicAdd(&ctrs->cg_active, 1);
         }
         sc->nph = sc->cg_active ? kPhPcg : kPhLocal;
-        const double a0 = Fin<Real>::div(g, d);
-        sc->cgf_gamma[0] = g;
-        sc->alpha = a0;
-        sc->alpha_f = float(a0);
-        sc->beta = 0.0;
+        const E a0 = g / d;
+        sc_put(&sc->cgf_gamma[0], g);
+        sc_put(&sc->alpha, a0);
+        sc->alpha_f = float(to_step(a0));
+        sc_put(&sc->beta, E(0));
         sc->beta_f = 0.0f;
-      } else if (sizeof(Real) == 4 && sd.cg_xe) {
-        cgf_verify_step(sd, ctrs, rr, g, d, su, ps, it);
+      } else if constexpr (sizeof(Real) == 4) {
+        cgf_verify_step(sd, ctrs, rr, g, d, v[NQ > 3 ? 3 : 0], v[NQ > 4 ? 4 : 0], it);
       } else {
         bool stop = false;
-        sc->cg_err = Fin<Real>::sqrt_ratio(rr, sc->cg_rhs_norm2);
-        if (rr < sc->cg_threshold) {
+        const E rr0 = sc_get<E>(&sc->cg_rhs_norm2);
+        sc->cg_err = cg_rel(rr, rr0);
+        if (cg_meets(sd, rr, rr0)) {
           stop = true;
         } else {
-          const double bn = Fin<Real>::div(g, sc->cgf_gamma[0]);
-          const double an = Fin<Real>::div(g, d - Fin<Real>::div(bn * g, sc->alpha));
-          sc->beta = bn;
-          sc->beta_f = float(bn);
-          sc->alpha = an;
-          sc->alpha_f = float(an);
-          sc->cgf_gamma[0] = g;
+          E an, bn;
+          cgf_steps(g, d, sc_get<E>(&sc->cgf_gamma[0]), sc_get<E>(&sc->alpha), &an, &bn);
+          sc_put(&sc->beta, bn);
+          sc_put(&sc->alpha, an);
+          sc_put(&sc->cgf_gamma[0], g);
           sc->cg_iter = it + 1;
           if (it + 1 >= sd.max_cg) {
             stop = true;
             sc->cg_status = 5;  // MFEM_ERR_CG_MAXITER
           }
         }
-        if (!(rr == rr)) {
+        if (is_nan(rr)) {
           stop = true;
           sc->status = 4;
         }
@@ -838,87 +660,6 @@ __device__ __forceinline__ void cgf_finish(const SceneDev& sd, BatchCounters* ct
         }
       }
     }
-  }
-}
-
-// ---------------------------------------- verified stop (mixed path) ---
-// In FP32 the single-reduction recurrences drift: the recursive residual
-// meets the tolerance while the true |b - A x| / |b| sits several times
-// above it (x itself rounded to FP32 floors it near eps32 |A||x| / |b|).
-// So when the recursion says "converged", the mixed path verifies before it
-// stops, in three further launches of the same kernel (the scene's
-// cgf_phase selects the work; the iteration count does not move):
-//   1  r = b - A (x_e + x), with each FP32 matrix entry times the df64
-//      x_e + x as an exact product summed in df64 (the reliable residual);
-//      u = M^-1 r;
-//   2  x_e += x, x = 0 (the FP32 x restarts as a correction, so its
-//      rounding shrinks with what is left to solve); w = A u and s = A p
-//      (the recursions' drift starts again from zero); the inner products
-//      of the true residual.  If it meets the tolerance: phase 3.
-//      Otherwise the recursion continues from the replaced r, w and s:
-//      the next direction u + b p is made A-conjugate to p directly (b =
-//      -(A p, u) / (p, A p)), because the drifted recursion's
-//      gamma_prev no longer describes the true residual, and a from the
-//      exact (p_new, A p_new).  After kCgfRounds failed verifications the
-//      next recursive stop is accepted as it is;
-//   3  x_e += x, and x = round(x_e) for the readers of the solution; stop.
-// A stop on max_iterative_solver_iters or a non-finite residual also goes
-// through phase 3, so the solution is always x_e + x.
-
-// The finalizer's part for the mixed path (thread 0 of the scene's last tile).
-constexpr int kCgfRounds = 4;
-__device__ __forceinline__ void cgf_verify_step(const SceneDev& sd, BatchCounters* ctrs, double rr, double g,
-                                                double d, double su, double ps, int it) {
-  SceneScalars* sc = sd.sc;
-  const int ph = sc->cgf_phase;
-  if (ph == 1) {
-    sc->cgf_phase = 2;
-    return;
-  }
-  if (ph == 3 || *(volatile int*)&ctrs->error) {
-    sc->cg_total += sc->cg_iter;
-    sc->cg_active = 0;
-    sc->nph = kPhLocal;
-    atomicSub(&ctrs->cg_active, 1);
-    return;
-  }
-  sc->cg_err = Fin<float>::sqrt_ratio(rr, sc->cg_rhs_norm2);
-  if (!(rr == rr)) {
-    sc->status = 4;
-    sc->cgf_phase = 3;
-    return;
-  }
-  if (rr < sc->cg_threshold) {
-    // phase 0: the recursion's residual passes, verify it (unless the
-    // verifications are used up); phase 2: the true residual passes, write
-    // the solution
-    sc->cgf_phase = (ph == 0 && sc->cgf_rounds < kCgfRounds) ? 1 : 3;
-    return;
-  }
-  double bn, an;
-  if (ph == 2) {
-    // A failed verification.  The recursion's gamma had drifted below the
-    // true residual's, so b = gamma / gamma_prev would be far too large: the
-    // new direction is made A-conjugate to the last one directly,
-    // b = -(A p, u) / (p, A p), and (p_new, A p_new) = d + 2 b (A p, u) +
-    // b^2 (p, A p) from phase 2's exact A p.
-    sc->cgf_rounds += 1;
-    bn = -Fin<float>::div(su, ps);
-    an = Fin<float>::div(g, d + 2.0 * bn * su + bn * bn * ps);
-  } else {
-    bn = Fin<float>::div(g, sc->cgf_gamma[0]);
-    an = Fin<float>::div(g, d - Fin<float>::div(bn * g, sc->alpha));
-  }
-  sc->beta = bn;
-  sc->beta_f = float(bn);
-  sc->alpha = an;
-  sc->alpha_f = float(an);
-  sc->cgf_gamma[0] = g;
-  sc->cg_iter = it + 1;
-  sc->cgf_phase = 0;
-  if (it + 1 >= sd.max_cg) {
-    sc->cg_status = 5;  // MFEM_ERR_CG_MAXITER
-    sc->cgf_phase = 3;
   }
 }
 

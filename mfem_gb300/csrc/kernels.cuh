@@ -71,11 +71,11 @@ struct SceneScalars {
   double E, E_prev, eres, decrement;
   // PCG (Eigen ConjugateGradient semantics)
   int cg_active, cg_iter, cg_total, cg_status;
-  double cg_rhs_norm2, cg_threshold, rz, alpha, beta, cg_err;
+  // (|b|^2, (r, z), step lengths: slots in the path's high precision, float
+  // pairs in the mixed path)
+  double cg_rhs_norm2, rz, alpha, beta, cg_err;
   double rz_prev;    // rz of the previous iteration (residual replacement)
-  // single-reduction PCG: (r, u) and alpha of iteration i in slot i & 1
-  // (kernel i reads slot (i+1) & 1 and its first block writes slot i & 1)
-  double cgf_gamma[2], cgf_alpha[2];
+  double cgf_gamma[1];  // single-reduction PCG: (r, u) of the last iteration
   // mixed path: verification phase of the single-reduction PCG (0: iterate;
   // 1: r = b - A (x_e + x) exactly; 2: fold x into x_e, w = A u and the
   // inner products of the true residual; 3: write the rounded solution)
@@ -143,6 +143,7 @@ struct SceneDev {
   double dt;         // beta*h
   float2 h2x;        // h2 as a float pair (df64), and float(h2) in .x
   double newton_tol, res_tol, cg_tol;
+  float2 cg_tolx, cg_itolx;  // cg_tol and 1 / cg_tol as float pairs
   double load_norm;  // |h^2 P M f| over the free dofs (scale of the residual test)
   int max_newton, max_ls, max_cg, bdf_order;
   double bdf_alpha[6];

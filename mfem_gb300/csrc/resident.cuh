@@ -1,0 +1,67 @@
+// A whole PCG solve in one cooperative launch with the matrix resident in
+// shared memory (k_resident.cu): the plan the host builds for a batch and the
+// launch wrappers.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "kernels.cuh"
+
+namespace mfem_gpu {
+
+// One block: a run of 32-row slices of one scene.
+struct CgrBlock {
+  int scene;        // slot in the batch
+  int slice0, nsl;  // its slices
+  int kres;         // ELL slots of each slice kept in shared memory (the rest read from L2)
+  int hoff, nh;     // its halo: columns outside its rows, CgrArgs::h_col[hoff ..]
+  int loff;         // its slots' local column indices, CgrArgs::lidx[loff ..] in slot order
+  int rec0, nrec;   // the scene's exchange records: first, count
+  int rec;          // the block's first record among them
+  int row0;         // the scene's first row in the exchanged vector
+  int nblk;         // blocks of the scene
+  int tile;         // 1: the block is a reduction tile (8 slices) and sends its sum; 0: its slices' sums
+};
+
+struct CgrArgs {
+  const CgrBlock* blocks;
+  const int* h_col;
+  const uint16_t* lidx;
+  uint4* recs;        // [parity][quantity 0..2][nrec_total] tagged partial sums
+  uint4* pub;         // [parity][rows (x 3 in FP64)] tagged vector
+  int nrec_total;
+  size_t pub_stride;  // records of one parity of pub
+  unsigned int* seq;  // per scene: the next exchange's tag
+  const SceneDev* sds;
+  BatchCounters* ctrs;
+  int max_iters;      // single-reduction form: iterations of this launch at most
+};
+
+constexpr int kCgrTile = kCgRows / 32;  // slices of a reduction tile
+constexpr int kCgrMaxSlices = 8;        // slices of a block
+constexpr int kCgrMaxSliceTiles = 96;   // reduction tiles of a scene whose blocks send slice sums
+
+// Dynamic shared memory of a block with `slots` resident slots, `own` rows
+// (32 per slice) and `nh` halo columns.
+constexpr size_t cgr_smem(bool fp64, bool fused, bool jacobi, size_t slots, size_t own, size_t nh) {
+  const size_t w = fp64 ? 8 : 4;
+  size_t b = slots * (288 * w + 64);                  // 9 planes and the column indices
+  b += fp64 ? 24 * (own + nh) : 16 * (own + nh);      // the multiplied vector
+  if (fp64) b += 48 * own;                            // exchange between the component warps
+  if (fused) b += 16 * nh + (jacobi ? 0 : 16 * nh + 36 * nh);
+  return b;
+}
+// Dynamic shared memory a block may take when one or two share an SM.
+constexpr size_t kCgrSmemOne = 223 * 1024 - 4096, kCgrSmemTwo = 105 * 1024;
+constexpr int cgr_threads(bool fp64, int spb) { return fp64 && spb > 2 ? 384 : 256; }
+constexpr int kCgrMaxSpb64 = 4;  // three component warps a slice
+
+// Blocks per SM that can be resident with this much dynamic shared memory.
+int cgr_blocks_per_sm(bool fp64, bool fused, bool jacobi, int threads, size_t smem);
+// The solve of every active scene.  fused: the single-reduction iteration
+// (mixed path), up to args.max_iters iterations or until a scene's stop is to
+// be verified; else Eigen's two-reduction iteration to its end.
+cudaError_t launch_cgr(const CgrArgs& args, bool fp64, bool fused, bool jacobi, int nblocks, int threads, size_t smem,
+                       cudaStream_t stream);
+
+}  // namespace mfem_gpu
