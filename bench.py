@@ -942,9 +942,7 @@ def run_tri2d(args):
                 "algorithmic_bytes_per_launch": abytes, "avg_launch_us": 1e3 * dom_ms / dom_n,
                 "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)",
                 "note": (f"{cg_per_launch:.1f} PCG iterations per launch; the sheet's system "
-                         "sits in L2; " + ("one thread block runs the solve" if sc.n_free <= 1024 else
-                                            "co-resident blocks with grid barriers run the solve "
-                                            "(t2_pcg_grid)"))
+                         "sits in shared memory (t2_pcg_res), too large a one in L2 (t2_pcg_grid)")
                         if dom == "t2_pcg" else None}
     sc.close()
     newton = float(np.mean([t["newton_iterations"] for t in stats]))

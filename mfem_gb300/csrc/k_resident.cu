@@ -28,10 +28,11 @@
 // form's vector has a second exchange between its reading and its writing.
 // Sequence numbers go on from launch to launch (CgrArgs::seq).
 //
-// Every wait is bounded: after kCgrTimeoutNs the block raises ctrs->error and
+// Every wait is bounded: after kExchangeTimeoutNs the block raises ctrs->error and
 // leaves, as do the others when they see the flag or time out themselves; the
 // host reports MFEM_ERR_TIMEOUT.  The launch is cooperative: all blocks are
 // co-resident, the exchange needs them all.
+#include "exchange.cuh"
 #include "pcg.cuh"
 #include "resident.cuh"
 
@@ -39,84 +40,16 @@ namespace mfem_gpu {
 
 namespace {
 
-constexpr unsigned long long kCgrTimeoutNs = 2000000000ull;
-constexpr unsigned int kCgrMaxPolls = 1u << 24;
-
-__device__ __forceinline__ uint4 ld_rec(const uint4* p) {
-  unsigned long long a, b;
-  asm volatile(
-      "{\n\t.reg .b128 q;\n\t"
-      "ld.relaxed.gpu.global.b128 q, [%2];\n\t"
-      "mov.b128 {%0, %1}, q;\n\t}"
-      : "=l"(a), "=l"(b)
-      : "l"(p)
-      : "memory");
-  return make_uint4((unsigned)a, (unsigned)(a >> 32), (unsigned)b, (unsigned)(b >> 32));
-}
-__device__ __forceinline__ void st_rec(uint4* p, uint4 v) {
-  const unsigned long long a = (unsigned long long)v.x | ((unsigned long long)v.y << 32);
-  const unsigned long long b = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
-  asm volatile(
-      "{\n\t.reg .b128 q;\n\t"
-      "mov.b128 q, {%1, %2};\n\t"
-      "st.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p),
-      "l"(a), "l"(b)
-      : "memory");
-}
+using mfem_gpu::rec_of;
 __device__ __forceinline__ uint4 rec_of(df64 v, unsigned tag) {
   return make_uint4(__float_as_uint(v.hi), __float_as_uint(v.lo), 0u, tag);
-}
-__device__ __forceinline__ uint4 rec_of(double v, unsigned tag) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  return make_uint4((unsigned)b, (unsigned)(b >> 32), 0u, tag);
 }
 template <typename E> __device__ __forceinline__ E rec_val(uint4 v);
 template <> __device__ __forceinline__ df64 rec_val<df64>(uint4 v) {
   return df64(__uint_as_float(v.x), __uint_as_float(v.y));
 }
 template <> __device__ __forceinline__ double rec_val<double>(uint4 v) {
-  return __longlong_as_double((long long)((unsigned long long)v.x | ((unsigned long long)v.y << 32)));
-}
-
-__device__ __forceinline__ unsigned long long cgr_now() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Whether a wait of the calling warp has run out, or another block has raised
-// the error flag; every 64th poll (n counts them, t0 is set on the first
-// call).  Warp-uniform.
-__device__ __noinline__ bool wait_over(unsigned n, unsigned long long* t0, BatchCounters* ctrs) {
-  const unsigned long long now = cgr_now();
-  if (*t0 == 0) *t0 = now;
-  bool over = *(volatile int*)&ctrs->error != 0;
-  if (now - *t0 > kCgrTimeoutNs || n > kCgrMaxPolls) {
-    atomicExch(&ctrs->error, 1);
-    over = true;
-  }
-  return __any_sync(0xffffffffu, over);
-}
-
-// Loads N records a lane and polls until all of them carry the tag, the whole
-// warp in step (a lane that stopped polling early would leave the warp
-// diverged for the shuffles that follow).  want: the records the lane needs;
-// the others' values are not looked at.  False: the wait ran out.
-template <int N, typename Ptr>
-__device__ __forceinline__ bool poll_recs(uint4 (&v)[N], const Ptr& at, const bool (&want)[N], unsigned tag,
-                                          BatchCounters* ctrs) {
-  unsigned long long t0 = 0;
-#pragma unroll 1
-  for (unsigned n = 1;; ++n) {
-    bool good = true;
-#pragma unroll
-    for (int q = 0; q < N; ++q) good = good && (!want[q] || v[q].w == tag);
-    if (__all_sync(0xffffffffu, good)) return true;
-    if ((n & 63u) == 0 && wait_over(n, &t0, ctrs)) return false;
-#pragma unroll
-    for (int q = 0; q < N; ++q)
-      if (want[q]) v[q] = ld_rec(at(q));
-  }
+  return rec_double(v);
 }
 
 __device__ __forceinline__ df64 shfl_to(df64 v, int lane) {
@@ -190,7 +123,7 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
       want[q] = i < n;
       w[q] = ld_rec(src + (size_t)q * A.nrec_total);
     }
-    const bool ok = poll_recs<NQ>(w, [&](int q) { return src + (size_t)q * A.nrec_total; }, want, seq, A.ctrs);
+    const bool ok = poll_recs<NQ>(w, [&](int q) { return src + (size_t)q * A.nrec_total; }, want, seq, &A.ctrs->error);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) a[q] = i < n ? rec_val<E>(w[q]) : E(0);
     return ok;
@@ -499,7 +432,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_cgr_split(const CgrArg
         } else {
           const uint4* src = A.pub + 3 * (size_t)(B.row0 + col) + c;
           uint4 v[1] = {ld_rec(src)};
-          ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, A.ctrs) && ok;
+          ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, &A.ctrs->error) && ok;
           zc = rec_val<double>(v[0]);
         }
         if (want[0]) {
@@ -516,7 +449,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_cgr_split(const CgrArg
                       : make_float4(fma(beta, o.x, z0), fma(beta, o.y, z1), fma(beta, o.z, z2), 0.f);
       };
       if (!first)
-        ok = poll_recs<kHaloRegs>(hv, [&](int j) { return A.pub + B.row0 + hc[j]; }, hw, ztag, A.ctrs) && ok;
+        ok = poll_recs<kHaloRegs>(hv, [&](int j) { return A.pub + B.row0 + hc[j]; }, hw, ztag, &A.ctrs->error) && ok;
 #pragma unroll
       for (int j = 0; j < kHaloRegs; ++j)
         if (hw[j]) put(threadIdx.x + j * kThreads, hv[j]);
@@ -527,7 +460,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_cgr_split(const CgrArg
         const uint4* src = first ? reinterpret_cast<const uint4*>(static_cast<const float*>(sd.cg_z) + 4 * (size_t)col)
                                  : A.pub + B.row0 + col;
         uint4 v[1] = {ld_rec(src)};
-        if (!first) ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, A.ctrs) && ok;
+        if (!first) ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, &A.ctrs->error) && ok;
         if (want[0]) put(h, v[0]);
       }
     }
@@ -857,7 +790,7 @@ __global__ void __launch_bounds__(256, 1) k_cgr_fused(const CgrArgs A) {
         u4[own + h] = make_float4(uc[0], uc[1], uc[2], 0.f);
       }
     };
-    if (!first) ok = poll_recs<kHaloRegs>(hv, [&](int j) { return pw + hc[j]; }, hw, wtag, A.ctrs) && ok;
+    if (!first) ok = poll_recs<kHaloRegs>(hv, [&](int j) { return pw + hc[j]; }, hw, wtag, &A.ctrs->error) && ok;
 #pragma unroll
     for (int j = 0; j < kHaloRegs; ++j)
       if (hw[j]) halo(threadIdx.x + j * kThreads, hv[j]);
@@ -867,7 +800,7 @@ __global__ void __launch_bounds__(256, 1) k_cgr_fused(const CgrArgs A) {
       const int col = want[0] ? __ldg(A.h_col + B.hoff + h) : 0;
       const uint4* src = first ? reinterpret_cast<const uint4*>(gw + 4 * (size_t)col) : pw + col;
       uint4 v[1] = {ld_rec(src)};
-      if (!first) ok = poll_recs<1>(v, [&](int) { return src; }, want, wtag, A.ctrs) && ok;
+      if (!first) ok = poll_recs<1>(v, [&](int) { return src; }, want, wtag, &A.ctrs->error) && ok;
       if (want[0]) halo(h, v[0]);
     }
     if (!__syncthreads_and(ok)) {

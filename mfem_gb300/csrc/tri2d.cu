@@ -25,13 +25,13 @@
 //               the Aloc of the incident triangles in the assembler's
 //               sorted order, + mass, Jacobi inverse, and its RHS
 //   t2_norm     one block: |rhs|^2
-//   t2_pcg      ONE thread block for the whole PCG solve: every reduction a
-//               fixed-order tree in shared memory, __syncthreads between the
-//               phases, no grid-wide waits; one launch per solve.  Sheets
-//               with more free rows than the block has threads run
-//               t2_pcg_grid instead: the single-reduction form of the same
-//               iteration over co-resident blocks, one bounded grid barrier
-//               an iteration, also one launch per solve
+//   t2_pcg_res  the whole PCG solve in one cooperative launch, the matrix in
+//               shared memory, at most 64 rows a block; the blocks exchange
+//               through tagged records (exchange.cuh).  t2_pcg_res2 is its
+//               two-reduction form for sheets of at most 1024 free rows.
+//               Sheets too large to be resident run
+//   t2_pcg_grid the same single-reduction iteration over co-resident blocks,
+//               the system read from L2, one bounded grid barrier an iteration
 //   t2_local    one thread per triangle: lambda and ds
 //   t2_energy   one thread per triangle and vertex: the three energy parts
 //   t2_esum     one block: the fixed-order sums (and max|dx|, max|ds|)
@@ -51,13 +51,14 @@
 
 #include "../../include/mfem_gb300.h"
 #include "device_math.cuh"
+#include "exchange.cuh"
 
 namespace {
 
 using mfem_gpu::psd_fix_n;
 
 constexpr int kThreads = 128;
-constexpr int kBlock = 1024;  // the single-block kernels (PCG, sums)
+constexpr int kBlock = 1024;  // the single-block kernels (sums)
 constexpr double kPsdTol = 1e-6;
 constexpr double kDsvdTol = 1e-4;  // dsvd.cpp:153
 
@@ -113,6 +114,18 @@ struct T2 {
   double* sr;     // the grid PCG's r, w, s by iteration parity: 6 x 2 nf (r0 r1 w0 w1 s0 s1)
   double* part;   // the grid PCG's block partials: 3 x kT2MaxGrid
   unsigned int* bar;  // the grid PCG's barrier: arrivals, generation, error flag
+  // resident PCG: block b's row i is res_first b + res_stride i (i <
+  // res_rows); the slots of each block's slices of 32 rows, each slot's column
+  // as an index into the block's rows and halo, the halos' rows, and the
+  // exchange's records
+  int res_first, res_stride, res_rows;
+  const int* res_slot;         // blocks x slices + 1: first slot of each slice
+  const int* res_hptr;         // blocks + 1
+  const int* res_hcol;
+  const uint16_t* res_lidx;    // 32 per slot
+  uint4* res_recs;             // [parity][3][2 blocks]
+  uint4* res_pub;              // [parity][2 nf]
+  unsigned int* res_seq;
   double* epart;  // 2 nt + nv energy parts
   double* scal;   // SC_COUNT device scalars
   int* status;    // worst status the kernels saw
@@ -438,93 +451,8 @@ __global__ void __launch_bounds__(kBlock) t2_norm(T2 d) {
   if (threadIdx.x == 0) d.scal[SC_RN2] = s;
 }
 
-// The whole Jacobi-PCG solve LHS dx = rhs from dx = 0 in one thread block,
-// Eigen's ConjugateGradient iteration: stop when |r|^2 < max(tol^2 |b|^2,
-// DBL_MIN) or after max_iter iterations (the breaking iteration is not
-// counted).  Every loop bound and break test is block-uniform: the
-// scalars come out of block_sum, which all threads read after a barrier.
-__global__ void __launch_bounds__(kBlock) t2_pcg(T2 d, int max_iter, double tol) {
-  __shared__ double sh[kBlock];
-  const int n = 2 * d.nf, t = threadIdx.x;
-  double part = 0;
-  for (int i = t; i < n; i += kBlock) {
-    const double ri = d.rhs[i];
-    d.dx[i] = 0.0;
-    d.r[i] = ri;
-    part += ri * ri;
-  }
-  const double b2 = block_sum(part, sh);
-  if (b2 == 0.0) {
-    if (t == 0) {
-      d.scal[SC_CG_IT] = 0;
-      d.scal[SC_CG_RN2] = 0;
-      d.scal[SC_CG_B2] = 0;
-    }
-    return;
-  }
-  const double thr = fmax(tol * tol * b2, DBL_MIN);
-  double rn2 = b2;
-  if (b2 < thr) {  // Eigen's test before the first iteration: no iteration
-    if (t == 0) {
-      d.scal[SC_CG_IT] = 0;
-      d.scal[SC_CG_RN2] = b2;
-      d.scal[SC_CG_B2] = b2;
-    }
-    return;
-  }
-  part = 0;
-  for (int i = t; i < n; i += kBlock) {
-    const double pi = d.dinv[i] * d.r[i];
-    d.p[i] = pi;
-    part += d.r[i] * pi;
-  }
-  double absNew = block_sum(part, sh);
-  int it = 0;
-  while (it < max_iter) {
-    part = 0;
-    for (int rr = t; rr < d.nf; rr += kBlock) {
-      double y0 = 0, y1 = 0;
-      for (int qq = d.b_ptr[rr]; qq < d.b_ptr[rr + 1]; ++qq) {
-        const double* a = d.A + 4 * size_t(qq);
-        const int c = d.b_col[qq];
-        const double p0 = d.p[2 * c], p1 = d.p[2 * c + 1];
-        y0 += a[0] * p0 + a[1] * p1;
-        y1 += a[2] * p0 + a[3] * p1;
-      }
-      d.q[2 * rr] = y0;
-      d.q[2 * rr + 1] = y1;
-      part += d.p[2 * rr] * y0 + d.p[2 * rr + 1] * y1;
-    }
-    const double alpha = absNew / block_sum(part, sh);
-    part = 0;
-    for (int i = t; i < n; i += kBlock) {
-      d.dx[i] += alpha * d.p[i];
-      const double ri = d.r[i] - alpha * d.q[i];
-      d.r[i] = ri;
-      part += ri * ri;
-    }
-    rn2 = block_sum(part, sh);
-    if (rn2 < thr) break;
-    part = 0;
-    for (int i = t; i < n; i += kBlock) part += d.r[i] * (d.dinv[i] * d.r[i]);
-    const double absOld = absNew;
-    absNew = block_sum(part, sh);
-    const double beta = absNew / absOld;
-    for (int i = t; i < n; i += kBlock) d.p[i] = d.dinv[i] * d.r[i] + beta * d.p[i];
-    __syncthreads();  // p complete before the next product gathers it
-    ++it;
-  }
-  if (t == 0) {
-    d.scal[SC_CG_IT] = it;
-    d.scal[SC_CG_RN2] = rn2;
-    d.scal[SC_CG_B2] = b2;
-  }
-}
-
 // ----------------------------------------------------- grid PCG ---
-// The Jacobi-PCG over many blocks for sheets too large for one (the FP64
-// work of a 10^4-triangle sheet on one SM at GB300's FP64 rate sets ~40 us
-// per iteration).  One cooperative launch of G blocks of kGridThreads, each
+// The Jacobi-PCG of sheets too large for t2_pcg_res.  One cooperative launch of G blocks of kGridThreads, each
 // owning a contiguous range of free rows; a reduction is each block's
 // fixed-order partial, a bounded grid barrier, and the G partials summed in
 // the same fixed order by every block (so every block takes the same
@@ -763,6 +691,548 @@ __global__ void __launch_bounds__(kGridThreads) t2_pcg_grid(T2 d, int max_iter, 
   }
 }
 
+// ------------------------------------------------- resident PCG ---
+// The whole solve in one launch with the matrix in shared memory.  What bounds
+// it is the latency of the FP64 pipe (66-79 cycles an instruction whatever its
+// lanes do, 576 a division) and of the exchange through L2.  So a block takes
+// few rows (a warp has one component of 32 of them), each quantity of a sum is
+// one warp's, quotients by numbers known beforehand are products with their
+// reciprocals (quotient_by), and p and x are updated while the sums are under
+// way.  The blocks exchange tagged records (exchange.cuh).  Two forms: sheets
+// of at most 1024 free rows iterate as Eigen does (two reductions), larger
+// ones in the single-reduction form.  The order of every sum is that of one
+// block of 1024 threads and of t2_pcg_grid's blocks: Newton's last steps on a
+// sheet are decided by energy differences near rounding, so that another
+// order would move the converged state by 1e-9.  An iteration, before (one
+// block up to 1024 rows, t2_pcg_grid above) and now: 99 rows 20.3 -> 6.9 us,
+// 1,071 rows 19.7 -> 5.7 us, 4,191 rows 20.5 -> 6.6 us, 9,999 rows (157
+// blocks, some SMs with two) 23.8 -> 8.4 us.
+//
+// A record is overwritten only after everybody has read it: records alternate
+// between two buffers by the exchange's parity, and a block writes exchange
+// k + 2 only after it has read k + 1 from every block, which each wrote after
+// reading k.
+constexpr int kResThreads = 256;
+constexpr int kResOwn = 64;  // local indices of a block's own rows; its halo follows
+
+// num / den for a den whose correctly rounded reciprocal is at hand: one
+// product and one correction of the remainder give the correctly rounded
+// quotient (Markstein 1990), in 3 instead of the division's 9 latencies.
+__device__ __forceinline__ double quotient_by(double num, double den, double rcp) {
+  const double q = num * rcp;
+  const double v = fma(fma(-den, q, num), rcp, q);
+  return isfinite(v) ? v : num / den;
+}
+
+// A block's rows, halo and matrix.  mat: [slot][4][32] doubles per slice,
+// li: [slot][32] local column indices.
+struct T2Block {
+  double* mat;
+  const uint16_t* li;
+  int nsl, h0, nh, slot0, slots;
+};
+constexpr size_t t2_res_smem(size_t slots, size_t nh) {
+  return slots * (1024 + 64) + (kResOwn + nh) * 16 + 16 * kResOwn * 3 + 16 * nh * 2;
+}
+
+// Row l of slice sl of block bk: consecutive rows, or (stride > 1) every
+// stride-th row.
+__device__ __forceinline__ int t2_res_row(const T2& d, int bk, int i) { return d.res_first * bk + d.res_stride * i; }
+
+__device__ __forceinline__ T2Block t2_res_load(const T2& d, unsigned char* smem, unsigned char** rest) {
+  T2Block B;
+  const int bk = blockIdx.x;
+  B.nsl = (d.res_rows + 31) / 32;
+  B.h0 = d.res_hptr[bk];
+  B.nh = d.res_hptr[bk + 1] - B.h0;
+  B.slot0 = d.res_slot[bk * B.nsl];
+  B.slots = d.res_slot[(bk + 1) * B.nsl] - B.slot0;
+  B.mat = reinterpret_cast<double*>(smem);
+  uint16_t* li = reinterpret_cast<uint16_t*>(B.mat + (size_t)B.slots * 128);
+  B.li = li;
+  *rest = reinterpret_cast<unsigned char*>(li + (size_t)B.slots * 32);
+  for (int s = 0; s < B.nsl; ++s) {
+    const int a0 = d.res_slot[bk * B.nsl + s] - B.slot0, len = d.res_slot[bk * B.nsl + s + 1] - B.slot0 - a0;
+    for (int i = threadIdx.x; i < 32 * len; i += kResThreads) {
+      const int k = i >> 5, l = i & 31, at = 32 * s + l;
+      const int r = t2_res_row(d, bk, at);
+      double2 v0 = make_double2(0.0, 0.0), v1 = v0;
+      if (at < d.res_rows && r < d.nf && d.b_ptr[r] + k < d.b_ptr[r + 1]) {
+        const double2* q = reinterpret_cast<const double2*>(d.A + 4 * (size_t)(d.b_ptr[r] + k));
+        v0 = q[0];
+        v1 = q[1];
+      }
+      double* m = B.mat + 128 * (size_t)(a0 + k) + l;
+      m[0] = v0.x;
+      m[32] = v0.y;
+      m[64] = v1.x;
+      m[96] = v1.y;
+      li[32 * (a0 + k) + l] = d.res_lidx[32 * (size_t)(B.slot0 + a0 + k) + l];
+    }
+  }
+  return B;
+}
+
+// One component of (A u) in a row: y += (a0 u0 + a1 u1) over the slots in
+// order, rounded as t2_pcg_grid's row-per-thread product rounds it.
+__device__ __forceinline__ double t2_res_mul(const T2Block& B, int s_at, int s_len, int comp, const double* u) {
+  const int lane = threadIdx.x & 31;
+  const double* m = B.mat + 128 * (size_t)s_at + 64 * comp + lane;
+  const uint16_t* l = B.li + 32 * s_at + lane;
+  double y = 0.0;
+#pragma unroll 4
+  for (int k = 0; k < s_len; ++k) {
+    const double2 uc = *reinterpret_cast<const double2*>(u + 2 * (int)l[32 * k]);
+    y = __dadd_rn(y, fma(m[128 * k], uc.x, __dmul_rn(m[128 * k + 32], uc.y)));
+  }
+  return y;
+}
+
+// n records of one quantity summed by the calling warp: lane l over records
+// l, l + 32, ..; then a tree.  ok is cleared when a wait ran out.
+__device__ __forceinline__ double t2_res_fetch(const uint4* rec, int n, unsigned seq, int* err, bool& ok) {
+  using namespace mfem_gpu;
+  const int lane = threadIdx.x & 31;
+  double v = 0.0;
+  for (int i0 = 0; i0 < n && ok; i0 += 128) {
+    uint4 g[4];
+    bool want[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      want[j] = i0 + 32 * j + lane < n;
+      if (want[j]) g[j] = ld_rec(rec + i0 + 32 * j + lane);
+    }
+    ok = poll_recs<4>(g, [&](int j) { return rec + i0 + 32 * j + lane; }, want, seq, err);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v += want[j] ? rec_double(g[j]) : 0.0;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+  return v;
+}
+
+__device__ __forceinline__ void t2_res_leave(const T2& d) {
+  if (threadIdx.x == 0) {
+    atomicExch(d.status, MFEM_ERR_TIMEOUT);
+    atomicAdd(d.res_seq, 0x100000u);  // later launches use other tags
+  }
+}
+
+// Single-reduction form (t2_pcg_grid's iteration and sums): blocks of at most
+// 64 consecutive rows; the exchange carries w and (r, u), (w, u), |r|^2, one
+// exchange an iteration; each block updates r and s at its halo itself.
+__global__ void __launch_bounds__(kResThreads) t2_pcg_res(T2 d, int max_iter, double tol) {
+  using namespace mfem_gpu;
+  extern __shared__ __align__(16) unsigned char res_smem[];
+  __shared__ double half[3][2], tot[3], step[2];
+  __shared__ int flags;  // 1: a wait ran out, 2: converged
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int G = gridDim.x, bk = blockIdx.x;
+  unsigned char* rest;
+  const T2Block B = t2_res_load(d, res_smem, &rest);
+  double* u = reinterpret_cast<double*>(rest);  // [own + nh][2]
+  double* ru = u + 2 * (kResOwn + B.nh);        // the own rows' r, u, y for the sums: [3][2 own]
+  double* rh = ru + 6 * kResOwn;                // r and s at the halo
+  double* sh = rh + 2 * B.nh;
+  const int sl = warp >> 1, comp = warp & 1;  // owner warps: 0..3
+  const bool roww = warp < 4 && sl < B.nsl;
+  const int at = 32 * sl + lane, row = t2_res_row(d, bk, at);
+  const bool live = roww && at < d.res_rows && row < d.nf;
+  const size_t dof = 2 * (size_t)row + comp;
+  const int mine = 2 * at + comp;
+  const int s_at = roww ? d.res_slot[bk * B.nsl + sl] - B.slot0 : 0;
+  const int s_len = roww ? d.res_slot[bk * B.nsl + sl + 1] - B.slot0 - s_at : 0;
+  unsigned seq = __ldcg(d.res_seq);
+  int* err = reinterpret_cast<int*>(d.bar + 2);
+  // halo entries (row, component) of this thread: the first two in registers
+  constexpr int kHalo = 2;
+  int hc[kHalo];
+  bool hw[kHalo];
+  uint4 hv[kHalo];
+  double hd[kHalo];
+#pragma unroll
+  for (int j = 0; j < kHalo; ++j) {
+    const int i = threadIdx.x + j * kResThreads;
+    hw[j] = i < 2 * B.nh;
+    hc[j] = hw[j] ? 2 * d.res_hcol[B.h0 + (i >> 1)] + (i & 1) : 0;
+    hd[j] = hw[j] ? d.dinv[hc[j]] : 0.0;
+  }
+  for (int i = threadIdx.x; i < 2 * B.nh; i += kResThreads) {
+    const size_t c = 2 * (size_t)d.res_hcol[B.h0 + (i >> 1)] + (i & 1);
+    rh[i] = d.rhs[c];
+    sh[i] = 0.0;
+    u[2 * kResOwn + i] = d.dinv[c] * d.rhs[c];
+  }
+  double di = 0.0, r = 0.0, un = 0.0, w = 0.0, s = 0.0, p = 0.0, x = 0.0;
+  if (live) {
+    di = d.dinv[dof];
+    r = d.rhs[dof];
+    un = di * r;
+  }
+  if (threadIdx.x == 0) flags = 0;
+  if (roww) u[mine] = un;
+
+  // w = A u and the sums' parts; then the three sums in tot.  `beside`: work
+  // of the owners while the sums are under way.  False: a wait ran out.
+  auto product_and_sums = [&](auto beside) -> bool {
+    if (roww) {
+      w = t2_res_mul(B, s_at, s_len, comp, u);
+      if (live && G > 1) st_rec(d.res_pub + (size_t)(seq & 1) * 2 * d.nf + dof, rec_of(w, seq));
+      ru[mine] = r;
+      ru[2 * kResOwn + mine] = un;
+      ru[4 * kResOwn + mine] = w;
+    }
+    __syncthreads();
+    // warp 2 + q + 3 s: quantity q over slice s's rows
+    const int task = warp - 2, q = task % 3, ts = task / 3;
+    if (task >= 0 && ts < B.nsl) {
+      const double* X = ru + (q == 1 ? 4 * kResOwn : 0) + 2 * (32 * ts + lane);
+      const double* Y = ru + (q == 2 ? 0 : 2 * kResOwn) + 2 * (32 * ts + lane);
+      double v = fma(X[1], Y[1], X[0] * Y[0]);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+      if (lane == 0) half[q][ts] = v;
+    }
+    __syncthreads();
+    if (task >= 0 && ts == 0) {
+      const double v = B.nsl > 1 ? half[q][0] + half[q][1] : half[q][0];
+      uint4* rec = d.res_recs + ((size_t)(seq & 1) * 3 + q) * G;
+      double t = v;
+      if (G > 1) {
+        if (lane == 0) st_rec(rec + bk, rec_of(v, seq));
+        bool ok = true;
+        if (task < 2) beside();  // owners (warps 2, 3)
+        t = t2_res_fetch(rec, G, seq, err, ok);
+        if (!ok && lane == 0) atomicOr(&flags, 1);
+      } else if (task < 2) {
+        beside();
+      }
+      if (lane == 0) tot[q] = t;
+    } else {
+      beside();
+    }
+    __syncthreads();
+    return (flags & 1) == 0;
+  };
+
+  __syncthreads();
+  if (!product_and_sums([] {})) {
+    t2_res_leave(d);
+    return;
+  }
+  ++seq;
+  double g = tot[0];
+  const double b2 = tot[2], thr = fmax(tol * tol * b2, DBL_MIN);
+  double a = g / tot[1], bt = 0.0, rn2 = b2, rg = 0.0, ra = 0.0;
+  int it = 0;
+  const bool any = !(b2 == 0.0 || b2 < thr);  // Eigen's test before the first iteration
+#pragma unroll
+  for (int j = 0; j < kHalo; ++j)
+    if (hw[j]) hv[j] = ld_rec(d.res_pub + (size_t)((seq - 1) & 1) * 2 * d.nf + hc[j]);
+  while (any && it < max_iter) {
+    // s_k, r_{k+1}, u_{k+1}: own rows, then the halo
+    const double u_old = un;
+    if (roww) {
+      t2_next(r, w, s, di, a, bt, s, r, un);
+      u[mine] = un;
+    }
+    bool ok = true;
+    if (G > 1) {
+      const uint4* pw = d.res_pub + (size_t)((seq - 1) & 1) * 2 * d.nf;
+      auto halo = [&](int i, double wc, double dc) {
+        double sn, rn, uc;
+        t2_next(rh[i], wc, sh[i], dc, a, bt, sn, rn, uc);
+        sh[i] = sn;
+        rh[i] = rn;
+        u[2 * kResOwn + i] = uc;
+      };
+      ok = poll_recs<kHalo>(hv, [&](int j) { return pw + hc[j]; }, hw, seq - 1, err);
+#pragma unroll
+      for (int j = 0; j < kHalo; ++j)
+        if (hw[j]) halo(threadIdx.x + j * kResThreads, rec_double(hv[j]), hd[j]);
+      for (int i0 = 32 * warp + kHalo * kResThreads; i0 < 2 * B.nh; i0 += kResThreads) {
+        const int i = i0 + lane;
+        const bool want[1] = {i < 2 * B.nh};
+        const int c = want[0] ? 2 * __ldg(d.res_hcol + B.h0 + (i >> 1)) + (i & 1) : 0;
+        uint4 v[1] = {ld_rec(pw + c)};
+        ok = poll_recs<1>(v, [&](int) { return pw + c; }, want, seq - 1, err) && ok;
+        if (want[0]) halo(i, rec_double(v[0]), __ldg(d.dinv + c));
+      }
+    }
+    if (!__syncthreads_and(ok)) {
+      t2_res_leave(d);
+      return;
+    }
+    if (!product_and_sums([&] {
+          if (live) {  // p_k = u_k + b p_{k-1}, x += a p
+            p = fma(bt, p, u_old);
+            x = fma(a, p, x);
+          }
+          if (warp == 0) {
+            rg = 1.0 / g;
+            ra = 1.0 / a;
+          }
+        })) {
+      t2_res_leave(d);
+      return;
+    }
+    // the next halo's records are under way while the step lengths are formed
+#pragma unroll
+    for (int j = 0; j < kHalo; ++j)
+      if (hw[j]) hv[j] = ld_rec(d.res_pub + (size_t)(seq & 1) * 2 * d.nf + hc[j]);
+    ++seq;
+    rn2 = tot[2];
+    if (warp == 0) {
+      const double gn = tot[0], dn = tot[1];
+      const double bn = quotient_by(gn, g, rg);
+      const double an = gn / (dn - quotient_by(bn * gn, a, ra));
+      if (lane == 0) {
+        step[0] = an;
+        step[1] = bn;
+      }
+    } else if (warp == 1 && lane == 0 && rn2 < thr) {
+      flags = 2;
+    }
+    __syncthreads();
+    if (flags & 2) break;
+    a = step[0];
+    bt = step[1];
+    g = tot[0];
+    ++it;
+  }
+  if (live) d.dx[dof] = x;
+  if (bk == 0 && threadIdx.x == 0) {
+    d.scal[SC_CG_IT] = it;
+    d.scal[SC_CG_RN2] = rn2;
+    d.scal[SC_CG_B2] = b2;
+    d.res_seq[0] = seq;
+  }
+}
+
+// Two-reduction form (Eigen's iteration) of sheets of at most 1024 free rows.
+// Its sums are those of one block of 1024 threads, thread t over entries t and
+// t + 1024 (dofs) or row t, then a tree that adds entry t + w to t for w =
+// 512, 256, .., 1.  With block c of B (a power of two) owning the rows c, c +
+// B, .., the tree's levels down to B (rows) or 2 B (dofs) stay inside a block,
+// and the rest are levels of a tree over the blocks' one or two values, which
+// every block adds up itself.
+__global__ void __launch_bounds__(kResThreads) t2_pcg_res2(T2 d, int max_iter, double tol) {
+  using namespace mfem_gpu;
+  extern __shared__ __align__(16) unsigned char res_smem[];
+  __shared__ double tot[2], beta_s;
+  __shared__ int flags;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int G = gridDim.x, bk = blockIdx.x;
+  unsigned char* rest;
+  const T2Block B = t2_res_load(d, res_smem, &rest);
+  double* pv = reinterpret_cast<double*>(rest);  // p: [own + nh][2]
+  double* ex = pv + 2 * (kResOwn + B.nh);        // entries of the sums: [2 or 3][2 own]
+  const int comp = warp & 1;  // owner warps: 0, 1
+  const bool roww = warp < 2;
+  const int row = t2_res_row(d, bk, lane);
+  const bool live = roww && lane < d.res_rows && row < d.nf;
+  const size_t dof = 2 * (size_t)row + comp;
+  const int mine = 2 * lane + comp;
+  const int s_len = B.slots;
+  unsigned seq = __ldcg(d.res_seq);
+  int* err = reinterpret_cast<int*>(d.bar + 2);
+  constexpr int kHalo = 2;
+  int hc[kHalo];
+  bool hw[kHalo];
+  uint4 hv[kHalo];
+  double hd[kHalo];
+#pragma unroll
+  for (int j = 0; j < kHalo; ++j) {
+    const int i = threadIdx.x + j * kResThreads;
+    hw[j] = i < 2 * B.nh;
+    hc[j] = hw[j] ? 2 * d.res_hcol[B.h0 + (i >> 1)] + (i & 1) : 0;
+    hd[j] = hw[j] ? d.dinv[hc[j]] : 0.0;
+  }
+  for (int i = threadIdx.x; i < 2 * B.nh; i += kResThreads) pv[2 * kResOwn + i] = 0.0;
+  double di = 0.0, r = 0.0, z = 0.0, p = 0.0, x = 0.0, y = 0.0;
+  if (live) {
+    di = d.dinv[dof];
+    r = d.rhs[dof];
+    z = di * r;
+  }
+  if (threadIdx.x == 0) flags = 0;
+
+  // One sum by the calling warp.  Lane i holds the entries of the block's row
+  // i (dofs: one per component, e0 and e1; else e0).  Rows i and i + k are k G
+  // rows (2 k G dofs) apart, so the levels inside the block run over i; absent
+  // rows are zeros.  Then the levels over blocks.
+  auto send_and_fetch = [&](int q, bool dofs, double e0, double e1, bool& ok) -> double {
+    // (dofs 1024 apart, rows 16 apart with 32 blocks, are one thread's: added
+    // by the caller)
+    for (int off = dofs && G == 32 ? 8 : 16; off > 0; off >>= 1) {
+      const double f0 = __shfl_down_sync(0xffffffffu, e0, off), f1 = __shfl_down_sync(0xffffffffu, e1, off);
+      e0 += f0;
+      if (dofs) e1 += f1;
+    }
+    const int n = dofs ? 2 * G : G;
+    if (G == 1) {
+      return dofs ? __shfl_sync(0xffffffffu, e0 + e1, 0) : __shfl_sync(0xffffffffu, e0, 0);
+    }
+    uint4* rec = d.res_recs + ((size_t)(seq & 1) * 3 + q) * 2 * G;
+    if (lane == 0) {
+      if (dofs) {
+        st_rec(rec + 2 * bk, rec_of(e0, seq));
+        st_rec(rec + 2 * bk + 1, rec_of(e1, seq));
+      } else {
+        st_rec(rec + bk, rec_of(e0, seq));
+      }
+    }
+    // n <= 64 values: lane l holds values l and l + 32
+    uint4 g[2];
+    bool want[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      want[j] = 32 * j + lane < n;
+      if (want[j]) g[j] = ld_rec(rec + 32 * j + lane);
+    }
+    ok = poll_recs<2>(g, [&](int j) { return rec + 32 * j + lane; }, want, seq, err);
+    double v = want[0] ? rec_double(g[0]) : 0.0;
+    if (n > 32) v += want[1] ? rec_double(g[1]) : 0.0;  // w = 32
+    for (int off = min(n, 32) >> 1; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    return __shfl_sync(0xffffffffu, v, 0);
+  };
+  // r, from which every block forms z = D^-1 r and p at its halo
+  auto publish_r = [&]() {
+    if (live && G > 1) st_rec(d.res_pub + (size_t)(seq & 1) * 2 * d.nf + dof, rec_of(r, seq));
+  };
+  // (r, r) and (r, z) in tot; False: a wait ran out
+  auto sums_rz = [&]() -> bool {
+    if (roww) {
+      ex[mine] = r;
+      ex[2 * kResOwn + mine] = z;
+    }
+    publish_r();
+    __syncthreads();
+    if (warp == 2 || warp == 3) {
+      const double2 rr = *reinterpret_cast<const double2*>(ex + 2 * lane);
+      const double2 oo = warp == 2 ? rr : *reinterpret_cast<const double2*>(ex + 2 * kResOwn + 2 * lane);
+      bool ok = true;
+      double e0 = rr.x * oo.x, e1 = rr.y * oo.y;
+      if (G == 32) {  // a thread's second entry
+        const double2 r2 = *reinterpret_cast<const double2*>(ex + 2 * ((lane + 16) & 31));
+        const double2 o2 = warp == 2 ? r2 : *reinterpret_cast<const double2*>(ex + 2 * kResOwn + 2 * ((lane + 16) & 31));
+        e0 = fma(r2.x, o2.x, e0);
+        e1 = fma(r2.y, o2.y, e1);
+      }
+      const double v = send_and_fetch(warp - 2, true, e0, e1, ok);
+      if (lane == 0) {
+        if (!ok) atomicOr(&flags, 1);
+        tot[warp - 2] = v;
+      }
+    }
+    __syncthreads();
+    return (flags & 1) == 0;
+  };
+
+  __syncthreads();
+  if (!sums_rz()) {
+    t2_res_leave(d);
+    return;
+  }
+  unsigned rtag = seq;
+  ++seq;
+  const double b2 = tot[0], thr = fmax(tol * tol * b2, DBL_MIN);
+  double rz = tot[1], beta = 0.0, rn2 = b2, rr_z = 0.0;
+  int it = 0;
+  const bool any = !(b2 == 0.0 || b2 < thr);  // Eigen's test before the first iteration
+  auto halo_ahead = [&](unsigned tag) {
+#pragma unroll
+    for (int j = 0; j < kHalo; ++j)
+      if (hw[j]) hv[j] = ld_rec(d.res_pub + (size_t)(tag & 1) * 2 * d.nf + hc[j]);
+  };
+  halo_ahead(rtag);
+  while (any && it < max_iter) {
+    // p = D^-1 r + beta p: own rows, then the halo
+    const bool first = it == 0;
+    if (roww) {
+      p = first ? z : fma(di, r, beta * p);
+      pv[mine] = p;
+    }
+    bool ok = true;
+    if (G > 1) {
+      const uint4* pr = d.res_pub + (size_t)(rtag & 1) * 2 * d.nf;
+      auto halo = [&](int i, double rc, double dc) {
+        double* q = pv + 2 * kResOwn + i;
+        *q = first ? dc * rc : fma(dc, rc, beta * *q);
+      };
+      ok = poll_recs<kHalo>(hv, [&](int j) { return pr + hc[j]; }, hw, rtag, err);
+#pragma unroll
+      for (int j = 0; j < kHalo; ++j)
+        if (hw[j]) halo(threadIdx.x + j * kResThreads, rec_double(hv[j]), hd[j]);
+      for (int i0 = 32 * warp + kHalo * kResThreads; i0 < 2 * B.nh; i0 += kResThreads) {
+        const int i = i0 + lane;
+        const bool want[1] = {i < 2 * B.nh};
+        const int c = want[0] ? 2 * __ldg(d.res_hcol + B.h0 + (i >> 1)) + (i & 1) : 0;
+        uint4 v[1] = {ld_rec(pr + c)};
+        ok = poll_recs<1>(v, [&](int) { return pr + c; }, want, rtag, err) && ok;
+        if (want[0]) halo(i, rec_double(v[0]), __ldg(d.dinv + c));
+      }
+    }
+    if (!__syncthreads_and(ok)) {
+      t2_res_leave(d);
+      return;
+    }
+    if (roww) {
+      y = t2_res_mul(B, 0, s_len, comp, pv);
+      ex[mine] = y;
+    }
+    __syncthreads();
+    if (warp == 2) {
+      const double2 yy = *reinterpret_cast<const double2*>(ex + 2 * lane);
+      const double2 pp = *reinterpret_cast<const double2*>(pv + 2 * lane);
+      const double v = send_and_fetch(0, false, fma(pp.x, yy.x, pp.y * yy.y), 0.0, ok);
+      if (lane == 0) {
+        if (!ok) atomicOr(&flags, 1);
+        tot[0] = rz / v;
+      }
+    } else if (warp == 3) {
+      rr_z = 1.0 / rz;  // for the next beta
+    }
+    __syncthreads();
+    if (flags & 1) {
+      t2_res_leave(d);
+      return;
+    }
+    ++seq;
+    const double alpha = tot[0];
+    if (roww) {
+      x = fma(alpha, p, x);
+      r = fma(-alpha, y, r);
+      z = di * r;
+    }
+    if (!sums_rz()) {
+      t2_res_leave(d);
+      return;
+    }
+    rtag = seq;
+    ++seq;
+    rn2 = tot[0];
+    if (rn2 < thr) break;
+    halo_ahead(rtag);
+    const double rz_old = rz;
+    rz = tot[1];
+    if (warp == 3) {
+      const double b = quotient_by(rz, rz_old, rr_z);
+      if (lane == 0) beta_s = b;
+    }
+    __syncthreads();
+    beta = beta_s;
+    ++it;
+  }
+  if (live) d.dx[dof] = x;
+  if (bk == 0 && threadIdx.x == 0) {
+    d.scal[SC_CG_IT] = it;
+    d.scal[SC_CG_RN2] = rn2;
+    d.scal[SC_CG_B2] = b2;
+    d.res_seq[0] = seq;
+  }
+}
+
 // MixedStretch::solve (mixed_stretch.cpp:243-259): Jdx = -vol Jloc dx,
 // lambda = -gl + Htil dSdF^T Jdx, ds = -H^-1 (Sym lambda + g).
 __global__ void __launch_bounds__(kThreads) t2_local(T2 d) {
@@ -928,8 +1398,10 @@ struct mfem_tri2d {
   struct Pending { int kernel, a, b; };
   std::vector<Pending> ev_pending;
   size_t ev_used = 0;
-  // blocks of the grid PCG (t2_pcg_grid), 0: the one-block t2_pcg
-  int pcg_grid = 0;
+  // blocks of the grid PCG (t2_pcg_grid), 0: the resident one, of res_grid
+  // blocks (t2_pcg_res2 up to 1024 free rows, t2_pcg_res above)
+  int pcg_grid = 0, res_grid = 0;
+  size_t res_smem = 0;
   // configuration
   int bdf = 1, max_newton = 5, ls_iters = 20, cg_iters = 500;
   double h = 0.0333, cg_tol = 1e-4, newton_tol = 1e-10, res_tol = 0, load_norm = 0;
@@ -1095,6 +1567,8 @@ void bc_step(mfem_tri2d& sc, double dt) {
     if ((expr) != cudaSuccess) return MFEM_ERR_CUDA; \
   } while (0)
 
+const void* t2_res_kernel(bool two_red) { return two_red ? (const void*)t2_pcg_res2 : (const void*)t2_pcg_res; }
+
 int launch_status() { return cudaGetLastError() == cudaSuccess ? MFEM_OK : MFEM_ERR_CUDA; }
 
 // An event of the scene's pool (created on first use, reused after each
@@ -1204,8 +1678,17 @@ int t2_step(mfem_tri2d& sc, mfem_step_stats* out) {
       });
       T2_CUDA(e);
     } else if (sc.nf > 0) {
-      launch(sc, MFEM_T2_K_PCG,
-             [&] { t2_pcg<<<1, kBlock, 0, sc.stream>>>(sc.d, sc.cg_iters, sc.cg_tol); });
+      T2_CUDA(cudaMemsetAsync(sc.d.bar, 0, 4 * sizeof(unsigned int), sc.stream));
+      cudaError_t e = cudaSuccess;
+      launch(sc, MFEM_T2_K_PCG, [&] {
+        T2 dd = sc.d;
+        int mi = sc.cg_iters;
+        double tl = sc.cg_tol;
+        void* args[] = {&dd, &mi, &tl};
+        e = cudaLaunchCooperativeKernel(t2_res_kernel(sc.nf <= 1024), dim3(sc.res_grid), dim3(kResThreads), args,
+                                        sc.res_smem, sc.stream);
+      });
+      T2_CUDA(e);
     }
     launch(sc, MFEM_T2_K_LOCAL, [&] { t2_local<<<grid_of(sc.nt), kThreads, 0, sc.stream>>>(sc.d); });
     if (launch_status() != MFEM_OK) return MFEM_ERR_CUDA;
@@ -1471,6 +1954,81 @@ int mfem_gpu_tri2d_create(const mfem_tri2d_desc* dsc, mfem_tri2d** out) {
                                        : std::vector<double>(2 * size_t(nv), 0.0);
 
   // one device allocation
+  // The resident PCG's blocks.  Up to 1024 free rows: the two-reduction form
+  // over a power of two of blocks with at most 32 rows each, every grid-th row.
+  // More: the single-reduction form over blocks of up to 64 consecutive rows.
+  const bool two_red = nf <= 1024;
+  int res_grid = 0, res_rows = 32, res_first = 1, res_stride = 1;
+  size_t res_smem = 0;
+  std::vector<int> res_slot(1, 0), res_hptr(1, 0), res_hcol;
+  std::vector<uint16_t> res_lidx;
+  if (nf > 0) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return MFEM_ERR_CUDA;
+    if (two_red) {
+      res_grid = 1;
+      while (32 * res_grid < nf) res_grid *= 2;
+      res_stride = res_grid;
+    } else {
+      res_grid = std::min((nf + 63) / 64, kT2MaxGrid);
+      res_rows = (nf + res_grid - 1) / res_grid;
+      res_first = res_rows;
+    }
+    const int nsl = (res_rows + 31) / 32;
+    bool fits = res_rows <= kResOwn;
+    std::vector<int> local(nf, -1);
+    for (int b = 0; b < res_grid && fits; ++b) {
+      const int h0 = int(res_hcol.size());
+      auto row_of = [&](int i) { return i < res_rows ? res_first * b + res_stride * i : nf; };
+      for (int i = 0; i < res_rows; ++i)
+        if (row_of(i) < nf) local[row_of(i)] = i;
+      for (int s = 0; s < nsl; ++s) {
+        int len = 0;
+        for (int l = 0; l < 32; ++l) {
+          const int r = row_of(32 * s + l);
+          if (r < nf) len = std::max(len, sc->b_ptr[r + 1] - sc->b_ptr[r]);
+        }
+        const size_t at = res_lidx.size();
+        res_lidx.resize(at + 32 * size_t(len));
+        for (int l = 0; l < 32; ++l) {
+          const int r = row_of(32 * s + l);
+          for (int k = 0; k < len; ++k) {
+            int c = 32 * s + l;  // past the row's end: the row itself, with a zero block
+            if (r < nf && sc->b_ptr[r] + k < sc->b_ptr[r + 1]) {
+              int& q = local[sc->b_col[sc->b_ptr[r] + k]];
+              if (q < 0) {
+                q = kResOwn + int(res_hcol.size()) - h0;
+                res_hcol.push_back(sc->b_col[sc->b_ptr[r] + k]);
+              }
+              c = q;
+            }
+            if (c > 65535) fits = false;
+            res_lidx[at + 32 * size_t(k) + l] = uint16_t(c & 65535);
+          }
+        }
+        res_slot.push_back(res_slot.back() + len);
+      }
+      for (int j = h0; j < int(res_hcol.size()); ++j) local[res_hcol[j]] = -1;
+      for (int i = 0; i < res_rows; ++i)
+        if (row_of(i) < nf) local[row_of(i)] = -1;
+      res_hptr.push_back(int(res_hcol.size()));
+      res_smem = std::max(res_smem, t2_res_smem(size_t(res_slot[(b + 1) * nsl] - res_slot[b * nsl]),
+                                                size_t(res_hptr[b + 1] - res_hptr[b])));
+    }
+    int per_sm = 0;
+    constexpr size_t kMaxSmem = 220 * 1024;
+    if (!fits || res_smem > kMaxSmem ||
+        cudaFuncSetAttribute(t2_res_kernel(two_red), cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxSmem)) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, t2_res_kernel(two_red), kResThreads, res_smem) !=
+            cudaSuccess ||
+        long(per_sm) * sms < res_grid) {
+      cudaGetLastError();
+      res_grid = 0;
+    }
+  }
   Layout L;
   const size_t o_tri = L.take<int>(3 * size_t(nt)), o_dX = L.take<double>(6 * size_t(nt)),
                o_vol = L.take<double>(nt), o_mu = L.take<double>(nt), o_la = L.take<double>(nt),
@@ -1496,6 +2054,11 @@ int mfem_gpu_tri2d_create(const mfem_tri2d_desc* dsc, mfem_tri2d** out) {
                o_q = L.take<double>(2 * size_t(std::max(nf, 1))),
                o_sr = L.take<double>(12 * size_t(std::max(nf, 1))), o_part = L.take<double>(3 * kT2MaxGrid),
                o_bar = L.take<unsigned int>(4),
+               o_rslot = L.take<int>(res_slot.size()), o_rhp = L.take<int>(res_hptr.size()),
+               o_rhc = L.take<int>(std::max<size_t>(res_hcol.size(), 1)),
+               o_rli = L.take<uint16_t>(std::max<size_t>(res_lidx.size(), 1)),
+               o_rrec = L.take<uint4>(12 * size_t(std::max(res_grid, 1))),
+               o_rpub = L.take<uint4>(4 * size_t(std::max(nf, 1))), o_rseq = L.take<unsigned int>(1),
                o_ep = L.take<double>(2 * size_t(nt) + nv), o_scal = L.take<double>(SC_COUNT),
                o_st = L.take<int>(4), o_xh = L.take<double>(2 * size_t(nv) * sc->bdf),
                o_vh = L.take<double>(2 * size_t(nv) * sc->bdf), o_xs = L.take<double>(2 * size_t(nv));
@@ -1510,9 +2073,9 @@ int mfem_gpu_tri2d_create(const mfem_tri2d_desc* dsc, mfem_tri2d** out) {
   }
   char* base = sc->dev;
   if (cudaMemsetAsync(base, 0, total, sc->stream) != cudaSuccess) return MFEM_ERR_CUDA;
-  // sheets with more free rows than the one-block PCG can carry (one row a
-  // thread) iterate over co-resident blocks of at least 64 rows each
-  if (nf > kBlock) {
+  // sheets that do not fit the resident PCG iterate over co-resident blocks
+  // of at least 64 rows each
+  if (nf > 0 && res_grid == 0) {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -1571,6 +2134,19 @@ int mfem_gpu_tri2d_create(const mfem_tri2d_desc* dsc, mfem_tri2d** out) {
   d.sr = dp(o_sr);
   d.part = dp(o_part);
   d.bar = reinterpret_cast<unsigned int*>(base + o_bar);
+  sc->res_smem = res_smem;
+  sc->res_grid = res_grid;
+  d.res_first = res_first;
+  d.res_stride = res_stride;
+  d.res_rows = res_rows;
+  d.res_slot = ip(o_rslot);
+  d.res_hptr = ip(o_rhp);
+  d.res_hcol = ip(o_rhc);
+  d.res_lidx = reinterpret_cast<uint16_t*>(base + o_rli);
+  d.res_recs = reinterpret_cast<uint4*>(base + o_rrec);
+  d.res_pub = reinterpret_cast<uint4*>(base + o_rpub);
+  d.res_seq = reinterpret_cast<unsigned int*>(base + o_rseq);
+  const unsigned int first_tag = 1;  // the records start with tag 0
   d.epart = dp(o_ep);
   d.scal = dp(o_scal);
   d.status = ip(o_st);
@@ -1591,7 +2167,9 @@ int mfem_gpu_tri2d_create(const mfem_tri2d_desc* dsc, mfem_tri2d** out) {
             up(o_mval, m_val.data(), 8 * m_val.size()) && up(o_bptr, sc->b_ptr.data(), 4 * sc->b_ptr.size()) &&
             up(o_bcol, sc->b_col.data(), 4 * sc->b_col.size()) && up(o_bmass, b_mass.data(), 8 * b_mass.size()) &&
             up(o_cptr, c_ptr.data(), 4 * c_ptr.size()) && up(o_cent, c_ent.data(), 4 * c_ent.size()) &&
-            up(o_iptr, i_ptr.data(), 4 * i_ptr.size()) && up(o_ient, i_ent.data(), 4 * i_ent.size());
+            up(o_rslot, res_slot.data(), 4 * res_slot.size()) && up(o_rhp, res_hptr.data(), 4 * res_hptr.size()) &&
+            up(o_rhc, res_hcol.data(), 4 * res_hcol.size()) && up(o_rli, res_lidx.data(), 2 * res_lidx.size()) &&
+            up(o_rseq, &first_tag, 4) && up(o_iptr, i_ptr.data(), 4 * i_ptr.size()) && up(o_ient, i_ent.data(), 4 * i_ent.size());
   // the BDF history: every slot holds (x0, v0)
   for (int i = 0; i < sc->bdf && ok; ++i)
     ok = up(o_xh + 8 * 2 * size_t(nv) * i, sc->V.data(), 8 * 2 * size_t(nv)) &&
