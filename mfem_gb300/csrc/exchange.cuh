@@ -81,4 +81,45 @@ __device__ __forceinline__ bool poll_recs(uint4 (&v)[N], const Ptr& at, const bo
   }
 }
 
+// Copies of each partial sum's record: blocks poll the copy of their number
+// modulo the copies, since records that every block polls queue up in L2.
+// An exchange of two sums between 34 / 66 / 117 / 152 blocks alone took 2421 /
+// 4956 / 7657 / 8758 cycles with one copy, 2701 / 3201 / 3392 / 3395 with
+// eight (and 2422 / 2868 / 3839 / 4789 with a copy for every block); a solve's
+// iteration 6.13 / 7.53 us with one / eight copies at 34 / 117 blocks against
+// 6.67 with two at 34 and 8.9 with one at 117.
+constexpr int kMaxCopies = 8;
+__host__ __device__ constexpr int exchange_copies(int blocks) { return blocks > 40 ? kMaxCopies : 1; }
+
+// n records of one quantity summed by the calling warp (valid in lane 0):
+// lane l over records l, l + 32, ..; then a tree.  ok is cleared when a wait ran out.
+__device__ __forceinline__ double fetch_sum(const uint4* rec, int n, unsigned seq, int* err, bool& ok) {
+  const int lane = threadIdx.x & 31;
+  double v = 0.0;
+  for (int i0 = 0; i0 < n && ok; i0 += 128) {
+    uint4 g[4];
+    bool want[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      want[j] = i0 + 32 * j + lane < n;
+      if (want[j]) g[j] = ld_rec(rec + i0 + 32 * j + lane);
+    }
+    ok = poll_recs<4>(g, [&](int j) { return rec + i0 + 32 * j + lane; }, want, seq, err);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v += want[j] ? rec_double(g[j]) : 0.0;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+  return v;
+}
+
+// num / den for a den whose correctly rounded reciprocal is at hand: one
+// product and one correction of the remainder give the correctly rounded
+// quotient (Markstein 1990), in 3 instead of the division's 9 latencies.
+__device__ __forceinline__ double quotient_by(double num, double den, double rcp) {
+  const double q = num * rcp;
+  const double v = fma(fma(-den, q, num), rcp, q);
+  return isfinite(v) ? v : num / den;
+}
+
 }  // namespace mfem_gpu

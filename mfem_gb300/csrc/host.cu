@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "../../include/mfem_gb300.h"
+#include "exchange.cuh"
 #include "kernels.cuh"
 #include "resident.cuh"
 
@@ -986,7 +987,7 @@ bool cgr_plan(mfem_batch* b) {
     a.blocks = A.take<CgrBlock>(blocks.size());
     a.h_col = A.take<int>(std::max<size_t>(h_col.size(), 1));
     a.lidx = A.take<uint16_t>(std::max<size_t>(lidx.size(), 1));
-    a.recs = A.take<uint4>(6 * (size_t)nrec);
+    a.recs = A.take<uint4>(2 * kMaxCopies * 3 * (size_t)nrec);
     a.pub = A.take<uint4>(2 * pub);
     a.seq = A.take<unsigned int>(n);
   };

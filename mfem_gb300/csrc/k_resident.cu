@@ -87,7 +87,14 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int par = seq & 1;
   const bool tiles = B.tile != 0;
-  uint4* rec = A.recs + (size_t)(par * 3) * A.nrec_total + B.rec0;
+  const int copies = exchange_copies(B.nblk);
+  const size_t cstride = 3 * (size_t)A.nrec_total;
+  uint4* rec = A.recs + par * kMaxCopies * cstride + B.rec0;
+  // lane 0's value as every copy of record i of quantity q (the whole warp)
+  auto send = [&](int q, int i, E val) {
+    const E a = shfl_to(val, 0);
+    if (lane < copies) st_rec(rec + lane * cstride + (size_t)q * A.nrec_total + i, rec_of(a, seq));
+  };
   if (lead) tree<E, NQ, 16>(v);
   if (tiles) {
     if (lead && lane == 0)
@@ -106,18 +113,18 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
     if (warp < NQ) {
       E a[1] = {lane < B.nsl ? Slot<E>::sget(&S.part[par][warp][lane]) : E(0)};
       tree<E, 1, 4>(a);
-      if (lane == 0) st_rec(rec + (size_t)warp * A.nrec_total + B.rec, rec_of(a[0], seq));
+      send(warp, B.rec, a[0]);
     }
-  } else if (lead && lane == 0) {
+  } else if (lead) {
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) st_rec(rec + (size_t)q * A.nrec_total + B.rec + sl, rec_of(v[q], seq));
+    for (int q = 0; q < NQ; ++q) send(q, B.rec + sl, v[q]);
   }
   const int n = B.nrec;
   // the sums of record i (0 for lanes without one), the warp in step
   auto fetch = [&](int i, E (&a)[NQ]) -> bool {
     uint4 w[NQ];
     bool want[NQ];
-    const uint4* src = rec + min(i, n - 1);
+    const uint4* src = rec + (B.rec % copies) * cstride + min(i, n - 1);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
       want[q] = i < n;

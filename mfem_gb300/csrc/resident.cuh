@@ -27,7 +27,7 @@ struct CgrArgs {
   const CgrBlock* blocks;
   const int* h_col;
   const uint16_t* lidx;
-  uint4* recs;        // [parity][quantity 0..2][nrec_total] tagged partial sums
+  uint4* recs;        // [parity][copy][quantity 0..2][nrec_total] tagged partial sums
   uint4* pub;         // [parity][rows (x 3 in FP64)] tagged vector
   int nrec_total;
   size_t pub_stride;  // records of one parity of pub

@@ -56,6 +56,7 @@
 namespace {
 
 using mfem_gpu::psd_fix_n;
+using mfem_gpu::quotient_by;
 
 constexpr int kThreads = 128;
 constexpr int kBlock = 1024;  // the single-block kernels (sums)
@@ -123,7 +124,7 @@ struct T2 {
   const int* res_hptr;         // blocks + 1
   const int* res_hcol;
   const uint16_t* res_lidx;    // 32 per slot
-  uint4* res_recs;             // [parity][3][2 blocks]
+  uint4* res_recs;             // [parity][copy][3][2 blocks]
   uint4* res_pub;              // [parity][2 nf]
   unsigned int* res_seq;
   double* epart;  // 2 nt + nv energy parts
@@ -715,15 +716,6 @@ __global__ void __launch_bounds__(kGridThreads) t2_pcg_grid(T2 d, int max_iter, 
 constexpr int kResThreads = 256;
 constexpr int kResOwn = 64;  // local indices of a block's own rows; its halo follows
 
-// num / den for a den whose correctly rounded reciprocal is at hand: one
-// product and one correction of the remainder give the correctly rounded
-// quotient (Markstein 1990), in 3 instead of the division's 9 latencies.
-__device__ __forceinline__ double quotient_by(double num, double den, double rcp) {
-  const double q = num * rcp;
-  const double v = fma(fma(-den, q, num), rcp, q);
-  return isfinite(v) ? v : num / den;
-}
-
 // A block's rows, halo and matrix.  mat: [slot][4][32] doubles per slice,
 // li: [slot][32] local column indices.
 struct T2Block {
@@ -786,29 +778,6 @@ __device__ __forceinline__ double t2_res_mul(const T2Block& B, int s_at, int s_l
     y = __dadd_rn(y, fma(m[128 * k], uc.x, __dmul_rn(m[128 * k + 32], uc.y)));
   }
   return y;
-}
-
-// n records of one quantity summed by the calling warp: lane l over records
-// l, l + 32, ..; then a tree.  ok is cleared when a wait ran out.
-__device__ __forceinline__ double t2_res_fetch(const uint4* rec, int n, unsigned seq, int* err, bool& ok) {
-  using namespace mfem_gpu;
-  const int lane = threadIdx.x & 31;
-  double v = 0.0;
-  for (int i0 = 0; i0 < n && ok; i0 += 128) {
-    uint4 g[4];
-    bool want[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      want[j] = i0 + 32 * j + lane < n;
-      if (want[j]) g[j] = ld_rec(rec + i0 + 32 * j + lane);
-    }
-    ok = poll_recs<4>(g, [&](int j) { return rec + i0 + 32 * j + lane; }, want, seq, err);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v += want[j] ? rec_double(g[j]) : 0.0;
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-  return v;
 }
 
 __device__ __forceinline__ void t2_res_leave(const T2& d) {
@@ -896,13 +865,15 @@ __global__ void __launch_bounds__(kResThreads) t2_pcg_res(T2 d, int max_iter, do
     __syncthreads();
     if (task >= 0 && ts == 0) {
       const double v = B.nsl > 1 ? half[q][0] + half[q][1] : half[q][0];
-      uint4* rec = d.res_recs + ((size_t)(seq & 1) * 3 + q) * G;
+      uint4* rec = d.res_recs + ((size_t)(seq & 1) * kMaxCopies * 3 + q) * 2 * G;
       double t = v;
       if (G > 1) {
-        if (lane == 0) st_rec(rec + bk, rec_of(v, seq));
+        const int copies = exchange_copies(G);
+        if (lane < copies) st_rec(rec + (size_t)lane * 6 * G + bk, rec_of(v, seq));
+        rec += (size_t)(bk % copies) * 6 * G;
         bool ok = true;
         if (task < 2) beside();  // owners (warps 2, 3)
-        t = t2_res_fetch(rec, G, seq, err, ok);
+        t = fetch_sum(rec, G, seq, err, ok);
         if (!ok && lane == 0) atomicOr(&flags, 1);
       } else if (task < 2) {
         beside();
@@ -1073,15 +1044,16 @@ __global__ void __launch_bounds__(kResThreads) t2_pcg_res2(T2 d, int max_iter, d
     if (G == 1) {
       return dofs ? __shfl_sync(0xffffffffu, e0 + e1, 0) : __shfl_sync(0xffffffffu, e0, 0);
     }
-    uint4* rec = d.res_recs + ((size_t)(seq & 1) * 3 + q) * 2 * G;
-    if (lane == 0) {
-      if (dofs) {
-        st_rec(rec + 2 * bk, rec_of(e0, seq));
-        st_rec(rec + 2 * bk + 1, rec_of(e1, seq));
-      } else {
-        st_rec(rec + bk, rec_of(e0, seq));
-      }
+    uint4* rec = d.res_recs + ((size_t)(seq & 1) * kMaxCopies * 3 + q) * 2 * G;
+    const int copies = exchange_copies(G);
+    e0 = __shfl_sync(0xffffffffu, e0, 0);
+    if (dofs) e1 = __shfl_sync(0xffffffffu, e1, 0);
+    if (lane < copies) {
+      uint4* to = rec + (size_t)lane * 6 * G + (dofs ? 2 * bk : bk);
+      st_rec(to, rec_of(e0, seq));
+      if (dofs) st_rec(to + 1, rec_of(e1, seq));
     }
+    rec += (size_t)(bk % copies) * 6 * G;
     // n <= 64 values: lane l holds values l and l + 32
     uint4 g[2];
     bool want[2];
@@ -2057,7 +2029,7 @@ int mfem_gpu_tri2d_create(const mfem_tri2d_desc* dsc, mfem_tri2d** out) {
                o_rslot = L.take<int>(res_slot.size()), o_rhp = L.take<int>(res_hptr.size()),
                o_rhc = L.take<int>(std::max<size_t>(res_hcol.size(), 1)),
                o_rli = L.take<uint16_t>(std::max<size_t>(res_lidx.size(), 1)),
-               o_rrec = L.take<uint4>(12 * size_t(std::max(res_grid, 1))),
+               o_rrec = L.take<uint4>(12 * mfem_gpu::kMaxCopies * size_t(std::max(res_grid, 1))),
                o_rpub = L.take<uint4>(4 * size_t(std::max(nf, 1))), o_rseq = L.take<unsigned int>(1),
                o_ep = L.take<double>(2 * size_t(nt) + nv), o_scal = L.take<double>(SC_COUNT),
                o_st = L.take<int>(4), o_xh = L.take<double>(2 * size_t(nv) * sc->bdf),
