@@ -350,9 +350,10 @@ int mfem_gpu_scene_pcg(mfem_scene* scene, const double* b, double* dx,
  * nnzb, val 9*nnzb row-major blocks, all FP64), solving A x = b from x = 0
  * with the stopping rule of mfem_gpu_scene_pcg: |r|^2 < tol^2 |b|^2, or
  * MFEM_ERR_CG_MAXITER after max_iters iterations.  It calls no allocator:
- * its scratch (five vectors, the inverted diagonal blocks, tile partials,
- * tickets and scalars, about 6 MiB) is one static __device__ array sized for
- * MFEM_NOALLOC_PCG_MAX_ROWS block rows; larger systems are rejected with
+ * its scratch (vectors, the inverted diagonal blocks, partial sums, the
+ * records its blocks exchange, about 8 MiB) is one static __device__ array
+ * sized for MFEM_NOALLOC_PCG_MAX_ROWS block rows; larger systems are rejected
+ * with
  * MFEM_ERR_CAPACITY.  It exists for callers that must not allocate device
  * memory at solve time: a host framework that hands out all device memory
  * from its own budget or pool, or a real-time loop where cudaMalloc's
@@ -360,8 +361,10 @@ int mfem_gpu_scene_pcg(mfem_scene* scene, const double* b, double* dx,
  * The first call on a device (with that device current) looks up the
  * scratch address with cudaGetSymbolAddress; that first call should come
  * before any stream capture.  Every call waits for its stream
- * (cudaStreamSynchronize) and copies the solver's scalars to the host
- * between chunks of iterations.  Calls on one device share the scratch,
+ * (cudaStreamSynchronize).  A system whose blocks fit shared memory is solved
+ * in one cooperative launch (a wait between its blocks that runs out returns
+ * MFEM_ERR_TIMEOUT); any other in chunks of iterations, the solver's scalars
+ * copied to the host between them.  Calls on one device share the scratch,
  * so overlapping calls would race: they are serialised by a per-device
  * lock held until the call's stream has drained.  All
  * pointers must be device memory of the current device; `stream` is a
