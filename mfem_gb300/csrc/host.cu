@@ -890,12 +890,14 @@ int worst_status(const SceneScalars& sc) {
 // Blocks of the resident solve for the whole batch (resident.cuh).  FP32: a
 // reduction tile of eight slices each (39k tets, 34 tiles: 6.5 us an
 // iteration, against 7.9 / 8.2 / 14.7 us with 4 / 2 / 1 slices, whose halos
-// overlap more and whose exchange has more records).  FP64: as few slices as
+// overlap more and whose exchange has more records); more tiles than SMs:
+// as many neighbouring pairs of tiles as it takes go to one block, those of a
+// scene's short last tile first (320k tets, 263 tiles: 12.9 us, against 15.2 us
+// with two blocks an SM and 25.4 us for the launches); a scene of two tiles
+// alone is one block (350 rows: 6.2 us, against 8.2 us with two).  FP64: as few slices as
 // leave every block an SM of its own, for the multiplication's 64-cycle
-// instructions (5,400 tets: 11.9 / 11.9 / 16.0 us with 1 / 2 / 4).  Above one
-// block an SM, two share it, each with half the shared memory (320k tets, 263
-// tiles: 17.2 us against 26.5 us for the launches).  False: the batch does not
-// fit, or its form has no resident kernel.
+// instructions (5,400 tets: 11.9 / 11.9 / 16.0 us with 1 / 2 / 4).  False: the
+// batch does not fit, or its form has no resident kernel.
 bool cgr_plan(mfem_batch* b) {
   if (b->cgr_state != 0) return b->cgr_state > 0;
   b->cgr_state = -1;
@@ -908,16 +910,48 @@ bool cgr_plan(mfem_batch* b) {
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
     return false;
   const int n = (int)b->scenes.size();
-  auto count = [&](int spb) {
-    long c = 0;
-    for (mfem_scene* s : b->scenes) c += ((s->M.nf + 31) / 32 + spb - 1) / spb;
-    return c;
-  };
+  // first slice of every block, per scene
+  std::vector<std::vector<int>> first(n);
   int spb = fp64 ? 1 : kCgrTile;
-  while (fp64 && spb < kCgrMaxSpb64 && count(spb) > sms) spb *= 2;
-  const bool two = count(spb) > sms;
-  if (count(spb) > 2 * sms) return false;
-  const size_t budget = two ? kCgrSmemTwo : kCgrSmemOne;
+  long total = 0;
+  for (;; spb *= 2) {
+    total = 0;
+    for (int i = 0; i < n; ++i) {
+      first[i].clear();
+      for (int s = 0; s < (b->scenes[i]->M.nf + 31) / 32; s += spb) first[i].push_back(s);
+      total += (long)first[i].size();
+    }
+    if (!fp64 || total <= sms || spb >= kCgrMaxSpb64) break;
+  }
+  if (!fp64 && total > sms) {
+    if (total > 2 * sms) return false;
+    struct Pair { int slices, scene, block; };
+    std::vector<Pair> pairs;
+    for (int i = 0; i < n; ++i) {
+      const int ns = (b->scenes[i]->M.nf + 31) / 32, nb = (int)first[i].size();
+      for (int k = nb - 2; k >= 0; k -= 2) pairs.push_back({std::min(ns - 8 * k, 16), i, k});
+    }
+    std::stable_sort(pairs.begin(), pairs.end(), [](const Pair& p, const Pair& q) { return p.slices < q.slices; });
+    if ((long)pairs.size() < total - sms) return false;
+    pairs.resize(total - sms);
+    std::vector<std::vector<char>> gone(n);
+    for (int i = 0; i < n; ++i) gone[i].assign(first[i].size(), 0);
+    for (const Pair& p : pairs) gone[p.scene][p.block + 1] = 1;
+    for (int i = 0; i < n; ++i) {
+      std::vector<int> keep;
+      for (size_t k = 0; k < first[i].size(); ++k)
+        if (!gone[i][k]) keep.push_back(first[i][k]);
+      first[i] = keep;
+    }
+    total = sms;
+    spb = 2 * kCgrTile;
+  }
+  if (total > sms) return false;
+  if (n == 1 && !fp64 && total == 2) {  // no exchange at all
+    first[0].pop_back();
+    spb = 2 * kCgrTile;
+    total = 1;
+  }
   std::vector<CgrBlock> blocks;
   std::vector<int> h_col;
   std::vector<uint16_t> lidx;
@@ -926,20 +960,21 @@ bool cgr_plan(mfem_batch* b) {
   for (int i = 0; i < n; ++i) {
     const HostMesh& M = b->scenes[i]->M;
     if (M.nf == 0) return false;
-    const int ns = (M.nf + 31) / 32, nblk = (ns + spb - 1) / spb;
-    const bool tile = spb == kCgrTile || nblk == 1;
+    const int ns = (M.nf + 31) / 32, nblk = (int)first[i].size();
+    const bool tile = spb >= kCgrTile || nblk == 1;
+    const int ntile = (ns + kCgrTile - 1) / kCgrTile;
     if (!tile && (ns + kCgrTile - 1) / kCgrTile > kCgrMaxSliceTiles) return false;
     std::vector<int> local(M.nf, -1);
     for (int k = 0; k < nblk; ++k) {
       CgrBlock B{};
       B.scene = i;
-      B.slice0 = k * spb;
-      B.nsl = std::min(spb, ns - B.slice0);
+      B.slice0 = first[i][k];
+      B.nsl = (k + 1 < nblk ? first[i][k + 1] : ns) - B.slice0;
       B.hoff = (int)h_col.size();
       B.loff = (int)lidx.size();
       B.rec0 = nrec;
-      B.nrec = tile ? nblk : ns;
-      B.rec = tile ? k : B.slice0;
+      B.nrec = tile ? ntile : ns;
+      B.rec = tile ? B.slice0 / kCgrTile : B.slice0;
       B.row0 = (int)rows;
       B.nblk = nblk;
       B.tile = tile ? 1 : 0;
@@ -968,17 +1003,16 @@ bool cgr_plan(mfem_batch* b) {
         return t;
       };
       int kres = kMaxRowBlocks + 1;
-      while (kres >= 0 && cgr_smem(fp64, fused, b->jacobi, slots(kres), own, B.nh) > budget) --kres;
+      while (kres >= 0 && cgr_smem(fp64, fused, b->jacobi, slots(kres), own, B.nh) > kCgrSmem) --kres;
       if (kres < 0) return false;
       B.kres = kres;
       smem = std::max(smem, cgr_smem(fp64, fused, b->jacobi, slots(kres), own, B.nh));
       blocks.push_back(B);
     }
-    nrec += tile ? nblk : ns;
+    nrec += tile ? ntile : ns;
     rows += M.nf;
   }
-  // blocks that can have an SM each are kept from sharing one
-  if (!two) smem = std::max(smem, kCgrSmemTwo + 8 * 1024);
+  smem = std::max(smem, kCgrSmem / 2 + 8 * 1024);  // every block an SM of its own
   const int threads = cgr_threads(fp64, spb);
   if ((long)cgr_blocks_per_sm(fp64, fused, b->jacobi, threads, smem) * sms < (long)blocks.size()) return false;
   const size_t pub = rows * (fp64 ? 3 : 1);
@@ -1389,8 +1423,10 @@ int batch_step_impl(mfem_batch* b, mfem_step_stats* stats) {
 
 int upload_sds(mfem_batch* b);
 
-// PCG iterations of one tick when they run as one resident launch.
-constexpr int kTickResident = 64;
+// PCG iterations of one tick when they run as one resident launch: 16 scenes
+// of 1.4k to 29k tets, three steps, take 39.1 / 37.2 / 35.8 / 37.1 ms with 32 /
+// 64 / 128 / 256 (and 58 ms with 16 launches of k_cgf_iter a tick).
+constexpr int kTickResident = 128;
 
 // One tick of the ticked multi-step form as a CUDA graph over the current
 // tables: every kernel of a Newton iteration once, each acting on the

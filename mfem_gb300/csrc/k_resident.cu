@@ -6,7 +6,7 @@
 // (k_cg_spmv, k_cg_update) or per iteration (k_cgf_iter) then costs is the
 // chain of latencies: launch boundaries, a row's slots walked one after
 // another (column -> gather -> FMA), tile tickets, a serial finalizer.  Here
-// each block owns up to eight 32-row slices for the whole solve and
+// each block owns up to sixteen 32-row slices for the whole solve and
 //   * copies its slices' blocks to shared memory once, as nine planes of 32
 //     lanes per slot, and keeps its rows' vectors in registers;
 //   * knows its halo, the distinct columns outside its rows (built by the
@@ -76,8 +76,8 @@ struct CgrShared {
 // in the block); the order is that of tile_partials and scene_sums: a tree
 // over a slice's 32 rows, a tree over the 8 slices of a tile, each thread over
 // tiles i, i + 256, .., a tree over 32 such sums, a tree over 8.  (Their
-// trees over absent entries only add zeros.)  A block of eight slices sends
-// its tile's sum, a smaller one its slices' sums, a scene of one block
+// trees over absent entries only add zeros.)  A block of one or two tiles
+// sends their sums, a smaller one its slices' sums, a scene of one block
 // nothing.  `ahead` runs once the other blocks' sums have come in, before the
 // last of the adding: loads issued there are under way meanwhile.  False: a
 // wait ran out.
@@ -101,19 +101,24 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
 #pragma unroll
       for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.part[par][q][sl], v[q]);
     __syncthreads();
+    const int nt = (B.nsl + kCgrTile - 1) / kCgrTile;  // 1 or 2
     if (B.nblk == 1) {
 #pragma unroll
       for (int q = 0; q < NQ; ++q) v[q] = lane < B.nsl ? Slot<E>::sget(&S.part[par][q][lane]) : E(0);
-      tree<E, NQ, 4>(v);
+      tree<E, NQ, 4>(v);  // the tiles' sums in lanes 0 and 8
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) v[q] = shfl_to(v[q], 0);
+      for (int q = 0; q < NQ; ++q) {
+        if (nt > 1) v[q] = radd(v[q], shfl_to(v[q], 8));
+        v[q] = shfl_to(v[q], 0);
+      }
       ahead();
       return true;
     }
-    if (warp < NQ) {
-      E a[1] = {lane < B.nsl ? Slot<E>::sget(&S.part[par][warp][lane]) : E(0)};
+    if (warp < NQ * nt) {
+      const int q = warp / nt, t = warp % nt, at = kCgrTile * t + lane;
+      E a[1] = {lane < kCgrTile && at < B.nsl ? Slot<E>::sget(&S.part[par][q][at]) : E(0)};
       tree<E, 1, 4>(a);
-      send(warp, B.rec, a[0]);
+      send(q, B.rec + t, a[0]);
     }
   } else if (lead) {
 #pragma unroll
@@ -124,7 +129,7 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
   auto fetch = [&](int i, E (&a)[NQ]) -> bool {
     uint4 w[NQ];
     bool want[NQ];
-    const uint4* src = rec + (B.rec % copies) * cstride + min(i, n - 1);
+    const uint4* src = rec + (blockIdx.x % copies) * cstride + min(i, n - 1);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
       want[q] = i < n;
@@ -319,8 +324,8 @@ constexpr int kHaloRegs = 4;  // halo columns a thread keeps in registers
 // the exchanged vector is z, and each block keeps p at its halo.  In FP64 a
 // row is three threads' (one component each), and the lead thread (component
 // 0) forms the row's share of the inner products in component order.
-template <typename Real, int kThreads, int kMinBlocks>
-__global__ void __launch_bounds__(kThreads, kMinBlocks) k_cgr_split(const CgrArgs A) {
+template <typename Real, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
   using E = typename Ext<Real>::T;
   constexpr bool k64 = sizeof(Real) == 8;
   constexpr int NC = k64 ? 1 : 3;
@@ -673,9 +678,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_cgr_split(const CgrArg
 // iteration done: until the recursion's stop is to be verified (cgf_phase set:
 // the next launches of k_cgf_iter verify), or max_iters iterations.  The
 // exchanged vector is w; each block keeps r and s at its halo.
-template <bool kScaled>
-__global__ void __launch_bounds__(256, 1) k_cgr_fused(const CgrArgs A) {
-  constexpr int kThreads = 256;
+template <bool kScaled, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
   extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
   __shared__ CgrShared S;
   const CgrBlock B = A.blocks[blockIdx.x];
@@ -892,23 +896,21 @@ __global__ void __launch_bounds__(256, 1) k_cgr_fused(const CgrArgs A) {
   }
 }
 
-template <typename F> auto with_kernel(bool fp64, bool fused, bool jacobi, int threads, bool two, F&& f) {
-  if (fused) return jacobi ? f((const void*)k_cgr_fused<true>) : f((const void*)k_cgr_fused<false>);
-  if (fp64) return threads > 256 ? f((const void*)k_cgr_split<double, 384, 1>) : f((const void*)k_cgr_split<double, 256, 1>);
-  return two ? f((const void*)k_cgr_split<float, 256, 2>) : f((const void*)k_cgr_split<float, 256, 1>);
+template <typename F> auto with_kernel(bool fp64, bool fused, bool jacobi, int threads, F&& f) {
+  if (fused && threads > 256) return jacobi ? f((const void*)k_cgr_fused<true, 512>) : f((const void*)k_cgr_fused<false, 512>);
+  if (fused) return jacobi ? f((const void*)k_cgr_fused<true, 256>) : f((const void*)k_cgr_fused<false, 256>);
+  if (fp64) return threads > 256 ? f((const void*)k_cgr_split<double, 384>) : f((const void*)k_cgr_split<double, 256>);
+  return threads > 256 ? f((const void*)k_cgr_split<float, 512>) : f((const void*)k_cgr_split<float, 256>);
 }
-
-// Blocks of at most half an SM's shared memory come in pairs.
-bool cgr_pairs(size_t smem) { return smem <= kCgrSmemTwo; }
 
 }  // namespace
 
 int cgr_blocks_per_sm(bool fp64, bool fused, bool jacobi, int threads, size_t smem) {
-  return with_kernel(fp64, fused, jacobi, threads, cgr_pairs(smem), [&](const void* k) {
+  return with_kernel(fp64, fused, jacobi, threads, [&](const void* k) {
     int nb = 0;
     // the function's limit is shared by every batch: always the largest
-    if (smem > kCgrSmemOne ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgrSmemOne) != cudaSuccess ||
+    if (smem > kCgrSmem ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgrSmem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, smem) != cudaSuccess) {
       cudaGetLastError();
       return 0;
@@ -919,7 +921,7 @@ int cgr_blocks_per_sm(bool fp64, bool fused, bool jacobi, int threads, size_t sm
 
 cudaError_t launch_cgr(const CgrArgs& args, bool fp64, bool fused, bool jacobi, int nblocks, int threads, size_t smem,
                        cudaStream_t stream) {
-  return with_kernel(fp64, fused, jacobi, threads, cgr_pairs(smem), [&](const void* k) {
+  return with_kernel(fp64, fused, jacobi, threads, [&](const void* k) {
     CgrArgs a = args;
     void* params[] = {&a};
     return cudaLaunchCooperativeKernel(k, dim3(nblocks), dim3(threads), params, smem, stream);

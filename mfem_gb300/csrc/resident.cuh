@@ -20,7 +20,8 @@ struct CgrBlock {
   int rec;          // the block's first record among them
   int row0;         // the scene's first row in the exchanged vector
   int nblk;         // blocks of the scene
-  int tile;         // 1: the block is a reduction tile (8 slices) and sends its sum; 0: its slices' sums
+  int tile;         // 1: the block is one or two reduction tiles (of 8 slices) and sends their sums;
+                    // 0: it sends its slices' sums
 };
 
 struct CgrArgs {
@@ -38,7 +39,7 @@ struct CgrArgs {
 };
 
 constexpr int kCgrTile = kCgRows / 32;  // slices of a reduction tile
-constexpr int kCgrMaxSlices = 8;        // slices of a block
+constexpr int kCgrMaxSlices = 16;       // slices of a block
 constexpr int kCgrMaxSliceTiles = 96;   // reduction tiles of a scene whose blocks send slice sums
 
 // Dynamic shared memory of a block with `slots` resident slots, `own` rows
@@ -51,9 +52,8 @@ constexpr size_t cgr_smem(bool fp64, bool fused, bool jacobi, size_t slots, size
   if (fused) b += 16 * nh + (jacobi ? 0 : 16 * nh + 36 * nh);
   return b;
 }
-// Dynamic shared memory a block may take when one or two share an SM.
-constexpr size_t kCgrSmemOne = 223 * 1024 - 4096, kCgrSmemTwo = 105 * 1024;
-constexpr int cgr_threads(bool fp64, int spb) { return fp64 && spb > 2 ? 384 : 256; }
+constexpr size_t kCgrSmem = 218 * 1024;  // dynamic shared memory a block may take
+constexpr int cgr_threads(bool fp64, int spb) { return fp64 ? (spb > 2 ? 384 : 256) : (spb > 8 ? 512 : 256); }
 constexpr int kCgrMaxSpb64 = 4;  // three component warps a slice
 
 // Blocks per SM that can be resident with this much dynamic shared memory.
