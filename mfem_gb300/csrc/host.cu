@@ -894,10 +894,10 @@ int worst_status(const SceneScalars& sc) {
 // as many neighbouring pairs of tiles as it takes go to one block, those of a
 // scene's short last tile first (320k tets, 263 tiles: 12.9 us, against 15.2 us
 // with two blocks an SM and 25.4 us for the launches); a scene of two tiles
-// alone is one block (350 rows: 6.2 us, against 8.2 us with two).  FP64: as few slices as
-// leave every block an SM of its own, for the multiplication's 64-cycle
-// instructions (5,400 tets: 11.9 / 11.9 / 16.0 us with 1 / 2 / 4).  False: the
-// batch does not fit, or its form has no resident kernel.
+// alone is one block (350 rows: 6.2 us, against 8.2 us with two).  FP64: the
+// fewest slices of 1, 2 and 4 for which every block has an SM of its own, for
+// a slice's product is 3400 cycles of its SM's FP64 pipe.  False: the batch
+// does not fit, or its form has no resident kernel.
 bool cgr_plan(mfem_batch* b) {
   if (b->cgr_state != 0) return b->cgr_state > 0;
   b->cgr_state = -1;
@@ -961,9 +961,8 @@ bool cgr_plan(mfem_batch* b) {
     const HostMesh& M = b->scenes[i]->M;
     if (M.nf == 0) return false;
     const int ns = (M.nf + 31) / 32, nblk = (int)first[i].size();
-    const bool tile = spb >= kCgrTile || nblk == 1;
     const int ntile = (ns + kCgrTile - 1) / kCgrTile;
-    if (!tile && (ns + kCgrTile - 1) / kCgrTile > kCgrMaxSliceTiles) return false;
+    if (fp64 && ntile > kCgrMaxTiles64) return false;
     std::vector<int> local(M.nf, -1);
     for (int k = 0; k < nblk; ++k) {
       CgrBlock B{};
@@ -973,11 +972,11 @@ bool cgr_plan(mfem_batch* b) {
       B.hoff = (int)h_col.size();
       B.loff = (int)lidx.size();
       B.rec0 = nrec;
-      B.nrec = tile ? ntile : ns;
-      B.rec = tile ? B.slice0 / kCgrTile : B.slice0;
+      B.nrec = fp64 ? ns : ntile;
+      B.rec = fp64 ? B.slice0 : B.slice0 / kCgrTile;
       B.row0 = (int)rows;
       B.nblk = nblk;
-      B.tile = tile ? 1 : 0;
+      B.spb = spb;
       const int r0 = 32 * B.slice0, own = 32 * B.nsl, r1 = std::min(M.nf, r0 + own);
       // every slot's column as an index into the block's rows, then its halo
       for (int q = M.slice_off[B.slice0]; q < M.slice_off[B.slice0 + B.nsl]; ++q) {
@@ -1009,7 +1008,7 @@ bool cgr_plan(mfem_batch* b) {
       smem = std::max(smem, cgr_smem(fp64, fused, b->jacobi, slots(kres), own, B.nh));
       blocks.push_back(B);
     }
-    nrec += tile ? ntile : ns;
+    nrec += fp64 ? ns : ntile;
     rows += M.nf;
   }
   smem = std::max(smem, kCgrSmem / 2 + 8 * 1024);  // every block an SM of its own

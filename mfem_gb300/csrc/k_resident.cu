@@ -48,9 +48,6 @@ template <typename E> __device__ __forceinline__ E rec_val(uint4 v);
 template <> __device__ __forceinline__ df64 rec_val<df64>(uint4 v) {
   return df64(__uint_as_float(v.x), __uint_as_float(v.y));
 }
-template <> __device__ __forceinline__ double rec_val<double>(uint4 v) {
-  return rec_double(v);
-}
 
 __device__ __forceinline__ df64 shfl_to(df64 v, int lane) {
   return df64(__shfl_sync(0xffffffffu, v.hi, lane), __shfl_sync(0xffffffffu, v.lo, lane));
@@ -66,9 +63,8 @@ __device__ __forceinline__ void tree(E (&v)[NQ]) {
 }
 
 struct CgrShared {
-  double part[2][3][kCgrMaxSlices];      // the block's slice sums
-  double tp[2][3][kCgrMaxSliceTiles];    // tile sums (slice records)
-  double red[2][3][8];                   // warp sums of the tiles
+  double part[2][3][kCgrMaxSlices];  // the block's slice sums
+  double red[2][3][8];               // warp sums of the tiles
 };
 
 // Sums over the scene's rows, the same in every thread of every block.  v
@@ -76,17 +72,15 @@ struct CgrShared {
 // in the block); the order is that of tile_partials and scene_sums: a tree
 // over a slice's 32 rows, a tree over the 8 slices of a tile, each thread over
 // tiles i, i + 256, .., a tree over 32 such sums, a tree over 8.  (Their
-// trees over absent entries only add zeros.)  A block of one or two tiles
-// sends their sums, a smaller one its slices' sums, a scene of one block
-// nothing.  `ahead` runs once the other blocks' sums have come in, before the
-// last of the adding: loads issued there are under way meanwhile.  False: a
-// wait ran out.
+// trees over absent entries only add zeros.)  A block sends the sums of its
+// one or two tiles, a scene of one block nothing.  `ahead` runs once the
+// other blocks' sums have come in, before the last of the adding: loads issued
+// there are under way meanwhile.  False: a wait ran out.
 template <typename E, int NQ, typename F>
 __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B, CgrShared& S, bool lead, int sl,
                                             unsigned seq, E (&v)[NQ], const F& ahead) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int par = seq & 1;
-  const bool tiles = B.tile != 0;
   const int copies = exchange_copies(B.nblk);
   const size_t cstride = 3 * (size_t)A.nrec_total;
   uint4* rec = A.recs + par * kMaxCopies * cstride + B.rec0;
@@ -96,33 +90,28 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
     if (lane < copies) st_rec(rec + lane * cstride + (size_t)q * A.nrec_total + i, rec_of(a, seq));
   };
   if (lead) tree<E, NQ, 16>(v);
-  if (tiles) {
-    if (lead && lane == 0)
+  if (lead && lane == 0)
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.part[par][q][sl], v[q]);
-    __syncthreads();
-    const int nt = (B.nsl + kCgrTile - 1) / kCgrTile;  // 1 or 2
-    if (B.nblk == 1) {
+    for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.part[par][q][sl], v[q]);
+  __syncthreads();
+  const int nt = (B.nsl + kCgrTile - 1) / kCgrTile;  // 1 or 2
+  if (B.nblk == 1) {
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) v[q] = lane < B.nsl ? Slot<E>::sget(&S.part[par][q][lane]) : E(0);
-      tree<E, NQ, 4>(v);  // the tiles' sums in lanes 0 and 8
+    for (int q = 0; q < NQ; ++q) v[q] = lane < B.nsl ? Slot<E>::sget(&S.part[par][q][lane]) : E(0);
+    tree<E, NQ, 4>(v);  // the tiles' sums in lanes 0 and 8
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        if (nt > 1) v[q] = radd(v[q], shfl_to(v[q], 8));
-        v[q] = shfl_to(v[q], 0);
-      }
-      ahead();
-      return true;
+    for (int q = 0; q < NQ; ++q) {
+      if (nt > 1) v[q] = radd(v[q], shfl_to(v[q], 8));
+      v[q] = shfl_to(v[q], 0);
     }
-    if (warp < NQ * nt) {
-      const int q = warp / nt, t = warp % nt, at = kCgrTile * t + lane;
-      E a[1] = {lane < kCgrTile && at < B.nsl ? Slot<E>::sget(&S.part[par][q][at]) : E(0)};
-      tree<E, 1, 4>(a);
-      send(q, B.rec + t, a[0]);
-    }
-  } else if (lead) {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) send(q, B.rec + sl, v[q]);
+    ahead();
+    return true;
+  }
+  if (warp < NQ * nt) {
+    const int q = warp / nt, t = warp % nt, at = kCgrTile * t + lane;
+    E a[1] = {lane < kCgrTile && at < B.nsl ? Slot<E>::sget(&S.part[par][q][at]) : E(0)};
+    tree<E, 1, 4>(a);
+    send(q, B.rec + t, a[0]);
   }
   const int n = B.nrec;
   // the sums of record i (0 for lanes without one), the warp in step
@@ -145,15 +134,7 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
     E a[NQ];
     if (!fetch(lane, a)) return false;
     ahead();
-    if (tiles) {
-      tree<E, NQ, 16>(a);
-    } else {
-      tree<E, NQ, 4>(a);  // tiles' sums in lanes 0, 8, 16, 24
-#pragma unroll
-      for (int off = 16; off >= 8; off >>= 1)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) a[q] = radd(a[q], shfl_down(a[q], off));
-    }
+    tree<E, NQ, 16>(a);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) v[q] = shfl_to(a[q], 0);
     return true;
@@ -161,48 +142,20 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
   E s[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) s[q] = E(0);
-  int nt = n;
-  if (!tiles) {
-    nt = (n + kCgrTile - 1) / kCgrTile;
-    for (int i0 = 32 * warp; i0 < n; i0 += (int)blockDim.x) {
-      const int i = i0 + lane;
-      E a[NQ];
-      if (!fetch(i, a)) return false;
-      tree<E, NQ, 4>(a);
-      if ((lane & 7) == 0 && i < n)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.tp[par][q][i >> 3], a[q]);
-    }
-    __syncthreads();
-    ahead();
-    if (nt <= 32) {
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) s[q] = lane < nt ? Slot<E>::sget(&S.tp[par][q][lane]) : E(0);
-      tree<E, NQ, 16>(s);
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) v[q] = shfl_to(s[q], 0);
-      return true;
-    }
-    if (warp < 8)
-      for (int i = threadIdx.x; i < nt; i += 256)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) s[q] = radd(s[q], Slot<E>::sget(&S.tp[par][q][i]));
-  } else if (warp < 8) {
+  if (warp < 8) {
     for (int i0 = 32 * warp; i0 < n; i0 += 256) {
       E a[NQ];
       if (!fetch(i0 + lane, a)) return false;
 #pragma unroll
       for (int q = 0; q < NQ; ++q) s[q] = radd(s[q], a[q]);
     }
-  }
-  if (warp < 8) {
     tree<E, NQ, 16>(s);
     if (lane == 0)
 #pragma unroll
       for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.red[par][q][warp], s[q]);
   }
   __syncthreads();
-  if (tiles) ahead();
+  ahead();
 #pragma unroll
   for (int q = 0; q < NQ; ++q) v[q] = lane < 8 ? Slot<E>::sget(&S.red[par][q][lane]) : E(0);
   tree<E, NQ, 4>(v);
@@ -290,26 +243,6 @@ __device__ __forceinline__ void cgr_multiply(const CgrMatrix<float>& M, const fl
     ell_block_fma(w0, w1, w2, w3, w4, p, acc[0], acc[1], acc[2]);
   }
 }
-// One component of the row in FP64 (three warps a slice: the FP64 pipe issues
-// a warp instruction every 64 cycles, so a row's 9 products a slot in one
-// thread are the iteration's longest chain); u: three doubles per local index.
-__device__ __forceinline__ void cgr_multiply(const CgrMatrix<double>& M, const double* u, int comp, double& acc) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll 4
-  for (int k = 0; k < M.res; ++k) {
-    const double* p = u + 3 * (int)M.li[32 * k + lane];
-    const double* m = M.mat + 288 * k + 96 * comp + lane;
-    acc = fma(m[64], p[2], fma(m[32], p[1], fma(m[0], p[0], acc)));
-  }
-  for (int k = M.res; k < M.len; ++k) {
-    const double* p = u + 3 * (int)M.gli[32 * k + lane];
-    const double a0 = M.gell[ell_entry(M.soff, k, lane, 3 * comp)],
-                 a1 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 1)],
-                 a2 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 2)];
-    acc = fma(a2, p[2], fma(a1, p[1], fma(a0, p[0], acc)));
-  }
-}
-
 // A solve that ended on a wait that ran out: later launches use other tags.
 __device__ __forceinline__ void cgr_abort(const CgrArgs& A, const CgrBlock& B) {
   if ((threadIdx.x & 31) == 0) atomicAdd(A.seq + B.scene, 0x100000u);
@@ -321,14 +254,10 @@ constexpr int kHaloRegs = 4;  // halo columns a thread keeps in registers
 // Eigen's iteration, as k_cg_spmv, k_cg_update and k_cg_replace run it:
 //   p = z + beta p;  Ap;  (p, Ap) -> alpha;  x += alpha p;  r -= alpha Ap;
 //   z = D^-1 r;  (r, r), (r, z) -> the stopping test and beta;
-// the exchanged vector is z, and each block keeps p at its halo.  In FP64 a
-// row is three threads' (one component each), and the lead thread (component
-// 0) forms the row's share of the inner products in component order.
-template <typename Real, int kThreads>
+// the exchanged vector is z, and each block keeps p at its halo.  Mixed path.
+template <int kThreads>
 __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
-  using E = typename Ext<Real>::T;
-  constexpr bool k64 = sizeof(Real) == 8;
-  constexpr int NC = k64 ? 1 : 3;
+  using E = df64;
   extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
   __shared__ CgrShared S;
   const CgrBlock B = A.blocks[blockIdx.x];
@@ -336,17 +265,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
   SceneScalars* sc = sd.sc;
   if (!sc->cg_active) return;
   unsigned seq = __ldcg(A.seq + B.scene);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sl = k64 ? warp / 3 : warp, comp = k64 ? warp % 3 : 0;
-  const bool roww = sl < B.nsl, lead = roww && comp == 0;
+  const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+  const bool roww = sl < B.nsl;
   const int row = 32 * (B.slice0 + sl) + lane;
   const bool live = roww && row < sd.nf;
   const int own = 32 * B.nsl, mine = 32 * sl + lane;
   unsigned char* rest;
-  const CgrMatrix<Real> M = cgr_load_matrix<Real>(A, B, sd, sl, cgr_smem_raw, &rest);
-  Real* vec = reinterpret_cast<Real*>(rest);                    // FP32: 4 per entry, FP64: 3
-  double* ex = reinterpret_cast<double*>(vec + 3 * (size_t)(own + B.nh));  // FP64: r, z of the rows
-  (void)ex;
+  const CgrMatrix<float> M = cgr_load_matrix<float>(A, B, sd, sl, cgr_smem_raw, &rest);
+  float4* vec = reinterpret_cast<float4*>(rest);  // p at the own rows and the halo
   // the first halo columns of each thread, and their records under way
   int hc[kHaloRegs];
   bool hw[kHaloRegs];
@@ -356,70 +282,53 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
     const int h = threadIdx.x + j * kThreads;
     hw[j] = h < B.nh;
     hc[j] = hw[j] ? A.h_col[B.hoff + h] : 0;
-    if (!k64 && hw[j])
+    if (hw[j])
       hv[j] = *reinterpret_cast<const uint4*>(static_cast<const float*>(sd.cg_z) + 4 * (size_t)hc[j]);
   }
   auto halo_ahead = [&]() {
-    if constexpr (!k64) {
 #pragma unroll
-      for (int j = 0; j < kHaloRegs; ++j)
-        if (hw[j]) hv[j] = ld_rec(A.pub + B.row0 + hc[j]);
-    }
+    for (int j = 0; j < kHaloRegs; ++j)
+      if (hw[j]) hv[j] = ld_rec(A.pub + B.row0 + hc[j]);
   };
   auto nothing = []() {};
 
   const size_t k4 = 4 * (size_t)row;
-  Real r[NC], z[NC], p[NC], x[NC], acc[NC], dv[k64 ? 3 : 9];
+  float r[3], z[3], p[3], acc[3], dv[9];
   X3 xe = zero_x3();
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    r[c] = live ? static_cast<const Real*>(sd.cg_r)[k4 + comp + c] : Real(0);
-    z[c] = live ? static_cast<const Real*>(sd.cg_z)[k4 + comp + c] : Real(0);
-    p[c] = x[c] = acc[c] = Real(0);
+  for (int c = 0; c < 3; ++c) {
+    r[c] = live ? static_cast<const float*>(sd.cg_r)[k4 + c] : 0.f;
+    z[c] = live ? static_cast<const float*>(sd.cg_z)[k4 + c] : 0.f;
+    p[c] = acc[c] = 0.f;
   }
-  if constexpr (k64) {
-    // the component's row of the preconditioner
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-      dv[c] = !live ? 0.0
-                    : sd.block_jacobi ? static_cast<const double*>(sd.dinv)[9 * (size_t)row + 3 * comp + c]
-                                      : (c == 0 ? static_cast<const double*>(sd.dinv)[k4 + comp] : 0.0);
-  } else {
-#pragma unroll
-    for (int c = 0; c < 9; ++c)
-      dv[c] = !live ? 0.f
-                    : sd.block_jacobi ? static_cast<const float*>(sd.dinv)[9 * (size_t)row + c]
-                                      : (c < 3 ? static_cast<const float*>(sd.dinv)[k4 + c] : 0.f);
-  }
+  for (int c = 0; c < 9; ++c)
+    dv[c] = !live ? 0.f
+                  : sd.block_jacobi ? static_cast<const float*>(sd.dinv)[9 * (size_t)row + c]
+                                    : (c < 3 ? static_cast<const float*>(sd.dinv)[k4 + c] : 0.f);
   const bool block_jacobi = sd.block_jacobi != 0;
   // apply_prec with the row's entries in registers
   auto precond = [&](const float (&rv)[3], float (&zv)[3]) {
-    if constexpr (!k64) {
-      if (block_jacobi) {
+    if (block_jacobi) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) zv[c] = fma(dv[3 * c + 2], rv[2], fma(dv[3 * c + 1], rv[1], dv[3 * c] * rv[0]));
-      } else {
+      for (int c = 0; c < 3; ++c) zv[c] = fma(dv[3 * c + 2], rv[2], fma(dv[3 * c + 1], rv[1], dv[3 * c] * rv[0]));
+    } else {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) zv[c] = dv[c] * rv[c];
-      }
+      for (int c = 0; c < 3; ++c) zv[c] = dv[c] * rv[c];
     }
   };
   E rz = sc_get<E>(&sc->rz), rz_prev = rz;
   const E rr0 = sc_get<E>(&sc->cg_rhs_norm2);
   E rr = rr0;
-  Real beta = Real(0);
+  float beta = 0.f;
   E alphaE = E(0), betaE = E(0);
   int it = 0, status = 0, cg_status = 0;
   unsigned ztag = 0;
 
   auto publish_z = [&](unsigned tag) {
-    if (!live || B.nblk == 1) return;
-    if constexpr (k64) {
-      st_rec(A.pub + 3 * (size_t)(B.row0 + row) + comp, rec_of(z[0], tag));
-    } else {
+    if (live && B.nblk > 1)
       st_rec(A.pub + B.row0 + row,
              make_uint4(__float_as_uint(z[0]), __float_as_uint(z[1]), __float_as_uint(z[2]), tag));
-    }
   };
 
   for (;;) {
@@ -427,54 +336,31 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
     // ---- p = z + beta p: own rows, then the halo
     if (roww) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) p[c] = first ? z[c] : fma(beta, p[c], z[c]);
-      if constexpr (k64) vec[3 * mine + comp] = p[0];
-      else reinterpret_cast<float4*>(vec)[mine] = make_float4(p[0], p[1], p[2], 0.f);
+      for (int c = 0; c < 3; ++c) p[c] = first ? z[c] : fma(beta, p[c], z[c]);
+      vec[mine] = make_float4(p[0], p[1], p[2], 0.f);
     }
     bool ok = true;
-    if constexpr (k64) {
-      const int nh3 = 3 * B.nh;
-      for (int h0 = 32 * warp; h0 < nh3; h0 += kThreads) {
-        const int h = h0 + lane;
-        const bool want[1] = {h < nh3};
-        const int col = want[0] ? __ldg(A.h_col + B.hoff + h / 3) : 0, c = h % 3;
-        double zc = 0.0;
-        if (first) {
-          if (want[0]) zc = static_cast<const double*>(sd.cg_z)[4 * (size_t)col + c];
-        } else {
-          const uint4* src = A.pub + 3 * (size_t)(B.row0 + col) + c;
-          uint4 v[1] = {ld_rec(src)};
-          ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, &A.ctrs->error) && ok;
-          zc = rec_val<double>(v[0]);
-        }
-        if (want[0]) {
-          double* pd = vec + 3 * own + h;
-          *pd = first ? zc : fma(beta, *pd, zc);
-        }
-      }
-    } else {
-      float4* ph = reinterpret_cast<float4*>(vec) + own;
-      auto put = [&](int h, const uint4& v) {
-        const float z0 = __uint_as_float(v.x), z1 = __uint_as_float(v.y), z2 = __uint_as_float(v.z);
-        const float4 o = ph[h];
-        ph[h] = first ? make_float4(z0, z1, z2, 0.f)
-                      : make_float4(fma(beta, o.x, z0), fma(beta, o.y, z1), fma(beta, o.z, z2), 0.f);
-      };
-      if (!first)
-        ok = poll_recs<kHaloRegs>(hv, [&](int j) { return A.pub + B.row0 + hc[j]; }, hw, ztag, &A.ctrs->error) && ok;
+    float4* ph = vec + own;
+    auto put = [&](int h, const uint4& v) {
+      const float z0 = __uint_as_float(v.x), z1 = __uint_as_float(v.y), z2 = __uint_as_float(v.z);
+      const float4 o = ph[h];
+      ph[h] = first ? make_float4(z0, z1, z2, 0.f)
+                    : make_float4(fma(beta, o.x, z0), fma(beta, o.y, z1), fma(beta, o.z, z2), 0.f);
+    };
+    if (!first)
+      ok = poll_recs<kHaloRegs>(hv, [&](int j) { return A.pub + B.row0 + hc[j]; }, hw, ztag, &A.ctrs->error) && ok;
 #pragma unroll
-      for (int j = 0; j < kHaloRegs; ++j)
-        if (hw[j]) put(threadIdx.x + j * kThreads, hv[j]);
-      for (int h0 = 32 * warp + kHaloRegs * kThreads; h0 < B.nh; h0 += kThreads) {
-        const int h = h0 + lane;
-        const bool want[1] = {h < B.nh};
-        const int col = want[0] ? __ldg(A.h_col + B.hoff + h) : 0;
-        const uint4* src = first ? reinterpret_cast<const uint4*>(static_cast<const float*>(sd.cg_z) + 4 * (size_t)col)
-                                 : A.pub + B.row0 + col;
-        uint4 v[1] = {ld_rec(src)};
-        if (!first) ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, &A.ctrs->error) && ok;
-        if (want[0]) put(h, v[0]);
-      }
+    for (int j = 0; j < kHaloRegs; ++j)
+      if (hw[j]) put(threadIdx.x + j * kThreads, hv[j]);
+    for (int h0 = 32 * sl + kHaloRegs * kThreads; h0 < B.nh; h0 += kThreads) {
+      const int h = h0 + lane;
+      const bool want[1] = {h < B.nh};
+      const int col = want[0] ? __ldg(A.h_col + B.hoff + h) : 0;
+      const uint4* src = first ? reinterpret_cast<const uint4*>(static_cast<const float*>(sd.cg_z) + 4 * (size_t)col)
+                               : A.pub + B.row0 + col;
+      uint4 v[1] = {ld_rec(src)};
+      if (!first) ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, &A.ctrs->error) && ok;
+      if (want[0]) put(h, v[0]);
     }
     if (!__syncthreads_and(ok)) {
       cgr_abort(A, B);
@@ -484,64 +370,27 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
     E d1[1] = {E(0)};
     if (roww) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) acc[c] = Real(0);
-      if constexpr (k64) cgr_multiply(M, vec, comp, acc[0]);
-      else cgr_multiply(M, reinterpret_cast<const float4*>(vec), acc);
+      for (int c = 0; c < 3; ++c) acc[c] = 0.f;
+      cgr_multiply(M, vec, acc);
     }
-    if constexpr (k64) {
-      if (roww) ex[96 * sl + 32 * comp + lane] = acc[0];
-      __syncthreads();
-      if (lead && live) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) d1[0] = acc_prod(d1[0], vec[3 * mine + c], ex[96 * sl + 32 * c + lane]);
-      }
-    } else if (live) {
+    if (live) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) d1[0] = acc_prod(d1[0], p[c], acc[c]);
     }
-    if (!scene_total<E, 1>(A, B, S, lead, sl, seq, d1, nothing)) {
+    if (!scene_total<E, 1>(A, B, S, roww, sl, seq, d1, nothing)) {
       cgr_abort(A, B);
       return;
     }
     ++seq;
     alphaE = rz / d1[0];
-    const Real alpha = Real(to_step(alphaE));
+    const float alpha = to_step(alphaE);
     // ---- x, r, z, (r, r), (r, z)
-    const bool replace = !k64 && (it + 1) % kCgReplace == 0;
+    const bool replace = (it + 1) % kCgReplace == 0;
     E d2[2] = {E(0), E(0)};
-    if constexpr (k64) {
-      double* exr = ex;
-      double* exz = ex + 96 * B.nsl;
-      x[0] = fma(alpha, p[0], x[0]);
-      r[0] = fma(-alpha, acc[0], r[0]);
-      // the lead warps have read Ap of the exchange buffer by now only if
-      // they are past their sum: a barrier before it is reused
-      __syncthreads();
-      if (roww) exr[96 * sl + 32 * comp + lane] = r[0];
-      if (block_jacobi) {
-        __syncthreads();
-        if (roww) {
-          const double* q = exr + 96 * sl + lane;
-          z[0] = fma(dv[2], q[64], fma(dv[1], q[32], dv[0] * q[0]));
-        }
-      } else {
-        z[0] = dv[0] * r[0];
-      }
-      if (roww) exz[96 * sl + 32 * comp + lane] = z[0];
-      publish_z(seq);
-      __syncthreads();
-      if (lead && live) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const double rc = exr[96 * sl + 32 * c + lane], zc = exz[96 * sl + 32 * c + lane];
-          d2[0] = acc_prod(d2[0], rc, rc);
-          d2[1] = acc_prod(d2[1], rc, zc);
-        }
-      }
-    } else if (live) {
+    if (live) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        xe.v[c] = xe.v[c] + two_prod(float(alpha), float(p[c]));
+        xe.v[c] = xe.v[c] + two_prod(alpha, p[c]);
         r[c] = fma(-alpha, acc[c], r[c]);
         d2[0] = acc_prod(d2[0], r[c], r[c]);
       }
@@ -549,19 +398,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
         xe_store(sd.cg_xe, row, xe);
         __threadfence();
       }
-      float r3[3] = {float(r[0]), float(r[1]), float(r[2])}, z3[3];
-      precond(r3, z3);
+      precond(r, z);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        z[c] = z3[c];
-        d2[1] = acc_prod(d2[1], r[c], z[c]);
-      }
+      for (int c = 0; c < 3; ++c) d2[1] = acc_prod(d2[1], r[c], z[c]);
       if (!replace) publish_z(seq);
     }
-    if constexpr (!k64) {
-      if (replace) __syncthreads();  // every row's x_e is visible before the block's sums
-    }
-    if (!scene_total<E, 2>(A, B, S, lead, sl, seq, d2, halo_ahead)) {
+    if (replace) __syncthreads();  // every row's x_e is visible before the block's sums
+    if (!scene_total<E, 2>(A, B, S, roww, sl, seq, d2, halo_ahead)) {
       cgr_abort(A, B);
       return;
     }
@@ -586,78 +429,374 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
       status = 4;
     }
     if (stop) break;
-    if constexpr (!k64) {
-      if (replace) {
-        // ---- r = b - A x with x in df64 (k_cg_replace)
-        __syncwarp();
-        __threadfence();
-        E d3[2] = {E(0), E(0)};
-        if (live) {
-          df64 ax[3] = {df64(0.f), df64(0.f), df64(0.f)};
+    if (replace) {
+      // ---- r = b - A x with x in df64 (k_cg_replace)
+      __syncwarp();
+      __threadfence();
+      E d3[2] = {E(0), E(0)};
+      if (live) {
+        df64 ax[3] = {df64(0.f), df64(0.f), df64(0.f)};
 #pragma unroll 4
-          for (int k = 0; k < M.len; ++k) {
-            const size_t q = ell_pair(M.soff, k, lane, 0);
-            const float* ell = static_cast<const float*>(sd.ell);
-            const float2 w0 = ld_pair<false>(ell, q), w1 = ld_pair<false>(ell, q + 32),
-                         w2 = ld_pair<false>(ell, q + 64), w3 = ld_pair<false>(ell, q + 96),
-                         w4 = ld_pair<false>(ell, q + 128);
-            const X3 xc = xe_load<true>(sd.cg_xe, pair_col(w0));
-            const float a[9] = {w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y, w4.x, w4.y};
+        for (int k = 0; k < M.len; ++k) {
+          const size_t q = ell_pair(M.soff, k, lane, 0);
+          const float* ell = static_cast<const float*>(sd.ell);
+          const float2 w0 = ld_pair<false>(ell, q), w1 = ld_pair<false>(ell, q + 32),
+                       w2 = ld_pair<false>(ell, q + 64), w3 = ld_pair<false>(ell, q + 96),
+                       w4 = ld_pair<false>(ell, q + 128);
+          const X3 xc = xe_load<true>(sd.cg_xe, pair_col(w0));
+          const float a[9] = {w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y, w4.x, w4.y};
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
+          for (int i = 0; i < 3; ++i)
 #pragma unroll
-              for (int j = 0; j < 3; ++j) {
-                const float aij = a[3 * i + j];
-                ax[i] = ax[i] + two_prod(aij, xc.v[j].hi) + df64(aij * xc.v[j].lo);
-              }
-          }
-          float b[3], r3[3], z3[3];
-          ld3<false>(static_cast<const float*>(sd.rhs) + k4, b);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) r3[c] = Ext<float>::to_real(df64(b[c]) - ax[c]);
-          precond(r3, z3);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            r[c] = r3[c];
-            z[c] = z3[c];
-            d3[0] = acc_prod(d3[0], r3[c], r3[c]);
-            d3[1] = acc_prod(d3[1], r3[c], z3[c]);
-          }
-          publish_z(seq);
+            for (int j = 0; j < 3; ++j) {
+              const float aij = a[3 * i + j];
+              ax[i] = ax[i] + two_prod(aij, xc.v[j].hi) + df64(aij * xc.v[j].lo);
+            }
         }
-        if (!scene_total<E, 2>(A, B, S, lead, sl, seq, d3, halo_ahead)) {
-          cgr_abort(A, B);
-          return;
+        float b[3];
+        ld3<false>(static_cast<const float*>(sd.rhs) + k4, b);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) r[c] = Ext<float>::to_real(df64(b[c]) - ax[c]);
+        precond(r, z);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          d3[0] = acc_prod(d3[0], r[c], r[c]);
+          d3[1] = acc_prod(d3[1], r[c], z[c]);
         }
-        ztag = seq;
-        ++seq;
-        rr = d3[0];
-        if (cg_meets(sd, rr, rr0) || is_nan(rr)) {
-          if (is_nan(rr)) status = 4;
-          it = it - 1;  // as in Eigen, the iteration that meets the threshold is not counted
-          break;
-        }
-        betaE = d3[1] / rz_prev;
-        rz = d3[1];
+        publish_z(seq);
       }
+      if (!scene_total<E, 2>(A, B, S, roww, sl, seq, d3, halo_ahead)) {
+        cgr_abort(A, B);
+        return;
+      }
+      ztag = seq;
+      ++seq;
+      rr = d3[0];
+      if (cg_meets(sd, rr, rr0) || is_nan(rr)) {
+        if (is_nan(rr)) status = 4;
+        it = it - 1;  // as in Eigen, the iteration that meets the threshold is not counted
+        break;
+      }
+      betaE = d3[1] / rz_prev;
+      rz = d3[1];
     }
-    beta = Real(to_step(betaE));
+    beta = to_step(betaE);
   }
   // ---- the solution and the scene's scalars
   if (live) {
-    if constexpr (k64) {
-      static_cast<double*>(sd.cg_x)[k4 + comp] = x[0];
-    } else {
-      float xf[3];
+    float xf[3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) xf[c] = Ext<float>::to_real(xe.v[c]);
-      st3(static_cast<float*>(sd.cg_x) + k4, xf);
-      xe_store(sd.cg_xe, row, xe);
-    }
+    for (int c = 0; c < 3; ++c) xf[c] = Ext<float>::to_real(xe.v[c]);
+    st3(static_cast<float*>(sd.cg_x) + k4, xf);
+    xe_store(sd.cg_xe, row, xe);
   }
   if (B.rec == 0 && threadIdx.x == 0) {
     sc_put(&sc->alpha, alphaE);
     sc_put(&sc->beta, betaE);
+    sc_put(&sc->rz, rz);
+    sc_put(&sc->rz_prev, rz_prev);
+    sc->cg_err = cg_rel(rr, rr0);
+    sc->cg_iter = it;
+    sc->cg_total += it;
+    if (status) sc->status = status;
+    if (cg_status) sc->cg_status = cg_status;
+    sc->cg_active = 0;
+    sc->nph = kPhLocal;
+    atomicSub(&A.ctrs->cg_active, 1);
+    A.seq[B.scene] = seq;
+  }
+}
+
+// The FP64 form.  What bounds it is the FP64 pipe, which takes a warp's
+// instruction every 17 to 19 cycles of the SM (and 66 for the next one of the
+// same warp, 576 for a division): a block has one slice, or two or four where
+// there are more slices than SMs, and always twelve warps, one per slice,
+// component and part of the slots (4, 2 or 1 parts: the slots k = j mod 4 are
+// four sums, see RowSum); the warps of part 0 own the rows' components.  A
+// slice's sums, the adding of the other blocks' and the scalars are one warp's
+// each, and the quotient by a number known before is a product with its
+// reciprocal, corrected (quotient_by).  An iteration at 90 / 1300 rows: 8.0 /
+// 8.5 us, against 10.2 / 11.5 with a slice's component in one warp and the sums
+// and scalars in every warp, and 34 / 38 in k_cg_solve.  Of the 16,100 cycles
+// at 1300 rows the product is 3400 (its 180 warp instructions a slice at the
+// pipe's rate), the two exchanges 5000, trees and divisions 4500.
+constexpr int kThreads64 = 384;
+__global__ void __launch_bounds__(kThreads64, 1) k_cgr_split64(const CgrArgs A) {
+  extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
+  __shared__ double part[2][kCgrMaxSpb64], tile[2][kCgrMaxTiles64], tot[2], step[2], rcp;
+  __shared__ int flags;  // 1: a wait ran out
+  const CgrBlock B = A.blocks[blockIdx.x];
+  const SceneDev& sd = A.sds[B.scene];
+  SceneScalars* sc = sd.sc;
+  if (!sc->cg_active) return;
+  unsigned seq = __ldcg(A.seq + B.scene);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int parts = B.spb >= 4 ? 1 : 4 / B.spb;
+  const int comp = warp % 3, sl = warp / 3 / parts, pt = warp / 3 % parts;
+  const bool roww = sl < B.nsl, owner = roww && pt == 0;
+  const int row = 32 * (B.slice0 + sl) + lane;
+  const bool live = owner && row < sd.nf;
+  const int own = 32 * B.nsl, mine = 32 * sl + lane;
+  unsigned char* rest;
+  const CgrMatrix<double> M = cgr_load_matrix<double>(A, B, sd, sl, cgr_smem_raw, &rest);
+  double* vec = reinterpret_cast<double*>(rest);  // p at the own rows and the halo, 3 each
+  double* ex = vec + 3 * (own + B.nh);            // [2][slice][3][32]: y / r, z
+  double* sums = ex + 192 * B.nsl;                // [3][slice][3][32]: the products of parts 1 ..
+  int* err = &A.ctrs->error;
+  const int ex_at = 96 * sl + 32 * comp + lane;
+
+  // the halo's entries (column, component) of this thread: the first in registers
+  constexpr int kHalo = 3;
+  int hc[kHalo];
+  bool hw[kHalo];
+  uint4 hv[kHalo];
+#pragma unroll
+  for (int j = 0; j < kHalo; ++j) {
+    const int i = threadIdx.x + j * kThreads64;
+    hw[j] = i < 3 * B.nh;
+    hc[j] = hw[j] ? 3 * (B.row0 + A.h_col[B.hoff + i / 3]) + i % 3 : 0;
+  }
+  for (int i = threadIdx.x; i < 3 * B.nh; i += kThreads64)
+    vec[3 * own + i] = static_cast<const double*>(sd.cg_z)[4 * (size_t)A.h_col[B.hoff + i / 3] + i % 3];
+  auto halo_ahead = [&]() {
+#pragma unroll
+    for (int j = 0; j < kHalo; ++j)
+      if (hw[j]) hv[j] = ld_rec(A.pub + hc[j]);
+  };
+
+  const size_t k4 = 4 * (size_t)row;
+  const bool block_jacobi = sd.block_jacobi != 0;
+  double r = 0.0, z = 0.0, p = 0.0, x = 0.0, y = 0.0, dv[3] = {0.0, 0.0, 0.0};
+  if (live) {
+    r = static_cast<const double*>(sd.cg_r)[k4 + comp];
+    z = static_cast<const double*>(sd.cg_z)[k4 + comp];
+    const double* dinv = static_cast<const double*>(sd.dinv);
+    if (block_jacobi) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) dv[c] = dinv[9 * (size_t)row + 3 * comp + c];
+    } else {
+      dv[0] = dinv[k4 + comp];
+    }
+  }
+  double rz = sc_get<double>(&sc->rz), rz_prev = rz, beta = 0.0;
+  const double rr0 = sc_get<double>(&sc->cg_rhs_norm2);
+  // (every FP64 instruction of all twelve warps takes 230 cycles of the pipe,
+  // comparisons too: a sum of squares or NaN compares like its bits)
+  const unsigned long long thr = __double_as_longlong(::fmax(sd.cg_tol * sd.cg_tol * rr0, DBL_MIN));  // as cg_meets
+  constexpr unsigned long long kInf = 0x7ff0000000000000ull;
+  double rr = rr0, alpha = 0.0;
+  const int max_cg = sd.max_cg;
+  int it = 0, status = 0, cg_status = 0;
+  unsigned ztag = 0;
+  if (threadIdx.x == 0) flags = 0;
+
+  // A slice's sum of the lanes' e (the whole warp), as tile_partials adds them.
+  auto slice_sum = [&](int q, double e) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) e += shfl_down(e, off);
+    if (lane == 0) part[q][sl] = e;
+    return e;
+  };
+  // The scene's sums of nq quantities in tot[], the slices' in part[][]: slices
+  // to tiles of eight, tiles i, i + 256, .. (there are fewer), a tree over 32
+  // tiles, a tree over 8 such sums; absent entries are zeros.  `beside`: the
+  // last warp's, during the wait; `then(q, sum)`: lane 0's of the warp that has
+  // the sum.  False: a wait ran out.
+  auto total = [&](int nq, auto beside, auto then) -> bool {
+    const int par = seq & 1, n = B.nrec, copies = exchange_copies(B.nblk);
+    const size_t cstride = 3 * (size_t)A.nrec_total;
+    uint4* rec = A.recs + par * kMaxCopies * cstride + B.rec0;
+    __syncthreads();
+    if (B.nblk > 1 && warp < nq * B.nsl) {
+      const int q = warp / B.nsl, t = warp % B.nsl;
+      const double v = part[q][t];
+      if (lane < copies) st_rec(rec + lane * cstride + (size_t)q * A.nrec_total + B.rec + t, rec_of(v, seq));
+    }
+    if (warp == kThreads64 / 32 - 1) beside();
+    const uint4* src = rec + (blockIdx.x % copies) * cstride;
+    const int chunks = (n + 31) / 32;
+    for (int job = warp; job < nq * chunks; job += kThreads64 / 32) {
+      const int q = job / chunks, i = 32 * (job % chunks) + lane;
+      double v = 0.0;
+      if (B.nblk > 1) {
+        const uint4* at = src + (size_t)q * A.nrec_total + min(i, n - 1);
+        uint4 w[1] = {ld_rec(at)};
+        const bool want[1] = {i < n};
+        if (!poll_recs<1>(w, [&](int) { return at; }, want, seq, err) && lane == 0) atomicOr(&flags, 1);
+        v = i < n ? rec_double(w[0]) : 0.0;
+      } else if (i < n) {
+        v = part[q][i];
+      }
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1) v += shfl_down(v, off);
+      if ((lane & 7) == 0 && i < n) tile[q][i >> 3] = v;
+    }
+    __syncthreads();
+    if (flags & 1) return false;
+    if (warp < nq) {
+      const int nt = (n + kCgrTile - 1) / kCgrTile;
+      double v = 0.0;
+      // (at most 96 tiles: three trees over 32, then 0 + 2 and that + 1, the
+      // order of the tree over eight)
+      double g[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        if (32 * j < nt) {  // warp-uniform
+          double e = 32 * j + lane < nt ? tile[warp][32 * j + lane] : 0.0;
+          for (int off = nt - 32 * j > 16 ? 16 : nt - 32 * j > 8 ? 8 : nt - 32 * j > 4 ? 4 : nt - 32 * j > 2 ? 2 : 1;
+               off > 0; off >>= 1)
+            e += shfl_down(e, off);
+          g[j] = e;
+        }
+      v = nt > 64 ? (g[0] + g[2]) + g[1] : nt > 32 ? g[0] + g[1] : g[0];
+      if (lane == 0) {
+        tot[warp] = v;
+        then(warp, v);
+      }
+    }
+    __syncthreads();
+    ++seq;
+    return true;
+  };
+
+  __syncthreads();
+  for (;;) {
+    const bool first = it == 0;
+    // ---- p = z + beta p: own rows, then the halo
+    if (owner) {
+      if (live) p = first ? z : fma(beta, p, z);
+      vec[3 * mine + comp] = p;
+    }
+    bool ok = true;
+    if (!first && B.nblk > 1) {
+      ok = poll_recs<kHalo>(hv, [&](int j) { return A.pub + hc[j]; }, hw, ztag, err);
+#pragma unroll
+      for (int j = 0; j < kHalo; ++j)
+        if (hw[j]) {
+          double* q = vec + 3 * own + threadIdx.x + j * kThreads64;
+          *q = fma(beta, *q, rec_double(hv[j]));
+        }
+      for (int i0 = 32 * warp + kHalo * kThreads64; i0 < 3 * B.nh; i0 += kThreads64) {
+        const int i = i0 + lane;
+        const bool want[1] = {i < 3 * B.nh};
+        const uint4* src = A.pub + (want[0] ? 3 * (size_t)(B.row0 + __ldg(A.h_col + B.hoff + i / 3)) + i % 3 : 0);
+        uint4 v[1] = {ld_rec(src)};
+        ok = poll_recs<1>(v, [&](int) { return src; }, want, ztag, err) && ok;
+        if (want[0]) {
+          double* q = vec + 3 * own + i;
+          *q = fma(beta, *q, rec_double(v[0]));
+        }
+      }
+    }
+    if (!__syncthreads_and(ok)) {
+      cgr_abort(A, B);
+      return;
+    }
+    // ---- Ap, (p, Ap)
+    double a[4] = {0.0, 0.0, 0.0, 0.0};  // of part pt: slots k = j mod 4, j = pt (4 parts), 2 pt, 2 pt + 1 (2), all (1)
+    if (roww) {
+      const int per = 4 / parts;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < per) {
+          const double* m = M.mat + 96 * comp + lane;
+          int k = per * pt + j;
+#pragma unroll 5
+          for (; k < M.res; k += 4) {
+            const double* u = vec + 3 * (int)M.li[32 * k + lane];
+            a[j] = fma(m[288 * k + 64], u[2], fma(m[288 * k + 32], u[1], fma(m[288 * k], u[0], a[j])));
+          }
+          for (; k < M.len; k += 4) {
+            const double* u = vec + 3 * (int)M.gli[32 * k + lane];
+            const double m0 = M.gell[ell_entry(M.soff, k, lane, 3 * comp)],
+                         m1 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 1)],
+                         m2 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 2)];
+            a[j] = fma(m2, u[2], fma(m1, u[1], fma(m0, u[0], a[j])));
+          }
+        }
+      if (parts == 4) {
+        if (pt > 0) sums[96 * B.nsl * (pt - 1) + ex_at] = a[0];
+      } else if (parts == 2 && pt == 1) {
+        sums[ex_at] = a[0] + a[1];
+      }
+    }
+    __syncthreads();
+    if (owner) {
+      if (parts == 4)
+        y = (a[0] + sums[ex_at]) + (sums[96 * B.nsl + ex_at] + sums[192 * B.nsl + ex_at]);
+      else
+        y = (a[0] + a[1]) + (parts == 2 ? sums[ex_at] : a[2] + a[3]);
+      if (!live) y = 0.0;  // a row past the scene's adds nothing, whatever p holds
+      ex[ex_at] = y;
+    }
+    __syncthreads();
+    if (owner && comp == 0) {
+      const double* q = ex + 96 * sl + lane;
+      const double* u = vec + 3 * mine;
+      slice_sum(0, fma(u[2], q[64], fma(u[1], q[32], u[0] * q[0])));
+    }
+    if (!total(1, [&]() { if (lane == 0) rcp = 1.0 / rz; }, [&](int, double v) { step[0] = rz / v; })) {
+      cgr_abort(A, B);
+      return;
+    }
+    alpha = step[0];
+    // ---- x, r, z, (r, r), (r, z)
+    if (owner) {
+      if (live) {
+        x = fma(alpha, p, x);
+        r = fma(-alpha, y, r);
+      }
+      ex[ex_at] = r;
+    }
+    if (block_jacobi) {
+      __syncthreads();
+      if (owner) {
+        const double* q = ex + 96 * sl + lane;
+        z = fma(dv[2], q[64], fma(dv[1], q[32], dv[0] * q[0]));
+      }
+    } else {
+      z = dv[0] * r;
+    }
+    if (owner) ex[96 * B.nsl + ex_at] = z;
+    if (live && B.nblk > 1) st_rec(A.pub + 3 * (size_t)(B.row0 + row) + comp, rec_of(z, seq));
+    __syncthreads();
+    if (owner && comp < 2) {
+      const double* q = ex + 96 * sl + lane;
+      const double* o = q + (comp == 1 ? 96 * B.nsl : 0);
+      slice_sum(comp, fma(q[64], o[64], fma(q[32], o[32], q[0] * o[0])));
+    }
+    ztag = seq;
+    if (!total(2, []() {}, [&](int q, double v) { if (q == 1) step[1] = quotient_by(v, rz, rcp); })) {
+      cgr_abort(A, B);
+      return;
+    }
+    if (B.nblk > 1) halo_ahead();
+    rr = tot[0];
+    const unsigned long long bits = __double_as_longlong(rr);
+    bool stop = false;
+    if (bits < thr) {
+      stop = true;
+    } else {
+      beta = step[1];
+      rz_prev = rz;
+      rz = tot[1];
+      it = it + 1;
+      if (it >= max_cg) {
+        stop = true;
+        cg_status = 5;  // MFEM_ERR_CG_MAXITER
+      }
+    }
+    if ((bits & ~(1ull << 63)) > kInf) {  // NaN
+      stop = true;
+      status = 4;
+    }
+    if (stop) break;
+  }
+  // ---- the solution and the scene's scalars
+  if (live) static_cast<double*>(sd.cg_x)[k4 + comp] = x;
+  if (B.rec == 0 && threadIdx.x == 0) {
+    sc_put(&sc->alpha, alpha);
+    sc_put(&sc->beta, beta);
     sc_put(&sc->rz, rz);
     sc_put(&sc->rz_prev, rz_prev);
     sc->cg_err = cg_rel(rr, rr0);
@@ -899,8 +1038,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
 template <typename F> auto with_kernel(bool fp64, bool fused, bool jacobi, int threads, F&& f) {
   if (fused && threads > 256) return jacobi ? f((const void*)k_cgr_fused<true, 512>) : f((const void*)k_cgr_fused<false, 512>);
   if (fused) return jacobi ? f((const void*)k_cgr_fused<true, 256>) : f((const void*)k_cgr_fused<false, 256>);
-  if (fp64) return threads > 256 ? f((const void*)k_cgr_split<double, 384>) : f((const void*)k_cgr_split<double, 256>);
-  return threads > 256 ? f((const void*)k_cgr_split<float, 512>) : f((const void*)k_cgr_split<float, 256>);
+  if (fp64) return f((const void*)k_cgr_split64);
+  return threads > 256 ? f((const void*)k_cgr_split<512>) : f((const void*)k_cgr_split<256>);
 }
 
 }  // namespace

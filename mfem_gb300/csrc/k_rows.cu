@@ -351,7 +351,7 @@ __device__ __forceinline__ void cg_spmv_tile(int tix, const Tile* tiles, const S
     const int slice = row >> 5, rs = row & 31;
     const int soff = sd.slice_off[slice], slen = (sd.slice_off[slice + 1] - soff) >> 5;
     const unsigned long long pol_s = l2_evict_first(), pol_k = l2_evict_last();
-    Real acc0 = 0, acc1 = 0, acc2 = 0;
+    RowSum<Real> sum;
 #pragma unroll 4
     for (int k = 0; k < slen; ++k) {
       const size_t q = ell_pair(soff, k, rs, 0);
@@ -367,9 +367,10 @@ __device__ __forceinline__ void cg_spmv_tile(int tix, const Tile* tiles, const S
 #pragma unroll
         for (int c = 0; c < 3; ++c) p[c] = fma(beta, pp[c], p[c]);
       }
-      ell_block_fma(w0, w1, w2, w3, w4, p, acc0, acc1, acc2);
+      sum.add(k, w0, w1, w2, w3, w4, p);
     }
-    const Real acc[3] = {acc0, acc1, acc2};
+    Real acc[3];
+    sum.total(acc);
     Real p[3];
     ld3<kCo>(z + 4 * (size_t)row, p);
     if (!first) {

@@ -163,6 +163,38 @@ __device__ __forceinline__ void ell_block_fma(const P& w0, const P& w1, const P&
   a2 = fma(w4.y, u[2], fma(w4.x, u[1], fma(w3.y, u[0], a2)));
 }
 
+// A row of the two-reduction iteration's product: FP32 one chain over the
+// slots; FP64 four, over the slots k = j mod 4, added up in pairs, so that the
+// resident solve can give the parts of a long chain of 66-cycle instructions
+// to different warps.
+template <typename Real> struct RowSum;
+template <> struct RowSum<float> {
+  float a[3] = {0.f, 0.f, 0.f};
+  template <typename P>
+  __device__ __forceinline__ void add(int, const P& w0, const P& w1, const P& w2, const P& w3, const P& w4,
+                                      const float u[3]) {
+    ell_block_fma(w0, w1, w2, w3, w4, u, a[0], a[1], a[2]);
+  }
+  __device__ __forceinline__ void total(float y[3]) const {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) y[c] = a[c];
+  }
+};
+template <> struct RowSum<double> {
+  double a[4][3] = {};
+  template <typename P>
+  __device__ __forceinline__ void add(int k, const P& w0, const P& w1, const P& w2, const P& w3, const P& w4,
+                                      const double u[3]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if ((k & 3) == j) ell_block_fma(w0, w1, w2, w3, w4, u, a[j][0], a[j][1], a[j][2]);
+  }
+  __device__ __forceinline__ void total(double y[3]) const {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) y[c] = (a[0][c] + a[1][c]) + (a[2][c] + a[3][c]);
+  }
+};
+
 // u_{i+1} of a row from r_i, w_i, s_{i-1}: the same operations, in the same
 // order, wherever a row's value is formed.
 template <typename Real>

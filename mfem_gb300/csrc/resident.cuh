@@ -16,12 +16,11 @@ struct CgrBlock {
   int kres;         // ELL slots of each slice kept in shared memory (the rest read from L2)
   int hoff, nh;     // its halo: columns outside its rows, CgrArgs::h_col[hoff ..]
   int loff;         // its slots' local column indices, CgrArgs::lidx[loff ..] in slot order
-  int rec0, nrec;   // the scene's exchange records: first, count
+  int rec0, nrec;   // the scene's exchange records (tiles; slices in FP64): first, count
   int rec;          // the block's first record among them
   int row0;         // the scene's first row in the exchanged vector
   int nblk;         // blocks of the scene
-  int tile;         // 1: the block is one or two reduction tiles (of 8 slices) and sends their sums;
-                    // 0: it sends its slices' sums
+  int spb;          // FP64: slices a block (1, 2 or 4; the last block may have fewer)
 };
 
 struct CgrArgs {
@@ -40,7 +39,7 @@ struct CgrArgs {
 
 constexpr int kCgrTile = kCgRows / 32;  // slices of a reduction tile
 constexpr int kCgrMaxSlices = 16;       // slices of a block
-constexpr int kCgrMaxSliceTiles = 96;   // reduction tiles of a scene whose blocks send slice sums
+constexpr int kCgrMaxTiles64 = 96;      // reduction tiles of an FP64 scene
 
 // Dynamic shared memory of a block with `slots` resident slots, `own` rows
 // (32 per slice) and `nh` halo columns.
@@ -48,13 +47,13 @@ constexpr size_t cgr_smem(bool fp64, bool fused, bool jacobi, size_t slots, size
   const size_t w = fp64 ? 8 : 4;
   size_t b = slots * (288 * w + 64);                  // 9 planes and the column indices
   b += fp64 ? 24 * (own + nh) : 16 * (own + nh);      // the multiplied vector
-  if (fp64) b += 48 * own;                            // exchange between the component warps
+  if (fp64) b += 120 * own;                           // exchange between the warps of a slice
   if (fused) b += 16 * nh + (jacobi ? 0 : 16 * nh + 36 * nh);
   return b;
 }
 constexpr size_t kCgrSmem = 218 * 1024;  // dynamic shared memory a block may take
-constexpr int cgr_threads(bool fp64, int spb) { return fp64 ? (spb > 2 ? 384 : 256) : (spb > 8 ? 512 : 256); }
-constexpr int kCgrMaxSpb64 = 4;  // three component warps a slice
+constexpr int cgr_threads(bool fp64, int spb) { return fp64 ? 384 : (spb > 8 ? 512 : 256); }
+constexpr int kCgrMaxSpb64 = 4;  // twelve warps: 3 components x 4, 2 or 1 parts of the slots
 
 // Blocks per SM that can be resident with this much dynamic shared memory.
 int cgr_blocks_per_sm(bool fp64, bool fused, bool jacobi, int threads, size_t smem);

@@ -90,3 +90,13 @@ def test_lanes_of_resident_batches_side_by_side(gpu_lib):
         assert np.array_equal(x.positions(), y.positions())
     lanes.close()
     one.close()
+
+
+# (free rows: 4,864 and 4,896, the last with one slice a block and the first
+# with two; 9,728 and 9,760, two and four; 17,550: 69 tiles, the sum's third group)
+@pytest.mark.parametrize("dims", [(19, 15, 15), (17, 17, 15), (19, 15, 31), (61, 15, 9), (26, 26, 24)])
+def test_fp64_blocks_of_one_two_and_four_slices(gpu_lib, dims):
+    kw = dict(max_iterative_solver_iters=40)
+    a, b = run(spec(dims, D, PERS, **kw), 1), run(spec(dims, D, SPLIT, **kw), 1)
+    assert a[2] > 0 and b[2] == 0
+    same(a, b)
