@@ -115,11 +115,14 @@ __device__ __forceinline__ double fetch_sum(const uint4* rec, int n, unsigned se
 
 // num / den for a den whose correctly rounded reciprocal is at hand: one
 // product and one correction of the remainder give the correctly rounded
-// quotient (Markstein 1990), in 3 instead of the division's 9 latencies.
+// quotient (Markstein 1990), in 3 instead of the division's 9 latencies.  (The
+// division proper, where a reciprocal or product is out of range, is a call:
+// inlined, both would be computed each time.)
+__device__ __noinline__ inline double quotient(double num, double den) { return num / den; }
 __device__ __forceinline__ double quotient_by(double num, double den, double rcp) {
   const double q = num * rcp;
   const double v = fma(fma(-den, q, num), rcp, q);
-  return isfinite(v) ? v : num / den;
+  return isfinite(v) ? v : quotient(num, den);
 }
 
 }  // namespace mfem_gpu

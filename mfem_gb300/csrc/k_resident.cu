@@ -515,11 +515,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
 // four sums, see RowSum); the warps of part 0 own the rows' components.  A
 // slice's sums, the adding of the other blocks' and the scalars are one warp's
 // each, and the quotient by a number known before is a product with its
-// reciprocal, corrected (quotient_by).  An iteration at 90 / 1300 rows: 8.0 /
-// 8.5 us, against 10.2 / 11.5 with a slice's component in one warp and the sums
-// and scalars in every warp, and 34 / 38 in k_cg_solve.  Of the 16,100 cycles
+// reciprocal, corrected (quotient_by).  An iteration at 90 / 1300 rows: 7.9 /
+// 8.1 us, against 10.2 / 11.5 with a slice's component in one warp and the sums
+// and scalars in every warp, and 34 / 38 in k_cg_solve.  Of the 15,600 cycles
 // at 1300 rows the product is 3400 (its 180 warp instructions a slice at the
-// pipe's rate), the two exchanges 5000, trees and divisions 4500.
+// pipe's rate), the two exchanges 5000, trees and divisions 4000.
 constexpr int kThreads64 = 384;
 __global__ void __launch_bounds__(kThreads64, 1) k_cgr_split64(const CgrArgs A) {
   extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
@@ -638,17 +638,16 @@ __global__ void __launch_bounds__(kThreads64, 1) k_cgr_split64(const CgrArgs A) 
       double v = 0.0;
       // (at most 96 tiles: three trees over 32, then 0 + 2 and that + 1, the
       // order of the tree over eight)
-      double g[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-        if (32 * j < nt) {  // warp-uniform
-          double e = 32 * j + lane < nt ? tile[warp][32 * j + lane] : 0.0;
-          for (int off = nt - 32 * j > 16 ? 16 : nt - 32 * j > 8 ? 8 : nt - 32 * j > 4 ? 4 : nt - 32 * j > 2 ? 2 : 1;
-               off > 0; off >>= 1)
-            e += shfl_down(e, off);
-          g[j] = e;
-        }
-      v = nt > 64 ? (g[0] + g[2]) + g[1] : nt > 32 ? g[0] + g[1] : g[0];
+#pragma unroll 1
+      for (int i = 0; i < 3; ++i) {
+        const int j = i ? 3 - i : 0, m = nt - 32 * j;
+        if (m <= 0) continue;
+        double e = lane < m ? tile[warp][32 * j + lane] : 0.0;
+#pragma unroll 1
+        for (int off = 16; off > 0; off >>= 1)
+          if (off < m) e += shfl_down(e, off);
+        v = i ? v + e : e;
+      }
       if (lane == 0) {
         tot[warp] = v;
         then(warp, v);
@@ -696,24 +695,29 @@ __global__ void __launch_bounds__(kThreads64, 1) k_cgr_split64(const CgrArgs A) 
     double a[4] = {0.0, 0.0, 0.0, 0.0};  // of part pt: slots k = j mod 4, j = pt (4 parts), 2 pt, 2 pt + 1 (2), all (1)
     if (roww) {
       const int per = 4 / parts;
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j < per) {
-          const double* m = M.mat + 96 * comp + lane;
-          int k = per * pt + j;
-#pragma unroll 5
-          for (; k < M.res; k += 4) {
-            const double* u = vec + 3 * (int)M.li[32 * k + lane];
-            a[j] = fma(m[288 * k + 64], u[2], fma(m[288 * k + 32], u[1], fma(m[288 * k], u[0], a[j])));
-          }
-          for (; k < M.len; k += 4) {
-            const double* u = vec + 3 * (int)M.gli[32 * k + lane];
-            const double m0 = M.gell[ell_entry(M.soff, k, lane, 3 * comp)],
-                         m1 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 1)],
-                         m2 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 2)];
-            a[j] = fma(m2, u[2], fma(m1, u[1], fma(m0, u[0], a[j])));
-          }
+#pragma unroll 1
+      for (int j = 0; j < per; ++j) {
+        const double* m = M.mat + 96 * comp + lane;
+        double e = 0.0;
+        int k = per * pt + j;
+#pragma unroll 1
+        for (; k < M.res; k += 4) {
+          const double* u = vec + 3 * (int)M.li[32 * k + lane];
+          e = fma(m[288 * k + 64], u[2], fma(m[288 * k + 32], u[1], fma(m[288 * k], u[0], e)));
         }
+#pragma unroll 1
+        for (; k < M.len; k += 4) {
+          const double* u = vec + 3 * (int)M.gli[32 * k + lane];
+          const double m0 = M.gell[ell_entry(M.soff, k, lane, 3 * comp)],
+                       m1 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 1)],
+                       m2 = M.gell[ell_entry(M.soff, k, lane, 3 * comp + 2)];
+          e = fma(m2, u[2], fma(m1, u[1], fma(m0, u[0], e)));
+        }
+        a[0] = j == 0 ? e : a[0];
+        a[1] = j == 1 ? e : a[1];
+        a[2] = j == 2 ? e : a[2];
+        a[3] = j == 3 ? e : a[3];
+      }
       if (parts == 4) {
         if (pt > 0) sums[96 * B.nsl * (pt - 1) + ex_at] = a[0];
       } else if (parts == 2 && pt == 1) {
