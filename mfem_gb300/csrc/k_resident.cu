@@ -52,7 +52,6 @@ template <> __device__ __forceinline__ df64 rec_val<df64>(uint4 v) {
 __device__ __forceinline__ df64 shfl_to(df64 v, int lane) {
   return df64(__shfl_sync(0xffffffffu, v.hi, lane), __shfl_sync(0xffffffffu, v.lo, lane));
 }
-__device__ __forceinline__ double shfl_to(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
 
 template <typename E, int NQ, int kFrom>
 __device__ __forceinline__ void tree(E (&v)[NQ]) {
@@ -75,10 +74,11 @@ struct CgrShared {
 // trees over absent entries only add zeros.)  A block sends the sums of its
 // one or two tiles, a scene of one block nothing.  `ahead` runs once the
 // other blocks' sums have come in, before the last of the adding: loads issued
-// there are under way meanwhile.  False: a wait ran out.
-template <typename E, int NQ, typename F>
+// there are under way meanwhile; `during` before, while the sums travel.
+// False: a wait ran out.
+template <typename E, int NQ, typename F, typename G>
 __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B, CgrShared& S, bool lead, int sl,
-                                            unsigned seq, E (&v)[NQ], const F& ahead) {
+                                            unsigned seq, E (&v)[NQ], const F& ahead, const G& during) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int par = seq & 1;
   const int copies = exchange_copies(B.nblk);
@@ -104,6 +104,7 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
       if (nt > 1) v[q] = radd(v[q], shfl_to(v[q], 8));
       v[q] = shfl_to(v[q], 0);
     }
+    during();
     ahead();
     return true;
   }
@@ -113,6 +114,7 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
     tree<E, 1, 4>(a);
     send(q, B.rec + t, a[0]);
   }
+  during();
   const int n = B.nrec;
   // the sums of record i (0 for lanes without one), the warp in step
   auto fetch = [&](int i, E (&a)[NQ]) -> bool {
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) d1[0] = acc_prod(d1[0], p[c], acc[c]);
     }
-    if (!scene_total<E, 1>(A, B, S, roww, sl, seq, d1, nothing)) {
+    if (!scene_total<E, 1>(A, B, S, roww, sl, seq, d1, nothing, nothing)) {
       cgr_abort(A, B);
       return;
     }
@@ -404,7 +406,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
       if (!replace) publish_z(seq);
     }
     if (replace) __syncthreads();  // every row's x_e is visible before the block's sums
-    if (!scene_total<E, 2>(A, B, S, roww, sl, seq, d2, halo_ahead)) {
+    if (!scene_total<E, 2>(A, B, S, roww, sl, seq, d2, halo_ahead, nothing)) {
       cgr_abort(A, B);
       return;
     }
@@ -465,7 +467,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
         }
         publish_z(seq);
       }
-      if (!scene_total<E, 2>(A, B, S, roww, sl, seq, d3, halo_ahead)) {
+      if (!scene_total<E, 2>(A, B, S, roww, sl, seq, d3, halo_ahead, nothing)) {
         cgr_abort(A, B);
         return;
       }
@@ -821,6 +823,60 @@ __global__ void __launch_bounds__(kThreads64, 1) k_cgr_split64(const CgrArgs A) 
 // iteration done: until the recursion's stop is to be verified (cgf_phase set:
 // the next launches of k_cgf_iter verify), or max_iters iterations.  The
 // exchanged vector is w; each block keeps r and s at its halo.
+struct CgfScalars {
+  df64 gamma, alphaE, betaE, rr0, rr, rg, ra;
+  float a, b;
+  int it, rounds, phase, status, cg_status;
+  bool swapped;  // an iteration left the recursion without counting (phase set)
+
+  __device__ __forceinline__ explicit CgfScalars(const SceneScalars* sc)
+      : gamma(sc_get<df64>(&sc->cgf_gamma[0])), alphaE(sc_get<df64>(&sc->alpha)), betaE(sc_get<df64>(&sc->beta)),
+        rr0(sc_get<df64>(&sc->cg_rhs_norm2)), rr(rr0), a(sc->alpha_f), b(sc->beta_f), it(sc->cg_iter),
+        rounds(sc->cgf_rounds), phase(0), status(0), cg_status(0), swapped(false) {}
+  // While the sums travel.
+  __device__ __forceinline__ void prepare() {
+    rg = df64(1.f) / gamma;
+    ra = df64(1.f) / alphaE;
+  }
+  // After an iteration's sums, as cgf_verify_step in phase 0: whether the launch ends.
+  __device__ __forceinline__ bool step(const SceneDev& sd, const df64 (&d)[3]) {
+    rr = d[0];
+    if (is_nan(rr)) {
+      status = 4;
+      phase = 3;
+    } else if (cg_meets(sd, rr, rr0)) {
+      phase = rounds < kCgfRounds ? 1 : 3;
+    }
+    if (phase) {
+      swapped = true;
+      return true;
+    }
+    cgf_steps(d[1], d[2], rg, ra, &alphaE, &betaE);
+    gamma = d[1];
+    a = to_step(alphaE);
+    b = to_step(betaE);
+    it += 1;
+    if (it >= sd.max_cg) {
+      cg_status = 5;  // MFEM_ERR_CG_MAXITER
+      phase = 3;
+      return true;
+    }
+    return false;
+  }
+  __device__ __forceinline__ void store(SceneScalars* sc) const {
+    sc->cg_err = cg_rel(rr, rr0);
+    sc_put(&sc->beta, betaE);
+    sc->beta_f = b;
+    sc_put(&sc->alpha, alphaE);
+    sc->alpha_f = a;
+    sc_put(&sc->cgf_gamma[0], gamma);
+    sc->cg_iter = it;
+    sc->cgf_phase = phase;
+    if (status) sc->status = status;
+    if (cg_status) sc->cg_status = cg_status;
+  }
+};
+
 template <bool kScaled, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
   extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
@@ -841,8 +897,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
   float4* sh = u4 + own + B.nh;                         // s at the halo
   float4* rh = kScaled ? u4 + own : sh + B.nh;          // r at the halo (scaled: u itself)
   float* Dh = reinterpret_cast<float*>(sh + 2 * B.nh);  // unscaled: M^-1 at the halo, 9 each
-  const int it0 = sc->cg_iter;
-  int it = it0;
+  CgfScalars q(sc);
+  const int it = q.it;
   const float* gr = static_cast<const float*>(sd.cgf_r[it & 1]);
   const float* gw = static_cast<const float*>(sd.cgf_w[it & 1]);
   const float* gs = static_cast<const float*>(sd.cgf_s[(it + 1) & 1]);
@@ -881,17 +937,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
     if (kScaled) ld3<false>(static_cast<const float*>(sd.dinv) + k4, dv);
     else ld3<false>(static_cast<const float*>(sd.cg_z) + k4, u);
   }
-  df64 gamma = sc_get<df64>(&sc->cgf_gamma[0]), alphaE = sc_get<df64>(&sc->alpha), betaE = sc_get<df64>(&sc->beta);
-  const df64 rr0 = sc_get<df64>(&sc->cg_rhs_norm2);
-  float a = sc->alpha_f, b = sc->beta_f;
-  const int rounds = sc->cgf_rounds;
-  int phase = 0, status = 0, cg_status = 0;
-  df64 rr = rr0;
   unsigned wtag = 0;
-  bool swapped = false;  // an iteration left the recursion without counting (phase set)
 
   for (int n = 0;; ++n) {
     const bool first = n == 0;
+    const float a = q.a, b = q.b;
     // ---- own rows: s, r, u, p, x of iteration it + 1
     float rn[3], un[3];
     if (live) {
@@ -984,38 +1034,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
 #pragma unroll
           for (int j = 0; j < kHaloRegs; ++j)
             if (hw[j]) hv[j] = ld_rec(A.pub + (size_t)(seq & 1) * A.pub_stride + B.row0 + hc[j]);
-        })) {
+        }, [&]() { q.prepare(); })) {
       cgr_abort(A, B);
       return;
     }
     wtag = seq;
     ++seq;
-    // ---- cgf_verify_step, phase 0
-    rr = d[0];
-    if (is_nan(rr)) {
-      status = 4;
-      phase = 3;
-    } else if (cg_meets(sd, rr, rr0)) {
-      phase = rounds < kCgfRounds ? 1 : 3;
-    }
-    if (phase) {
-      swapped = true;
-      break;
-    }
-    cgf_steps(d[1], d[2], gamma, alphaE, &alphaE, &betaE);
-    gamma = d[1];
-    a = to_step(alphaE);
-    b = to_step(betaE);
-    it += 1;
-    if (it >= sd.max_cg) {
-      cg_status = 5;  // MFEM_ERR_CG_MAXITER
-      phase = 3;
-      break;
-    }
+    if (q.step(sd, d)) break;
     if (n + 1 >= A.max_iters) break;
   }
   // ---- the vectors as k_cgf_iter leaves them after iteration `last`
-  const int last = swapped ? it : it - 1;
+  const int last = q.swapped ? q.it : q.it - 1;
   if (live) {
     st3(static_cast<float*>(sd.cgf_r[(last + 1) & 1]) + k4, r);
     st3(static_cast<float*>(sd.cgf_w[(last + 1) & 1]) + k4, w);
@@ -1025,16 +1054,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
     if (!kScaled) st3(static_cast<float*>(sd.cg_z) + k4, u);
   }
   if (B.rec == 0 && threadIdx.x == 0) {
-    sc->cg_err = cg_rel(rr, rr0);
-    sc_put(&sc->beta, betaE);
-    sc->beta_f = b;
-    sc_put(&sc->alpha, alphaE);
-    sc->alpha_f = a;
-    sc_put(&sc->cgf_gamma[0], gamma);
-    sc->cg_iter = it;
-    sc->cgf_phase = phase;
-    if (status) sc->status = status;
-    if (cg_status) sc->cg_status = cg_status;
+    q.store(sc);
     A.seq[B.scene] = seq;
   }
 }

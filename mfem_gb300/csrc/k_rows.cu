@@ -638,7 +638,7 @@ __device__ __forceinline__ void cgf_finish(const SceneDev& sd, BatchCounters* ct
           stop = true;
         } else {
           E an, bn;
-          cgf_steps(g, d, sc_get<E>(&sc->cgf_gamma[0]), sc_get<E>(&sc->alpha), &an, &bn);
+          cgf_steps(g, d, E(1) / sc_get<E>(&sc->cgf_gamma[0]), E(1) / sc_get<E>(&sc->alpha), &an, &bn);
           sc_put(&sc->beta, bn);
           sc_put(&sc->alpha, an);
           sc_put(&sc->cgf_gamma[0], g);
