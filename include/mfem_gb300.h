@@ -93,7 +93,8 @@ enum { MFEM_FORMULATION_MIXED_STRETCH = 0, MFEM_FORMULATION_STRETCH = 1 };
  * SPLIT in between.  A batch of PERSISTENT, or of AUTO where it picked SPLIT
  * or at most four tiles, runs each solve as one launch with the matrix
  * resident in shared memory if that fits (up to two tiles per SM; FP64 up to
- * 128 rows per SM), with the results of the picked form's launches, bitwise;
+ * 128 rows per SM), or, where AUTO picked FUSED, streamed through it (up to
+ * six tiles per SM), with the results of the picked form's launches, bitwise;
  * mfem_gpu_batch_step_n runs FUSED batches that way too. */
 enum { MFEM_PCG_KERNEL_PERSISTENT = 0, MFEM_PCG_KERNEL_SPLIT = 1, MFEM_PCG_KERNEL_FUSED = 2,
        MFEM_PCG_KERNEL_AUTO = 3 };

@@ -11,6 +11,8 @@
 //   Newton loop       src/optimizers/newton_optimizer.cpp:11-89
 #include <cuda_runtime.h>
 
+#include <limits.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -566,6 +568,7 @@ struct mfem_batch {
   CgrArgs cgr_args{};
   int cgr_blocks = 0, cgr_nthreads = 0;
   size_t cgr_smem_bytes = 0;
+  bool cgr_wide = false;
   bool loop_resident = false;  // the PCG loop graph's body starts with the resident solve
   int pstride = 0;  // tiles per partials quantity
   // instrumentation
@@ -894,7 +897,12 @@ int worst_status(const SceneScalars& sc) {
 // as many neighbouring pairs of tiles as it takes go to one block, those of a
 // scene's short last tile first (320k tets, 263 tiles: 12.9 us, against 15.2 us
 // with two blocks an SM and 25.4 us for the launches); a scene of two tiles
-// alone is one block (350 rows: 6.2 us, against 8.2 us with two).  FP64: the
+// alone is one block (350 rows: 6.2 us, against 8.2 us with two).  More than
+// two tiles an SM (single-reduction form): the fewest tiles a block, three to
+// six, for which every block has an SM, in the form that streams the matrix
+// (338 / 873 tiles: 17.9 / 32.0 us, against 25.4 / 37.9 us for the launches); a
+// block's slices go to its warps by length, the longest to the warp with the
+// fewest slots, since a tile's rows are sorted by length.  FP64: the
 // fewest slices of 1, 2 and 4 for which every block has an SM of its own, for
 // a slice's product is 3400 cycles of its SM's FP64 pipe.  False: the batch
 // does not fit, or its form has no resident kernel.
@@ -923,7 +931,19 @@ bool cgr_plan(mfem_batch* b) {
     }
     if (!fp64 || total <= sms || spb >= kCgrMaxSpb64) break;
   }
-  if (!fp64 && total > sms) {
+  const bool wide = fused && total > 2 * sms;
+  if (wide) {
+    // the fewest tiles a block for which every block has an SM
+    for (spb = 3 * kCgrTile; spb <= kCgrWideSlices; spb += kCgrTile) {
+      total = 0;
+      for (int i = 0; i < n; ++i) {
+        first[i].clear();
+        for (int s = 0; s < (b->scenes[i]->M.nf + 31) / 32; s += spb) first[i].push_back(s);
+        total += (long)first[i].size();
+      }
+      if (total <= sms) break;
+    }
+  } else if (!fp64 && total > sms) {
     if (total > 2 * sms) return false;
     struct Pair { int slices, scene, block; };
     std::vector<Pair> pairs;
@@ -955,6 +975,7 @@ bool cgr_plan(mfem_batch* b) {
   std::vector<CgrBlock> blocks;
   std::vector<int> h_col;
   std::vector<uint16_t> lidx;
+  std::vector<unsigned char> pick;
   size_t rows = 0, smem = 0;
   int nrec = 0;
   for (int i = 0; i < n; ++i) {
@@ -962,7 +983,7 @@ bool cgr_plan(mfem_batch* b) {
     if (M.nf == 0) return false;
     const int ns = (M.nf + 31) / 32, nblk = (int)first[i].size();
     const int ntile = (ns + kCgrTile - 1) / kCgrTile;
-    if (fp64 && ntile > kCgrMaxTiles64) return false;
+    if (ntile > (fp64 ? kCgrMaxTiles64 : wide ? kCgrWideTiles : INT_MAX)) return false;
     std::vector<int> local(M.nf, -1);
     for (int k = 0; k < nblk; ++k) {
       CgrBlock B{};
@@ -1002,6 +1023,31 @@ bool cgr_plan(mfem_batch* b) {
         return t;
       };
       int kres = kMaxRowBlocks + 1;
+      if (wide) {
+        kres = 64;
+        while (kres >= 3 && cgr_wide_smem(kres, own, B.nh) > kCgrSmem) --kres;
+        if (kres < 3) return false;
+        B.kres = kres;
+        // three slices a warp, the longest first to the warp with the fewest slots
+        std::vector<std::pair<int, int>> by_len;
+        for (int s = 0; s < B.nsl; ++s)
+          by_len.push_back({M.slice_off[B.slice0 + s] - M.slice_off[B.slice0 + s + 1], s});
+        std::sort(by_len.begin(), by_len.end());
+        constexpr int warps = kCgrWideWarps, per_warp = kCgrWideSlices / warps;
+        int sum[warps] = {}, cnt[warps] = {};
+        pick.resize(pick.size() + kCgrWideSlices, 255);
+        unsigned char* mine = pick.data() + pick.size() - kCgrWideSlices;
+        for (const auto& e : by_len) {
+          int w = -1;
+          for (int i = 0; i < warps; ++i)
+            if (cnt[i] < per_warp && (w < 0 || sum[i] < sum[w])) w = i;
+          mine[per_warp * w + cnt[w]++] = (unsigned char)e.second;
+          sum[w] -= e.first;
+        }
+        smem = std::max(smem, cgr_wide_smem(kres, own, B.nh));
+        blocks.push_back(B);
+        continue;
+      }
       while (kres >= 0 && cgr_smem(fp64, fused, b->jacobi, slots(kres), own, B.nh) > kCgrSmem) --kres;
       if (kres < 0) return false;
       B.kres = kres;
@@ -1012,14 +1058,16 @@ bool cgr_plan(mfem_batch* b) {
     rows += M.nf;
   }
   smem = std::max(smem, kCgrSmem / 2 + 8 * 1024);  // every block an SM of its own
-  const int threads = cgr_threads(fp64, spb);
-  if ((long)cgr_blocks_per_sm(fp64, fused, b->jacobi, threads, smem) * sms < (long)blocks.size()) return false;
+  const int threads = cgr_threads(fp64, spb);  // 512 in the wide form
+  if ((long)cgr_blocks_per_sm(fp64, fused, b->jacobi, wide, threads, smem) * sms < (long)blocks.size()) return false;
   const size_t pub = rows * (fp64 ? 3 : 1);
   CgrArgs& a = b->cgr_args;
+  unsigned char* pick_dev = nullptr;
   auto lay = [&](Arena& A) {
     a.blocks = A.take<CgrBlock>(blocks.size());
     a.h_col = A.take<int>(std::max<size_t>(h_col.size(), 1));
     a.lidx = A.take<uint16_t>(std::max<size_t>(lidx.size(), 1));
+    pick_dev = A.take<unsigned char>(std::max<size_t>(pick.size(), 1));
     a.recs = A.take<uint4>(2 * kMaxCopies * 3 * (size_t)nrec);
     a.pub = A.take<uint4>(2 * pub);
     a.seq = A.take<unsigned int>(n);
@@ -1034,6 +1082,8 @@ bool cgr_plan(mfem_batch* b) {
   Arena real;
   real.base = b->cgr_mem;
   lay(real);
+  if (wide)
+    for (size_t k = 0; k < blocks.size(); ++k) blocks[k].pick = pick_dev + kCgrWideSlices * k;
   a.nrec_total = nrec;
   a.pub_stride = pub;
   a.sds = b->d_sds;
@@ -1046,6 +1096,7 @@ bool cgr_plan(mfem_batch* b) {
   const bool ok = cudaMemsetAsync(b->cgr_mem, 0, dry.used, b->stream) == cudaSuccess &&
                   up(a.blocks, blocks.data(), sizeof(CgrBlock) * blocks.size()) &&
                   up(a.h_col, h_col.data(), sizeof(int) * h_col.size()) &&
+                  up(pick_dev, pick.data(), pick.size()) &&
                   up(a.lidx, lidx.data(), sizeof(uint16_t) * lidx.size()) &&
                   up(a.seq, seq.data(), sizeof(unsigned int) * n) &&
                   cudaStreamSynchronize(b->stream) == cudaSuccess;
@@ -1058,6 +1109,7 @@ bool cgr_plan(mfem_batch* b) {
   b->cgr_blocks = (int)blocks.size();
   b->cgr_nthreads = threads;
   b->cgr_smem_bytes = smem;
+  b->cgr_wide = wide;
   b->cgr_state = 1;
   return true;
 }
@@ -1065,7 +1117,7 @@ bool cgr_plan(mfem_batch* b) {
 cudaError_t cgr_launch(mfem_batch* b, int max_iters) {
   CgrArgs a = b->cgr_args;
   a.max_iters = max_iters;
-  return launch_cgr(a, b->fp64 != 0, b->pcg_kernel == MFEM_PCG_KERNEL_FUSED, b->jacobi != 0, b->cgr_blocks,
+  return launch_cgr(a, b->fp64 != 0, b->pcg_kernel == MFEM_PCG_KERNEL_FUSED, b->jacobi != 0, b->cgr_wide, b->cgr_blocks,
                     b->cgr_nthreads, b->cgr_smem_bytes, b->stream);
 }
 

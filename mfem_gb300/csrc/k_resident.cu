@@ -32,6 +32,10 @@
 // leaves, as do the others when they see the flag or time out themselves; the
 // host reports MFEM_ERR_TIMEOUT.  The launch is cooperative: all blocks are
 // co-resident, the exchange needs them all.
+#include <new>
+#include <type_traits>
+
+#include "async_copy.cuh"
 #include "exchange.cuh"
 #include "pcg.cuh"
 #include "resident.cuh"
@@ -1059,7 +1063,419 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
   }
 }
 
-template <typename F> auto with_kernel(bool fp64, bool fused, bool jacobi, int threads, F&& f) {
+// The same iteration for batches whose matrices outgrow the shared memory of
+// all SMs (more than two tiles an SM; up to six).  A block is up to 48 slices,
+// a warp up to three, with their rows' vectors in registers; the matrix streams
+// through a ring of slots in shared memory, as in the staged k_cgf_iter, and
+// little else leaves the SM: the rows' u, their x and the sums, where the launch
+// per iteration reads three vectors at every neighbour and writes five.  The
+// ring runs on from one iteration into the next, so that it is full when the
+// sums of the last have come in.  The exchanged vector is u itself: the halo
+// takes 20 bytes of shared memory a column, and the iteration waits twice, for
+// the neighbours' rows and for the sums.
+//
+// An iteration at 85k / 130k / 148k / 223k rows: 17.9 / 21.3 / 21.6 / 32.0 us,
+// against 25.4 / 28.1 / 30.2 / 37.9 us in launches (block Jacobi: 18.3 / 21.9 /
+// 22.3 / 33.7 against 32.3 / 35.3 / 37.0 / 50.9).  Of the 62,000 cycles at 223k
+// rows the product is 30,000 (128 MB, 19 us of DRAM time, of which the L2 keeps
+// a quarter; a slot passes shared memory twice, 20,000 cycles), the own rows
+// 6,500, the halo 3,500, waiting for the slowest warp and block and the sums
+// the rest.  One slot at a time with its refill: 38,000 cycles for the product;
+// neighbouring slices in a warp, of unlike lengths: 36,000; the matrix in
+// registers from plain loads with a fifth of it resident: 62,000.  Prefetching
+// the next iteration's slots to L2 while the sums travel slowed the sums by
+// what it saved.
+constexpr int kCgrTake = 2;  // slots out of the ring at a time
+constexpr int kWideWarps = kCgrWideWarps, kWideThreads = 32 * kWideWarps, kWideSlices = kCgrWideSlices / kWideWarps;
+
+// `tree` over 32 lanes for N values at once: each level leaves one half of the
+// lanes one value of a pair and the other half the other, so that N values
+// take about N + 5 additions in place of 5 N.  (The pairs added are the
+// tree's, and an addition's operands may change places.)  Afterwards lane l
+// holds the value of index *i.
+template <int N, int kOff = 16>
+__device__ __forceinline__ df64 trees(const df64 (&v)[N], int* i) {
+  const int lane = threadIdx.x & 31;
+  const bool up = (lane & kOff) != 0;
+  constexpr int M = (N + 1) / 2;
+  df64 a[M];
+#pragma unroll
+  for (int j = 0; j < M; ++j) {
+    const df64 lo = v[2 * j], hi = v[2 * j + 1 < N ? 2 * j + 1 : 2 * j];
+    const df64 keep = up ? hi : lo, send = up ? lo : hi;
+    a[j] = keep + df64(__shfl_xor_sync(0xffffffffu, send.hi, kOff), __shfl_xor_sync(0xffffffffu, send.lo, kOff));
+  }
+  if constexpr (kOff > 1) {
+    const df64 t = trees<M, kOff / 2>(a, i);
+    *i = min(2 * *i + (up ? 1 : 0), N - 1);
+    return t;
+  } else {
+    static_assert(M == 1, "at most 32 values");
+    *i = min(up ? 1 : 0, N - 1);
+    return a[0];
+  }
+}
+
+template <bool kScaled>
+__global__ void __launch_bounds__(kWideThreads, 1) k_cgr_wide(const CgrArgs A) {
+  extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
+  __shared__ double part[3][kCgrWideSlices], red[3][8];
+  __shared__ int lens[kCgrWideSlices], offs[kCgrWideSlices], who[kCgrWideSlices];  // of the slices in the warps' order
+  __shared__ __align__(8) unsigned char q_raw[sizeof(CgfScalars)];
+  CgfScalars& q = *reinterpret_cast<CgfScalars*>(q_raw);
+  __shared__ int leave;
+  constexpr int kHalo = 4;
+  const CgrBlock B = A.blocks[blockIdx.x];
+  const SceneDev& sd = A.sds[B.scene];
+  SceneScalars* sc = sd.sc;
+  if (!sc->cg_active || sc->cgf_phase) return;
+  unsigned seq = __ldcg(A.seq + B.scene);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int* err = &A.ctrs->error;
+
+  // ---- the warp's slices (B.pick: of like numbers of slots in all warps) and
+  // its ring: S stages of a slot's 160 pairs and 32 local column indices, one
+  // mbarrier each; the slots of the slices one after another, over and over
+  const int first = kWideSlices * warp;
+  int sl[kWideSlices], nslots = 0, ns = 0;
+  const int soff0 = sd.slice_off[B.slice0];
+#pragma unroll
+  for (int j = 0; j < kWideSlices; ++j) {
+    sl[j] = B.pick[first + j];
+    if (sl[j] < B.nsl) {
+      const int off = sd.slice_off[B.slice0 + sl[j]], len = (sd.slice_off[B.slice0 + sl[j] + 1] - off) >> 5;
+      nslots += len;
+      ns = j + 1;
+      if (lane == 0) {
+        lens[first + j] = len;
+        offs[first + j] = off;
+        who[first + j] = sl[j];
+      }
+    }
+  }
+  __syncwarp();
+  const int own = 32 * B.nsl;
+  float4* u4 = reinterpret_cast<float4*>(cgr_smem_raw);  // u at the own rows and the halo
+  int* hcol = reinterpret_cast<int*>(u4 + own + B.nh);  // the halo's columns
+  for (int h = threadIdx.x; h < B.nh; h += kWideThreads) hcol[h] = A.h_col[B.hoff + h];
+  const uint32_t ring = smem_addr(hcol + (B.nh + 3) / 4 * 4);
+  const uint32_t bar0 = ring + 8u * (uint32_t)(warp * B.kres);
+  const uint32_t stage0 = ring + 8u * (uint32_t)(kWideWarps * B.kres) +
+                          kCgrStage * (uint32_t)(warp * B.kres);
+  const float2* ell = static_cast<const float2*>(sd.ell);
+  const uint16_t* gli = A.lidx + B.loff;
+  const int S = min(B.kres, nslots);
+  // the slot the next fill fetches (lane 0): slice, slots left of it, addresses
+  int fj = -1, frem = 0;
+  const float2* fe = ell;
+  const uint16_t* fl = gli;
+  const unsigned long long pol = l2_matrix_policy<2>();
+  auto to_next = [&]() {
+    fj = fj + 1 == ns ? 0 : fj + 1;
+    frem = lens[first + fj];
+    fe = ell + 5 * (size_t)offs[first + fj];
+    fl = gli + (offs[first + fj] - soff0);
+  };
+  auto fill = [&](int stage) {
+    const uint32_t bar = bar0 + 8u * stage, dst = stage0 + kCgrStage * stage;
+    mbar_arrive_expect_tx(bar, kCgrStage);
+    bulk_g2s(dst, fe, 1280u, bar, pol);
+    bulk_g2s(dst + 1280u, fl, 64u, bar, pol);
+    fe += 160;
+    fl += 32;
+    if (--frem == 0) to_next();
+  };
+  if (lane == 0)
+    for (int i = 0; i < S; ++i) mbar_init(bar0 + 8u * i, 1u);
+  fence_mbar_init();
+  __syncwarp();
+  if (lane == 0 && S > 0) {
+    to_next();
+    for (int i = 0; i < S; ++i) fill(i);
+  }
+  int st = 0;          // the stage read next
+  uint32_t round = 0;  // its parity
+  // every copy in flight lands before the block leaves (S of them, always)
+  auto drain = [&]() {
+    for (int i = 0; i < S; ++i) {
+      mbar_wait(bar0 + 8u * st, round);
+      st = st + 1 == S ? 0 : st + 1;
+      round ^= st == 0;
+    }
+    __syncwarp();
+  };
+
+  // ---- the rows' vectors
+  if (threadIdx.x == 0) new (&q) CgfScalars(sc);
+  const int it = sc->cg_iter;
+  const float* gr = static_cast<const float*>(sd.cgf_r[it & 1]);
+  const float* gw = static_cast<const float*>(sd.cgf_w[it & 1]);
+  const float* gs = static_cast<const float*>(sd.cgf_s[(it + 1) & 1]);
+  // (u, which is the scaled r, stays in u4); dr: M^-1 (scaled) or r
+  float w[kWideSlices][3], sv[kWideSlices][3], p[kWideSlices][3], dr[kWideSlices][3];
+  float* gx = static_cast<float*>(sd.cg_x);  // x: read and written once an iteration, off the chain
+  bool live[kWideSlices];
+#pragma unroll
+  for (int j = 0; j < kWideSlices; ++j) {
+    const int row = 32 * (B.slice0 + sl[j]) + lane;
+    live[j] = j < ns && row < sd.nf;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) w[j][c] = sv[j][c] = p[j][c] = dr[j][c] = 0.f;
+    if (live[j]) {
+      const size_t k4 = 4 * (size_t)row;
+      ld3<false>(gw + k4, w[j]);
+      ld3<false>(gs + k4, sv[j]);
+      ld3<false>(static_cast<const float*>(sd.cg_p[0]) + k4, p[j]);
+      float u[3];
+      ld3<false>(kScaled ? static_cast<const float*>(sd.dinv) + k4 : gr + k4, dr[j]);
+      ld3<false>(kScaled ? gr + k4 : static_cast<const float*>(sd.cg_z) + k4, u);
+      u4[32 * sl[j] + lane] = make_float4(u[0], u[1], u[2], 0.f);
+    }
+  }
+  uint4* pub = A.pub + B.row0;
+  const int copies = exchange_copies(B.nblk);
+  const size_t cstride = 3 * (size_t)A.nrec_total;
+  __syncthreads();
+
+  for (int n = 0;; ++n) {
+    const float a = q.a, b = q.b;
+    // ---- own rows: s, r, u, p, x of iteration it + 1; (r, r), (r, u)
+    {
+      df64 e[2 * kWideSlices];
+#pragma unroll
+      for (int j = 0; j < kWideSlices; ++j) {
+        const int row = 32 * (B.slice0 + sl[j]) + lane;
+        float un[3] = {0.f, 0.f, 0.f};
+        e[2 * j] = e[2 * j + 1] = df64(0.f);
+        if (live[j]) {
+          float rn[3], sn[3];
+          const float4 u = u4[32 * sl[j] + lane];
+          const float uv[3] = {u.x, u.y, u.z};
+          if (kScaled) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              sn[c] = fma(b, sv[j][c], w[j][c]);
+              un[c] = fma(-a, sn[c], uv[c]);
+              rn[c] = un[c] / dr[j][c];
+            }
+          } else {
+            cgf_next<float>(sd, row, dr[j], w[j], sv[j], a, b, sn, rn, un);
+          }
+          if (B.nblk > 1)
+            st_rec(pub + row,
+                   make_uint4(__float_as_uint(un[0]), __float_as_uint(un[1]), __float_as_uint(un[2]), seq));
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            p[j][c] = fma(b, p[j][c], uv[c]);
+            sv[j][c] = sn[c];
+            if (!kScaled) dr[j][c] = rn[c];
+            e[2 * j] = acc_prod(e[2 * j], rn[c], rn[c]);
+            e[2 * j + 1] = acc_prod(e[2 * j + 1], rn[c], un[c]);
+          }
+        }
+        if (j < ns) u4[32 * sl[j] + lane] = make_float4(un[0], un[1], un[2], 0.f);
+      }
+      int i;
+      const df64 t = trees(e, &i);
+      if ((i >> 1) < ns) Slot<df64>::put(&part[i & 1][who[first + (i >> 1)]], t);
+    }
+    // ---- the halo's u
+    bool ok = true;
+    for (int h0 = 32 * warp; h0 < B.nh; h0 += kHalo * kWideThreads) {
+      uint4 v[kHalo];
+      bool want[kHalo];
+      int col[kHalo];
+#pragma unroll
+      for (int j = 0; j < kHalo; ++j) {
+        const int h = h0 + j * kWideThreads + lane;
+        want[j] = h < B.nh;
+        col[j] = want[j] ? hcol[h] : 0;
+      }
+#pragma unroll
+      for (int j = 0; j < kHalo; ++j)
+        if (want[j]) v[j] = ld_rec(pub + col[j]);
+      ok = poll_recs<kHalo>(v, [&](int j) { return pub + col[j]; }, want, seq, err) && ok;
+#pragma unroll
+      for (int j = 0; j < kHalo; ++j)
+        if (want[j])
+          u4[own + h0 + j * kWideThreads + lane] =
+              make_float4(__uint_as_float(v[j].x), __uint_as_float(v[j].y), __uint_as_float(v[j].z), 0.f);
+    }
+    if (!__syncthreads_and(ok)) {
+      drain();
+      cgr_abort(A, B);
+      return;
+    }
+    // ---- w = A u, (w, u)
+    float aw[kWideSlices][3];
+#pragma unroll 1
+    for (int j = 0; j < ns && ok; ++j) {
+      float acc[3] = {0.f, 0.f, 0.f};
+      const int len = lens[first + j];
+      // n slots: out of their stages, the stages refilled, the products
+      auto take = [&](auto n_) -> bool {
+        constexpr int n = decltype(n_)::value;
+        int at[n];
+        bool got = true;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          at[i] = st;
+          got = mbar_wait(bar0 + 8u * st, round) && got;
+          st = st + 1 == S ? 0 : st + 1;
+          round ^= st == 0;
+        }
+        if (!__all_sync(0xffffffffu, got)) return false;
+        float2 e[n][5];
+        unsigned short col[n];
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          const uint32_t src = stage0 + kCgrStage * at[i];
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(col[i]) : "r"(src + 1280u + 2u * lane) : "memory");
+#pragma unroll
+          for (int c = 0; c < 5; ++c) e[i][c] = lds_pair(src + 256u * c + 8u * lane, 0.f);
+        }
+        __syncwarp();
+        if (lane == 0) {
+          fence_proxy_async_smem();
+#pragma unroll
+          for (int i = 0; i < n; ++i) fill(at[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          const float4 t = u4[col[i]];
+          const float uc[3] = {t.x, t.y, t.z};
+          ell_block_fma(e[i][0], e[i][1], e[i][2], e[i][3], e[i][4], uc, acc[0], acc[1], acc[2]);
+        }
+        return true;
+      };
+      int k = 0;
+#pragma unroll 1
+      for (; ok && k + kCgrTake <= len; k += kCgrTake) ok = take(std::integral_constant<int, kCgrTake>());
+#pragma unroll 1
+      for (; ok && k < len; ++k) ok = take(std::integral_constant<int, 1>());
+#pragma unroll
+      for (int i = 0; i < kWideSlices; ++i)
+        if (i == j)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) aw[i][c] = acc[c];
+    }
+    if (!ok && lane == 0) atomicExch(err, 1);
+    {
+      df64 e[kWideSlices];
+#pragma unroll
+      for (int j = 0; j < kWideSlices; ++j) {
+        e[j] = df64(0.f);
+        if (live[j]) {
+          const float4 t = u4[32 * sl[j] + lane];
+          const float u[3] = {t.x, t.y, t.z};
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            w[j][c] = kScaled ? dr[j][c] * aw[j][c] : aw[j][c];
+            e[j] = acc_prod(e[j], aw[j][c], u[c]);
+          }
+        }
+      }
+      int i;
+      const df64 t = trees(e, &i);
+      if (i < ns) Slot<df64>::put(&part[2][who[first + i]], t);
+    }
+    if (!__syncthreads_and(ok)) {
+      drain();
+      cgr_abort(A, B);
+      return;
+    }
+    // ---- the tiles' sums to every block: lane 8 t + c sends copy c of tile t
+    {
+      uint4* rec = A.recs + (seq & 1) * kMaxCopies * cstride + B.rec0 + B.rec;
+      const int groups = (B.nsl + 31) / 32;
+      for (int job = warp; job < 3 * groups; job += kWideWarps) {
+        const int i = job / groups, s = 32 * (job % groups) + lane;
+        df64 v[1] = {s < B.nsl ? Slot<df64>::sget(&part[i][s]) : df64(0.f)};
+        tree<df64, 1, 4>(v);
+        const df64 t(__shfl_sync(0xffffffffu, v[0].hi, lane & 24), __shfl_sync(0xffffffffu, v[0].lo, lane & 24));
+        if ((lane & 7) < copies && (s & ~7) < B.nsl)
+          st_rec(rec + (lane & 7) * cstride + (size_t)i * A.nrec_total + (s >> 3), rec_of(t, seq));
+      }
+    }
+    // ---- x, while the sums travel
+    if (threadIdx.x == 0) q.prepare();
+#pragma unroll
+    for (int j = 0; j < kWideSlices; ++j)
+      if (live[j]) {
+        float x[3];
+        float* at = gx + 4 * (size_t)(32 * (B.slice0 + sl[j]) + lane);
+        ld3<false>(at, x);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) x[c] = fma(a, p[j][c], x[c]);
+        st3(at, x);
+      }
+    // ---- all sums, in the order of scene_sums (a thread the tiles i, i + 256,
+    // ..): eight warps a sum, the third one's the first eight's second
+    {
+      const int g = warp & 7, first = 32 * g + lane;
+      const uint4* src = A.recs + ((seq & 1) * kMaxCopies + blockIdx.x % copies) * cstride + B.rec0 + first;
+#pragma unroll 1
+      for (int i = warp >> 3; i < 3; i += 2) {
+        const uint4* at = src + i * (size_t)A.nrec_total;
+        uint4 v[4];
+        bool want[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          want[j] = first + 256 * j < B.nrec;
+          if (want[j]) v[j] = ld_rec(at + 256 * j);
+        }
+        ok = poll_recs<4>(v, [&](int j) { return at + 256 * j; }, want, seq, err) && ok;
+        df64 e[1] = {df64(0.f)};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (want[j]) e[0] = e[0] + rec_val<df64>(v[j]);
+        tree<df64, 1, 16>(e);
+        if (lane == 0) Slot<df64>::put(&red[i][g], e[0]);
+      }
+    }
+    if (!__syncthreads_and(ok)) {
+      drain();
+      cgr_abort(A, B);
+      return;
+    }
+    if (warp == 0) {
+      df64 d[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) d[i] = lane < 8 ? Slot<df64>::sget(&red[i][lane]) : df64(0.f);
+      tree<df64, 3, 4>(d);
+      if (lane == 0) leave = q.step(sd, d) || n + 1 >= A.max_iters;
+    }
+    __syncthreads();
+    ++seq;
+    if (leave) break;
+  }
+  drain();
+  // ---- the vectors as k_cgf_iter leaves them after iteration `last`
+  const int last = q.swapped ? q.it : q.it - 1;
+#pragma unroll
+  for (int j = 0; j < kWideSlices; ++j)
+    if (live[j]) {
+      const size_t k4 = 4 * (size_t)(32 * (B.slice0 + sl[j]) + lane);
+      const float4 t = u4[32 * sl[j] + lane];
+      const float u[3] = {t.x, t.y, t.z};
+      if (kScaled) {
+        st3(static_cast<float*>(sd.cgf_r[(last + 1) & 1]) + k4, u);
+      } else {
+        st3(static_cast<float*>(sd.cgf_r[(last + 1) & 1]) + k4, dr[j]);
+        st3(static_cast<float*>(sd.cg_z) + k4, u);
+      }
+      st3(static_cast<float*>(sd.cgf_w[(last + 1) & 1]) + k4, w[j]);
+      st3(static_cast<float*>(sd.cgf_s[last & 1]) + k4, sv[j]);
+      st3(static_cast<float*>(sd.cg_p[0]) + k4, p[j]);
+    }
+  if (B.rec == 0 && threadIdx.x == 0) {
+    q.store(sc);
+    A.seq[B.scene] = seq;
+  }
+}
+
+template <typename F> auto with_kernel(bool fp64, bool fused, bool jacobi, bool wide, int threads, F&& f) {
+  if (wide) return jacobi ? f((const void*)k_cgr_wide<true>) : f((const void*)k_cgr_wide<false>);
   if (fused && threads > 256) return jacobi ? f((const void*)k_cgr_fused<true, 512>) : f((const void*)k_cgr_fused<false, 512>);
   if (fused) return jacobi ? f((const void*)k_cgr_fused<true, 256>) : f((const void*)k_cgr_fused<false, 256>);
   if (fp64) return f((const void*)k_cgr_split64);
@@ -1068,8 +1484,8 @@ template <typename F> auto with_kernel(bool fp64, bool fused, bool jacobi, int t
 
 }  // namespace
 
-int cgr_blocks_per_sm(bool fp64, bool fused, bool jacobi, int threads, size_t smem) {
-  return with_kernel(fp64, fused, jacobi, threads, [&](const void* k) {
+int cgr_blocks_per_sm(bool fp64, bool fused, bool jacobi, bool wide, int threads, size_t smem) {
+  return with_kernel(fp64, fused, jacobi, wide, threads, [&](const void* k) {
     int nb = 0;
     // the function's limit is shared by every batch: always the largest
     if (smem > kCgrSmem ||
@@ -1082,9 +1498,9 @@ int cgr_blocks_per_sm(bool fp64, bool fused, bool jacobi, int threads, size_t sm
   });
 }
 
-cudaError_t launch_cgr(const CgrArgs& args, bool fp64, bool fused, bool jacobi, int nblocks, int threads, size_t smem,
-                       cudaStream_t stream) {
-  return with_kernel(fp64, fused, jacobi, threads, [&](const void* k) {
+cudaError_t launch_cgr(const CgrArgs& args, bool fp64, bool fused, bool jacobi, bool wide, int nblocks, int threads,
+                       size_t smem, cudaStream_t stream) {
+  return with_kernel(fp64, fused, jacobi, wide, threads, [&](const void* k) {
     CgrArgs a = args;
     void* params[] = {&a};
     return cudaLaunchCooperativeKernel(k, dim3(nblocks), dim3(threads), params, smem, stream);

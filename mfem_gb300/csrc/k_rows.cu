@@ -1007,19 +1007,6 @@ constexpr size_t cgf_staged_smem_bytes(int warps) {
   return (size_t)warps * S * kSlotPairs * sizeof(typename PairOf<Real>::T) + (size_t)warps * S * 8;
 }
 
-// L2 policy of the matrix stream: all lines evict-first (keep = 0), or half
-// of them evict-last (keep = 1), so that about half the matrix can stay in
-// L2 from one iteration to the next.
-template <int kKeep>
-__device__ __forceinline__ unsigned long long l2_matrix_policy() {
-  unsigned long long p;
-  if constexpr (kKeep == 0)
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  else
-    asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, 0.5;" : "=l"(p));
-  return p;
-}
-
 // Programmatic dependent launch: this grid lets the next one launch, and
 // waits for the previous one's completion (and its writes) before it reads
 // anything the previous iteration wrote.

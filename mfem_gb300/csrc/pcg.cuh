@@ -72,6 +72,21 @@ __device__ __forceinline__ unsigned long long l2_evict_last() {
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
+// L2 policy of the matrix stream: all lines evict-first (keep = 0), or half
+// (keep = 1) or three eighths (keep = 2) of them evict-last, so that about
+// that much of the matrix can stay in L2 from one iteration to the next.
+template <int kKeep>
+__device__ __forceinline__ unsigned long long l2_matrix_policy() {
+  unsigned long long p;
+  if constexpr (kKeep == 0)
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  else if constexpr (kKeep == 1)
+    asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, 0.5;" : "=l"(p));
+  else
+    asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, 0.375;" : "=l"(p));
+  return p;
+}
+
 __device__ __forceinline__ float2 ld_stream(const float* ell, size_t pair, unsigned long long pol) {
   float2 v;
   asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"

@@ -100,3 +100,26 @@ def test_fp64_blocks_of_one_two_and_four_slices(gpu_lib, dims):
     a, b = run(spec(dims, D, PERS, **kw), 1), run(spec(dims, D, SPLIT, **kw), 1)
     assert a[2] > 0 and b[2] == 0
     same(a, b)
+
+
+# (free rows: 86,526 = 338 tiles, three a block; 223,138 = 872 tiles, six)
+@pytest.mark.parametrize("dims,kw", [((57, 32, 45), {}), ((57, 32, 45), dict(linear_solver=abi.SOLVER_GPU_PCG_BLOCK)),
+                                     ((57, 32, 45), dict(max_iterative_solver_iters=7)), ((59, 60, 61), {})])
+def test_blocks_of_several_tiles_that_stream_the_matrix(gpu_lib, dims, kw):
+    a, b = run(spec(dims, M, AUTO, **kw), 1), run(spec(dims, M, FUSED, **kw), 1)
+    same(a, b)
+
+
+def test_batch_of_scenes_whose_blocks_hold_several_tiles(gpu_lib):
+    """18 scenes together of more than two tiles an SM (one to 35 tiles each):
+    the steps are those of each scene alone in single launches."""
+    specs = [spec(d, M, FUSED) for d in [(20, 20, 20)] * 10 + [(7, 5, 5), (13, 9, 9), (4, 2, 2), (16, 21, 23)] * 2]
+    one = [gpu.Scene(s) for s in specs]
+    ref = [run(s, 2) for s in (specs[0], *specs[10:14])]
+    batch = gpu.Batch(one)
+    batch.step_n(2)
+    for sc, i in zip(one, [0] * 10 + [1, 2, 3, 4] * 2):
+        st = sc.get_state()
+        for k in ("x", "v", "s", "R"):
+            assert np.array_equal(st[k], ref[i][1][k]), (i, k)
+    batch.close()
