@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
   const E rr0 = sc_get<E>(&sc->cg_rhs_norm2);
   E rr = rr0;
   float beta = 0.f;
-  E alphaE = E(0), betaE = E(0);
+  E alphaE = E(0), betaE = E(0), rz_rcp = E(0);
   int it = 0, status = 0, cg_status = 0;
   unsigned ztag = 0;
 
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) d1[0] = acc_prod(d1[0], p[c], acc[c]);
     }
-    if (!scene_total<E, 1>(A, B, S, roww, sl, seq, d1, nothing, nothing)) {
+    if (!scene_total<E, 1>(A, B, S, roww, sl, seq, d1, nothing, [&]() { rz_rcp = rcp_of(rz); })) {
       cgr_abort(A, B);
       return;
     }
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
     if (cg_meets(sd, rr, rr0)) {
       stop = true;
     } else {
-      betaE = d2[1] / rz;
+      betaE = by_rcp(d2[1], rz, rz_rcp);
       rz_prev = rz;
       rz = d2[1];
       it = it + 1;
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
         it = it - 1;  // as in Eigen, the iteration that meets the threshold is not counted
         break;
       }
-      betaE = d3[1] / rz_prev;
+      betaE = by_rcp(d3[1], rz_prev, rz_rcp);
       rz = d3[1];
     }
     beta = to_step(betaE);
@@ -839,8 +839,8 @@ struct CgfScalars {
         rounds(sc->cgf_rounds), phase(0), status(0), cg_status(0), swapped(false) {}
   // While the sums travel.
   __device__ __forceinline__ void prepare() {
-    rg = df64(1.f) / gamma;
-    ra = df64(1.f) / alphaE;
+    rg = rcp_of(gamma);
+    ra = rcp_of(alphaE);
   }
   // After an iteration's sums, as cgf_verify_step in phase 0: whether the launch ends.
   __device__ __forceinline__ bool step(const SceneDev& sd, const df64 (&d)[3]) {
@@ -855,7 +855,7 @@ struct CgfScalars {
       swapped = true;
       return true;
     }
-    cgf_steps(d[1], d[2], rg, ra, &alphaE, &betaE);
+    cgf_steps(d[1], d[2], gamma, alphaE, rg, ra, &alphaE, &betaE);
     gamma = d[1];
     a = to_step(alphaE);
     b = to_step(betaE);

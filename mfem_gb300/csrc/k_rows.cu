@@ -455,7 +455,7 @@ __device__ __forceinline__ void cg_update_tile(int tix, const Tile* tiles, const
         stop = true;
       } else {
         const E rz_old = sc_get<E>(&sc->rz);
-        const E b = v[1] / rz_old;
+        const E b = by_rcp(v[1], rz_old, rcp_of(rz_old));
         sc_put(&sc->beta, b);
         sc->beta_f = float(to_step(b));
         sc_put(&sc->rz_prev, rz_old);
@@ -546,7 +546,7 @@ __device__ __forceinline__ void cg_replace_tile(int tix, const Tile* tiles, cons
         sc->nph = kPhLocal;
         atomicSub(&ctrs->cg_active, 1);
       } else {
-        const df64 b2 = v[1] / sc_get<df64>(&sc->rz_prev);
+        const df64 rz_prev = sc_get<df64>(&sc->rz_prev), b2 = by_rcp(v[1], rz_prev, rcp_of(rz_prev));
         sc_put(&sc->beta, b2);
         sc->beta_f = to_step(b2);
         sc_put(&sc->rz, v[1]);
@@ -638,7 +638,8 @@ __device__ __forceinline__ void cgf_finish(const SceneDev& sd, BatchCounters* ct
           stop = true;
         } else {
           E an, bn;
-          cgf_steps(g, d, E(1) / sc_get<E>(&sc->cgf_gamma[0]), E(1) / sc_get<E>(&sc->alpha), &an, &bn);
+          const E g_prev = sc_get<E>(&sc->cgf_gamma[0]), a_prev = sc_get<E>(&sc->alpha);
+          cgf_steps(g, d, g_prev, a_prev, rcp_of(g_prev), rcp_of(a_prev), &an, &bn);
           sc_put(&sc->beta, bn);
           sc_put(&sc->alpha, an);
           sc_put(&sc->cgf_gamma[0], g);
