@@ -92,24 +92,31 @@ constexpr int kMaxCopies = 8;
 __host__ __device__ constexpr int exchange_copies(int blocks) { return blocks > 40 ? kMaxCopies : 1; }
 
 // n records of one quantity summed by the calling warp (valid in lane 0):
-// lane l over records l, l + 32, ..; then a tree.  ok is cleared when a wait ran out.
+// lane l over records l, l + 32, ..; then a tree; 160 records in flight, so
+// that a block an SM takes one wait.  Absent records are not added: a zero
+// takes an addition's 66 cycles too.  ok is cleared when a wait ran out.
 __device__ __forceinline__ double fetch_sum(const uint4* rec, int n, unsigned seq, int* err, bool& ok) {
   const int lane = threadIdx.x & 31;
   double v = 0.0;
-  for (int i0 = 0; i0 < n && ok; i0 += 128) {
-    uint4 g[4];
-    bool want[4];
+  for (int i0 = 0; i0 < n && ok; i0 += 160) {
+    uint4 g[5];
+    bool want[5];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 5; ++j) {
       want[j] = i0 + 32 * j + lane < n;
       if (want[j]) g[j] = ld_rec(rec + i0 + 32 * j + lane);
     }
-    ok = poll_recs<4>(g, [&](int j) { return rec + i0 + 32 * j + lane; }, want, seq, err);
+    ok = poll_recs<5>(g, [&](int j) { return rec + i0 + 32 * j + lane; }, want, seq, err);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v += want[j] ? rec_double(g[j]) : 0.0;
+    for (int j = 0; j < 5; ++j)
+      if (i0 + 32 * j < n) {  // warp-uniform
+        const double e = want[j] ? rec_double(g[j]) : 0.0;
+        v = i0 + j == 0 ? e : v + e;
+      }
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+  for (int off = 16; off > 0; off >>= 1)
+    if (off < n) v += __shfl_down_sync(0xffffffffu, v, off);
   return v;
 }
 

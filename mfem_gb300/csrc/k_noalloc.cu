@@ -337,25 +337,31 @@ __global__ void __launch_bounds__(kNaThreads) k_na_update(int n, double* x, NaVi
 //   p = z + beta p;  Ap;  (p, Ap) -> alpha;  x += alpha p;  r -= alpha Ap;
 //   z = D^-1 r;  (r, r), (r, z) -> the stopping test and beta
 // 9,000 rows, 109k blocks, 230 iterations: 10.9 ms with the launches (two an
-// iteration, one thread summing 36 tiles' partials in turn), 3.25 ms so.
+// iteration, one thread summing 36 tiles' partials in turn), 2.4 ms so (10.4 us
+// an iteration; 3.15 ms with the quotients and comparisons in every warp, since
+// the pipe takes 19 cycles of the SM for each, and the halo's records fetched
+// when they are used).  Of the 20,000 cycles the product is 5,400, the two
+// exchanges of 141 blocks 6,800, trees and a division 3,000.
 // A partial record is overwritten two exchanges after everybody has read it
 // (two buffers by parity), z only after the exchange of (p, Ap), before which
 // everybody has read it.
 constexpr int kNaMaxSlices = 7;      // 32768 rows over 147 blocks
+constexpr int kNaFewSlices = 3;      // up to 14592 rows over 152 blocks: no spilled registers
 constexpr int kNaMaxHalo = 2560;
 constexpr int kNaMaxSlots = 448;     // of a block's slices
 constexpr int kNaHash = 8192;
 constexpr size_t kNaSmem = 220 * 1024;
 constexpr size_t kNaOffTable = 64 * (size_t)kNaMaxSlots + 4 * (size_t)kNaMaxHalo;  // li, halo columns
 
-__global__ void __launch_bounds__(96 * kNaMaxSlices) k_na_resident(NaMatrix A, const double* b, double* x, NaView v,
+template <int kSlices>  // the most slices a block may have: the registers a thread may take
+__global__ void __launch_bounds__(96 * kSlices) k_na_resident(NaMatrix A, const double* b, double* x, NaView v,
                                                                    int max_iters, double tol) {
   using namespace mfem_gpu;
   extern __shared__ __align__(16) unsigned char na_smem[];
   __shared__ int slot0[kNaMaxSlices + 1], nh_s, bad_s, flags;
   __shared__ int len_s[32 * kNaMaxSlices];
   __shared__ uint8_t row_at[32 * kNaMaxSlices], place_of[32 * kNaMaxSlices];
-  __shared__ double part[2][kNaMaxSlices], tot[2], coef;
+  __shared__ double part[2][kNaMaxSlices], tot[2], coef, rcp;
   const int T = blockDim.x, S = T / 96, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sl = warp / 3, comp = warp % 3, G = gridDim.x, bk = blockIdx.x;
   const int row0 = 32 * S * bk, row1 = min(A.n, row0 + 32 * S), own = 32 * S;
@@ -493,8 +499,9 @@ __global__ void __launch_bounds__(96 * kNaMaxSlices) k_na_resident(NaMatrix A, c
 
   // The sums of quantities 0 .. nq - 1, whose parts of the block's slices are
   // in part[][]: one warp per quantity sends the block's sum and adds up
-  // everybody's.  False: a wait ran out.
-  auto total = [&](int nq) -> bool {
+  // everybody's.  `beside`: the last warp's, during the wait; `then(q, sum)`:
+  // lane 0's of the warp that has the sum.  False: a wait ran out.
+  auto total = [&](int nq, auto beside, auto then) -> bool {
     __syncthreads();
     if (warp < nq) {
       double t = 0.0;
@@ -508,7 +515,12 @@ __global__ void __launch_bounds__(96 * kNaMaxSlices) k_na_resident(NaMatrix A, c
         t = fetch_sum(rec, G, seq, &sc->error, ok);
         if (!ok && lane == 0) atomicOr(&flags, 1);
       }
-      if (lane == 0) tot[warp] = t;
+      if (lane == 0) {
+        tot[warp] = t;
+        then(warp, t);
+      }
+    } else if (warp == T / 32 - 1) {
+      beside();
     }
     __syncthreads();
     ++seq;
@@ -531,6 +543,8 @@ __global__ void __launch_bounds__(96 * kNaMaxSlices) k_na_resident(NaMatrix A, c
       slice_sum(comp, fma(q[64], o[64], fma(q[32], o[32], q[0] * o[0])));
     }
   };
+  auto nothing = []() {};
+  auto keep = [](int, double) {};
   auto leave = [&]() {
     if (threadIdx.x == 0) atomicAdd(v.seq, 0x100000u);  // later calls use other tags
   };
@@ -538,7 +552,7 @@ __global__ void __launch_bounds__(96 * kNaMaxSlices) k_na_resident(NaMatrix A, c
   // ---- does every block fit, is every row in order: then |b|^2 and (r, z)
   __syncthreads();
   if (lead) slice_sum(0, lane == 0 && sl == 0 && bad_s ? 1.0 : 0.0);
-  if (!total(1)) {
+  if (!total(1, nothing, keep)) {
     leave();
     return;
   }
@@ -546,7 +560,7 @@ __global__ void __launch_bounds__(96 * kNaMaxSlices) k_na_resident(NaMatrix A, c
   __syncthreads();
   put_rz();
   unsigned ztag = seq;
-  if (!total(2)) {
+  if (!total(2, nothing, keep)) {
     leave();
     return;
   }
@@ -558,14 +572,39 @@ __global__ void __launch_bounds__(96 * kNaMaxSlices) k_na_resident(NaMatrix A, c
   }
   bool active = rr0 != 0.0 && rr0 >= thr && max_iters > 0;
   int status = rr0 != 0.0 && rr0 >= thr && max_iters == 0 ? MFEM_ERR_CG_MAXITER : 0, it = 0;
+  constexpr unsigned long long kSign = 1ull << 63, kInf = 0x7ff0000000000000ull;
+  const unsigned long long thr_bits = __double_as_longlong(thr);
+  // the halo's first records of this thread, under way ahead of their use
+  constexpr int kAhead = kSlices > kNaFewSlices ? 1 : 4;
+  int hc[kAhead];
+  bool hw[kAhead];
+  uint4 hv[kAhead];
+#pragma unroll
+  for (int j = 0; j < kAhead; ++j) {
+    const int i = threadIdx.x + j * T;
+    hw[j] = i < 3 * nh;
+    hc[j] = hw[j] ? 3 * hcol[i / 3] + i % 3 : 0;
+  }
+  auto halo_ahead = [&]() {
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j)
+      if (hw[j]) hv[j] = ld_rec(v.pub + hc[j]);
+  };
+  halo_ahead();
   __syncthreads();
   while (active) {
     // ---- p = z + beta p: own rows, then the halo
     const bool first = it == 0;
     p = first ? z : fma(beta, p, z);
     vec[3 * mine + comp] = p;
-    bool ok = true;
-    for (int i0 = 32 * warp; i0 < 3 * nh; i0 += 4 * T) {  // four records a lane in flight
+    bool ok = poll_recs<kAhead>(hv, [&](int j) { return v.pub + hc[j]; }, hw, ztag, &sc->error);
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j)
+      if (hw[j]) {
+        double* q = vec + 3 * own + threadIdx.x + j * T;
+        *q = first ? rec_double(hv[j]) : fma(beta, *q, rec_double(hv[j]));
+      }
+    for (int i0 = 32 * warp + kAhead * T; i0 < 3 * nh; i0 += 4 * T) {  // four records a lane in flight
       bool want[4];
       uint4 w[4];
       const uint4* src[4];
@@ -614,13 +653,10 @@ __global__ void __launch_bounds__(96 * kNaMaxSlices) k_na_resident(NaMatrix A, c
       const double* pp = vec + 3 * mine;
       slice_sum(0, fma(pp[2], q[64], fma(pp[1], q[32], pp[0] * q[0])));
     }
-    if (!total(1)) {
+    if (!total(1, [&]() { if (lane == 0) rcp = 1.0 / rz; }, [&](int, double t) { coef = rz / t; })) {
       leave();
       return;
     }
-    if (warp == 0 && lane == 0) coef = rz / tot[0];
-    const double rcp = warp == 1 ? 1.0 / rz : 0.0;
-    __syncthreads();
     // ---- x, r, z, (r, r), (r, z)
     const double alpha = coef;
     xv = fma(alpha, p, xv);
@@ -633,28 +669,28 @@ __global__ void __launch_bounds__(96 * kNaMaxSlices) k_na_resident(NaMatrix A, c
     }
     put_rz();
     ztag = seq;
-    if (!total(2)) {
+    if (!total(2, nothing, [&](int q, double t) { if (q == 1) coef = quotient_by(t, rz, rcp); })) {
       leave();
       return;
     }
-    const double rr = tot[0], rz_new = tot[1];
-    if (warp == 1 && lane == 0) coef = quotient_by(rz_new, rz, rcp);
-    rr_last = rr;
+    halo_ahead();
+    // (comparisons take the FP64 pipe, 19 cycles a warp: as bits they don't)
+    const unsigned long long rr_bits = __double_as_longlong(tot[0]), rz_bits = __double_as_longlong(tot[1]);
+    rr_last = tot[0];
     // as in Eigen's loop, the iteration that meets the threshold is not counted
-    if (!(rr == rr) || !(rz_new == rz_new)) {
+    if ((rr_bits & ~kSign) > kInf || (rz_bits & ~kSign) > kInf) {  // NaN
       status = MFEM_ERR_NONFINITE;
       active = false;
-    } else if (rr < thr) {
+    } else if (rr_bits < thr_bits) {
       active = false;
     } else {
-      rz = rz_new;
+      rz = tot[1];
       ++it;
       if (it >= max_iters) {
         status = MFEM_ERR_CG_MAXITER;
         active = false;
       }
     }
-    __syncthreads();
     beta = coef;
   }
   if (live) x[3 * (size_t)row + comp] = xv;
@@ -715,9 +751,14 @@ extern "C" int mfem_gpu_bsr_pcg_noalloc(int32_t n_block_rows, int32_t nnzb, cons
                         cudaMemcpyHostToDevice, static_cast<cudaStream_t>(stream)) != cudaSuccess ||
         cudaStreamSynchronize(static_cast<cudaStream_t>(stream)) != cudaSuccess)
       return MFEM_ERR_CUDA;
-    if (cudaFuncSetAttribute(k_na_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNaSmem) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_na_resident, 96 * kNaMaxSlices, kNaSmem) == cudaSuccess)
+    auto ready = [&](const void* k, int slices_) {
+      return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNaSmem) == cudaSuccess &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 96 * slices_, kNaSmem) == cudaSuccess &&
+             per_sm > 0;
+    };
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        ready((const void*)k_na_resident<kNaFewSlices>, kNaFewSlices) &&
+        ready((const void*)k_na_resident<kNaMaxSlices>, kNaMaxSlices))
       g_na_sms[dev] = per_sm > 0 ? std::min(sms, kNaMaxBlocks) : 0;
     else
       cudaGetLastError();
@@ -737,7 +778,9 @@ extern "C" int mfem_gpu_bsr_pcg_noalloc(int32_t n_block_rows, int32_t nnzb, cons
   const int spb = sms > 0 ? (slices + sms - 1) / sms : kNaMaxSlices + 1;
   if (spb <= kNaMaxSlices) {
     void* args[] = {(void*)&A, (void*)&b, (void*)&x, (void*)&v, (void*)&max_iters, (void*)&tol};
-    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_na_resident, dim3((slices + spb - 1) / spb),
+    const cudaError_t e = cudaLaunchCooperativeKernel(spb <= kNaFewSlices ? (const void*)k_na_resident<kNaFewSlices>
+                                                                          : (const void*)k_na_resident<kNaMaxSlices>,
+                                                      dim3((slices + spb - 1) / spb),
                                                       dim3(96 * spb), args, kNaSmem, st);
     if (e != cudaSuccess) return MFEM_ERR_CUDA;
     if (cudaMemcpyAsync(&h, v.sc, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -705,9 +705,9 @@ __global__ void __launch_bounds__(kGridThreads) t2_pcg_grid(T2 d, int max_iter, 
 // block of 1024 threads and of t2_pcg_grid's blocks: Newton's last steps on a
 // sheet are decided by energy differences near rounding, so that another
 // order would move the converged state by 1e-9.  An iteration, before (one
-// block up to 1024 rows, t2_pcg_grid above) and now: 99 rows 20.3 -> 6.9 us,
-// 1,071 rows 19.7 -> 5.7 us, 4,191 rows 20.5 -> 6.6 us, 9,999 rows (157
-// blocks, some SMs with two) 23.8 -> 8.4 us.
+// block up to 1024 rows, t2_pcg_grid above) and now: 99 rows 20.3 -> 7.0 us,
+// 1,071 rows 19.7 -> 4.9 us, 4,191 rows 20.5 -> 5.4 us, 9,999 rows (157
+// blocks, some SMs with two) 23.8 -> 6.6 us.
 //
 // A record is overwritten only after everybody has read it: records alternate
 // between two buffers by the exchange's parity, and a block writes exchange

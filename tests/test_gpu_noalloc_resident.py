@@ -101,3 +101,8 @@ def test_limits_and_refusals(gpu_lib):
     # and the next good system solves
     rc, _, err, x = solve(rp, col, val, b)
     assert rc == abi.OK and residual(rp, col, val, b, x) <= 10 * TOL
+
+
+@pytest.mark.parametrize("n", [14592, 14593])  # three and four slices a block: each its own build of the kernel
+def test_sizes_at_the_change_of_kernel(gpu_lib, n):
+    test_sizes(gpu_lib, n)
