@@ -20,6 +20,9 @@
 //     partials in the same fixed order and takes the same decisions.
 // The arithmetic, the order of every sum included, is that of the launches
 // it replaces (pcg.cuh), so the results are bitwise the same.
+// k_cgr_split (mixed path) and k_cgr_split64 run the two-reduction iteration,
+// k_cgr_fused the single-reduction one, and k_cgr_wide that one for systems
+// that outgrow shared memory, whose matrix it streams.
 //
 // A record is overwritten only after everybody has read it: partials and the
 // single-reduction form's vector alternate between two buffers by the
