@@ -544,6 +544,8 @@ def run_ours(args):
     if dom == "k_cg_solve" and cg_per_solve:
         # per PCG iteration, so that the figure compares with the split kernels
         roof_note = f"k_cg_solve: {cg_per_solve:.1f} PCG iterations per launch"
+    elif dom.startswith("k_cg") and timed_launches.get("k_cg_solve"):
+        roof_note = "the profiled replay runs the PCG's launches; the timed steps ran each solve in one"
     else:
         roof_note = None
     roof = {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
