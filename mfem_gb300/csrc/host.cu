@@ -2015,8 +2015,6 @@ int batch_autotune(mfem_batch* b) {
   std::vector<SceneDev> tsd = b->h_sds;
   for (SceneDev& d : tsd) {
     d.cg_tol = 0.0;
-    d.cg_tolx = make_float2(0.f, 0.f);
-    d.cg_itolx = make_float2(0.f, 0.f);
     d.max_cg = 1 << 30;
   }
   CUDA_OR(cudaMemcpyAsync(b->d_sds, tsd.data(), sizeof(SceneDev) * n, cudaMemcpyHostToDevice, b->stream),
@@ -2298,9 +2296,6 @@ int scene_init_device(mfem_scene* s) {
   D.newton_tol = s->cfg.newton_tol;
   D.res_tol = s->cfg.newton_residual_tolerance;
   D.cg_tol = s->cfg.iterative_solver_tolerance;
-  D.cg_tolx = split_df(D.cg_tol);
-  // (below FP32's range the tolerance counts as 0: the solve never meets it)
-  D.cg_itolx = D.cg_tol > 1e-37 ? split_df(1.0 / D.cg_tol) : make_float2(0.f, 0.f);
   D.max_newton = s->cfg.max_newton_iterations;
   D.max_ls = s->cfg.max_linesearch_iterations;
   D.max_cg = s->cfg.max_iterative_solver_iters;

@@ -328,6 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
   };
   E rz = sc_get<E>(&sc->rz), rz_prev = rz;
   const E rr0 = sc_get<E>(&sc->cg_rhs_norm2);
+  const float2 thr = sc->cg_thr;
   E rr = rr0;
   float beta = 0.f;
   E alphaE = E(0), betaE = E(0), rz_rcp = E(0);
@@ -421,7 +422,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
     ++seq;
     rr = d2[0];
     bool stop = false;
-    if (cg_meets(sd, rr, rr0)) {
+    if (cg_meets(sd, thr, rr, rr0)) {
       stop = true;
     } else {
       betaE = by_rcp(d2[1], rz, rz_rcp);
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
       ztag = seq;
       ++seq;
       rr = d3[0];
-      if (cg_meets(sd, rr, rr0) || is_nan(rr)) {
+      if (cg_meets(sd, thr, rr, rr0) || is_nan(rr)) {
         if (is_nan(rr)) status = 4;
         it = it - 1;  // as in Eigen, the iteration that meets the threshold is not counted
         break;
@@ -832,13 +833,14 @@ __global__ void __launch_bounds__(kThreads64, 1) k_cgr_split64(const CgrArgs A) 
 // exchanged vector is w; each block keeps r and s at its halo.
 struct CgfScalars {
   df64 gamma, alphaE, betaE, rr0, rr, rg, ra;
+  float2 thr;
   float a, b;
   int it, rounds, phase, status, cg_status;
   bool swapped;  // an iteration left the recursion without counting (phase set)
 
   __device__ __forceinline__ explicit CgfScalars(const SceneScalars* sc)
       : gamma(sc_get<df64>(&sc->cgf_gamma[0])), alphaE(sc_get<df64>(&sc->alpha)), betaE(sc_get<df64>(&sc->beta)),
-        rr0(sc_get<df64>(&sc->cg_rhs_norm2)), rr(rr0), a(sc->alpha_f), b(sc->beta_f), it(sc->cg_iter),
+        rr0(sc_get<df64>(&sc->cg_rhs_norm2)), rr(rr0), thr(sc->cg_thr), a(sc->alpha_f), b(sc->beta_f), it(sc->cg_iter),
         rounds(sc->cgf_rounds), phase(0), status(0), cg_status(0), swapped(false) {}
   // While the sums travel.
   __device__ __forceinline__ void prepare() {
@@ -851,7 +853,7 @@ struct CgfScalars {
     if (is_nan(rr)) {
       status = 4;
       phase = 3;
-    } else if (cg_meets(sd, rr, rr0)) {
+    } else if (cg_meets(sd, thr, rr, rr0)) {
       phase = rounds < kCgfRounds ? 1 : 3;
     }
     if (phase) {

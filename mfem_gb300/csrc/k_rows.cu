@@ -305,6 +305,8 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_init(const Tile* tiles, const
     scene_sums<E, 2>(partials, pstride, 0, t0, tc, v);
     if (threadIdx.x == 0) {
       sc_put(&sc->cg_rhs_norm2, v[0]);
+      const float2 thr = cg_threshold(sd, v[0]);
+      sc->cg_thr = thr;
       sc->cg_iter = 0;
       sc_put(&sc->beta, E(0));
       sc->beta_f = 0.0f;
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_init(const Tile* tiles, const
       if (is_zero(v[0])) {
         sc->cg_active = 0;
         sc->nph = kPhLocal;
-      } else if (cg_meets(sd, v[0], v[0]) || sd.max_cg <= 0) {
+      } else if (cg_meets(sd, thr, v[0], v[0]) || sd.max_cg <= 0) {
         sc->cg_active = 0;
         sc->nph = kPhLocal;
         sc->cg_err = 1.0;
@@ -451,7 +453,7 @@ __device__ __forceinline__ void cg_update_tile(int tix, const Tile* tiles, const
       const E rr0 = sc_get<E>(&sc->cg_rhs_norm2);
       sc->cg_err = cg_rel(v[0], rr0);
       bool stop = false;
-      if (cg_meets(sd, v[0], rr0)) {
+      if (cg_meets(sd, sc->cg_thr, v[0], rr0)) {
         stop = true;
       } else {
         const E rz_old = sc_get<E>(&sc->rz);
@@ -535,7 +537,7 @@ __device__ __forceinline__ void cg_replace_tile(int tix, const Tile* tiles, cons
     if (threadIdx.x == 0) {
       const df64 rr0 = sc_get<df64>(&sc->cg_rhs_norm2);
       sc->cg_err = cg_rel(v[0], rr0);
-      if (cg_meets(sd, v[0], rr0) || is_nan(v[0])) {
+      if (cg_meets(sd, sc->cg_thr, v[0], rr0) || is_nan(v[0])) {
         if (is_nan(v[0])) sc->status = 4;
         // x_{cg_iter} meets the threshold: as in Eigen, that iteration is not counted
         const int done = ldv<kCo>(&sc->cg_iter) - 1;
@@ -608,13 +610,15 @@ __device__ __forceinline__ void cgf_finish(const SceneDev& sd, BatchCounters* ct
       const E rr = v[0], g = v[1], d = v[2];
       if (kInit) {
         sc_put(&sc->cg_rhs_norm2, rr);
+        const float2 thr = cg_threshold(sd, rr);
+        sc->cg_thr = thr;
         sc->cg_iter = 0;
         sc->cg_err = 0.0;
         sc->cgf_phase = 0;
         sc->cgf_rounds = 0;
         if (is_zero(rr)) {
           sc->cg_active = 0;
-        } else if (cg_meets(sd, rr, rr) || sd.max_cg <= 0) {
+        } else if (cg_meets(sd, thr, rr, rr) || sd.max_cg <= 0) {
           sc->cg_active = 0;
           sc->cg_err = 1.0;
         } else {
@@ -634,7 +638,7 @@ __device__ __forceinline__ void cgf_finish(const SceneDev& sd, BatchCounters* ct
         bool stop = false;
         const E rr0 = sc_get<E>(&sc->cg_rhs_norm2);
         sc->cg_err = cg_rel(rr, rr0);
-        if (cg_meets(sd, rr, rr0)) {
+        if (cg_meets(sd, sc->cg_thr, rr, rr0)) {
           stop = true;
         } else {
           E an, bn;

@@ -76,6 +76,7 @@ struct SceneScalars {
   double cg_rhs_norm2, rz, alpha, beta, cg_err;
   double rz_prev;    // rz of the previous iteration (residual replacement)
   double cgf_gamma[1];  // single-reduction PCG: (r, u) of the last iteration
+  float2 cg_thr;        // mixed path: the stopping test's threshold (cg_threshold)
   // mixed path: verification phase of the single-reduction PCG (0: iterate;
   // 1: r = b - A (x_e + x) exactly; 2: fold x into x_e, w = A u and the
   // inner products of the true residual; 3: write the rounded solution)
@@ -143,7 +144,6 @@ struct SceneDev {
   double dt;         // beta*h
   float2 h2x;        // h2 as a float pair (df64), and float(h2) in .x
   double newton_tol, res_tol, cg_tol;
-  float2 cg_tolx, cg_itolx;  // cg_tol and 1 / cg_tol as float pairs
   double load_norm;  // |h^2 P M f| over the free dofs (scale of the residual test)
   int max_newton, max_ls, max_cg, bdf_order;
   double bdf_alpha[6];

@@ -237,13 +237,28 @@ __device__ __forceinline__ bool is_zero(double v) { return v == 0.0; }
 __device__ __forceinline__ float to_step(df64 v) { return __fadd_rn(v.hi, v.lo); }
 __device__ __forceinline__ double to_step(double v) { return v; }
 
-// |r|^2 < tol^2 |b|^2 (or r = 0).  The mixed path compares |r|^2 / tol with
-// |b|^2 tol, which stays in FP32's range where tol^2 |b|^2 may not.
-__device__ __forceinline__ bool cg_meets(const SceneDev& sd, df64 rr, df64 rr0) {
-  return rr.hi == 0.f || rr * df64(sd.cg_itolx.x, sd.cg_itolx.y) < rr0 * df64(sd.cg_tolx.x, sd.cg_tolx.y);
+// The stopping test |r|^2 < max(tol^2 |b|^2, DBL_MIN).  The mixed path forms
+// the threshold in FP64 once a solve, for any tolerance, and keeps it as two
+// floats: the nearest float and the rest rounded up.  A float-float |r|^2 then
+// lies below it exactly when the pairs compare so, with no FP64 instruction an
+// iteration: where the first floats differ they decide, and a float lies below
+// the rest when it lies below the next float above.  (A threshold past FP32's
+// range becomes (inf, -inf), which every finite sum meets, one below it (0,
+// 1.4e-45), which only zero meets.)
+__device__ __forceinline__ double cg_threshold_fp64(const SceneDev& sd, double rr0) {
+  return ::fmax(sd.cg_tol * sd.cg_tol * rr0, DBL_MIN);
 }
-__device__ __forceinline__ bool cg_meets(const SceneDev& sd, double rr, double rr0) {
-  return rr < ::fmax(sd.cg_tol * sd.cg_tol * rr0, DBL_MIN);
+__device__ __forceinline__ float2 cg_threshold(const SceneDev& sd, df64 rr0) {
+  const double t = cg_threshold_fp64(sd, rr0.to_double());
+  const float hi = float(t);
+  return make_float2(hi, __double2float_ru(t - double(hi)));
+}
+__device__ __forceinline__ float2 cg_threshold(const SceneDev&, double) { return make_float2(0.f, 0.f); }
+__device__ __forceinline__ bool cg_meets(const SceneDev&, float2 thr, df64 rr, df64) {
+  return rr < df64(thr.x, thr.y);
+}
+__device__ __forceinline__ bool cg_meets(const SceneDev& sd, float2, double rr, double rr0) {
+  return rr < cg_threshold_fp64(sd, rr0);
 }
 __device__ __forceinline__ double cg_rel(df64 rr, df64 rr0) { return double(sqrtf(rr.hi / rr0.hi)); }
 __device__ __forceinline__ double cg_rel(double rr, double rr0) { return ::sqrt(rr / rr0); }
@@ -319,7 +334,7 @@ __device__ __forceinline__ void cgf_verify_step(const SceneDev& sd, BatchCounter
     sc->cgf_phase = 3;
     return;
   }
-  if (cg_meets(sd, rr, rr0)) {
+  if (cg_meets(sd, sc->cg_thr, rr, rr0)) {
     // phase 0: the recursion's residual passes, verify it (unless the
     // verifications are used up); phase 2: the true residual passes, write
     // the solution
