@@ -890,12 +890,25 @@ template <bool kScaled, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
   extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
   __shared__ CgrShared S;
+  // The scalars, some 400 instructions an iteration: with 16 warps they are
+  // thread 0's, with a barrier more (two steps of 350 rows: 3.10 ms, against
+  // 3.24 ms with every warp for itself), with 8 every warp's own (three steps
+  // of 16 scenes: 26.4 ms against 26.9)
+  constexpr bool kOne = kThreads > 256;
+  __shared__ __align__(8) unsigned char q_raw[sizeof(CgfScalars)];
+  __shared__ int leave;
   const CgrBlock B = A.blocks[blockIdx.x];
   const SceneDev& sd = A.sds[B.scene];
   SceneScalars* sc = sd.sc;
   if (!sc->cg_active || sc->cgf_phase) return;
   unsigned seq = __ldcg(A.seq + B.scene);
   const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+  CgfScalars q_own(sc);
+  CgfScalars& q = kOne ? *reinterpret_cast<CgfScalars*>(q_raw) : q_own;
+  if (kOne) {
+    if (threadIdx.x == 0) new (&q) CgfScalars(sc);
+    __syncthreads();
+  }
   const bool roww = sl < B.nsl;
   const int row = 32 * (B.slice0 + sl) + lane;
   const bool live = roww && row < sd.nf;
@@ -906,7 +919,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
   float4* sh = u4 + own + B.nh;                         // s at the halo
   float4* rh = kScaled ? u4 + own : sh + B.nh;          // r at the halo (scaled: u itself)
   float* Dh = reinterpret_cast<float*>(sh + 2 * B.nh);  // unscaled: M^-1 at the halo, 9 each
-  CgfScalars q(sc);
   const int it = q.it;
   const float* gr = static_cast<const float*>(sd.cgf_r[it & 1]);
   const float* gw = static_cast<const float*>(sd.cgf_w[it & 1]);
@@ -1043,14 +1055,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
 #pragma unroll
           for (int j = 0; j < kHaloRegs; ++j)
             if (hw[j]) hv[j] = ld_rec(A.pub + (size_t)(seq & 1) * A.pub_stride + B.row0 + hc[j]);
-        }, [&]() { q.prepare(); })) {
+        }, [&]() { if (!kOne || threadIdx.x == 0) q.prepare(); })) {
       cgr_abort(A, B);
       return;
     }
     wtag = seq;
     ++seq;
-    if (q.step(sd, d)) break;
-    if (n + 1 >= A.max_iters) break;
+    if (kOne) {
+      if (threadIdx.x == 0) leave = q.step(sd, d) || n + 1 >= A.max_iters;
+      __syncthreads();
+      if (leave) break;
+    } else if (q.step(sd, d) || n + 1 >= A.max_iters) {
+      break;
+    }
   }
   // ---- the vectors as k_cgf_iter leaves them after iteration `last`
   const int last = q.swapped ? q.it : q.it - 1;

@@ -8,6 +8,7 @@
 
 #include "device_math.cuh"
 #include "kernels.cuh"
+#include "pcg_scalars.cuh"
 #include "reduce.cuh"
 
 namespace mfem_gpu {
@@ -263,29 +264,6 @@ __device__ __forceinline__ bool cg_meets(const SceneDev& sd, float2, double rr, 
 __device__ __forceinline__ double cg_rel(df64 rr, df64 rr0) { return double(sqrtf(rr.hi / rr0.hi)); }
 __device__ __forceinline__ double cg_rel(double rr, double rr0) { return ::sqrt(rr / rr0); }
 
-// num / den for a den known long before num, whose reciprocal is at hand.  A
-// den near the ends of FP32's range, whose reciprocal or its low part would
-// not be in it, is divided by.  FP64: the division (its kernels have their own
-// form of this, quotient_by).
-__device__ __forceinline__ df64 by_rcp(df64 num, df64 den, df64 rcp) {
-  const float m = fabsf(den.hi);
-  if (m > 1e-30f && m < 1e30f) return num * rcp;
-  return num / den;
-}
-__device__ __forceinline__ double by_rcp(double num, double den, double) { return num / den; }
-__device__ __forceinline__ df64 rcp_of(df64 v) { return df64(1.f) / v; }
-__device__ __forceinline__ double rcp_of(double) { return 0.0; }
-
-// Step lengths of the single-reduction iteration from (r, u), (w, u), the
-// previous (r, u) and alpha and their reciprocals, which are known before the
-// sums are: one division after them instead of three.
-template <typename E>
-__device__ __forceinline__ void cgf_steps(E g, E d, E g_prev, E a_prev, E g_rcp, E a_rcp, E* a, E* b) {
-  const E bn = by_rcp(g, g_prev, g_rcp);
-  *b = bn;
-  *a = g / (d - by_rcp(bn * g, a_prev, a_rcp));
-}
-
 // ---------------------------------------- verified stop (mixed path) ---
 // In FP32 the single-reduction recurrences drift: the recursive residual
 // meets the tolerance while the true |b - A x| / |b| sits several times
@@ -344,13 +322,10 @@ __device__ __forceinline__ void cgf_verify_step(const SceneDev& sd, BatchCounter
   df64 bn, an;
   if (ph == 2) {
     // A failed verification.  The recursion's gamma had drifted below the
-    // true residual's, so b = gamma / gamma_prev would be far too large: the
-    // new direction is made A-conjugate to the last one directly,
-    // b = -(A p, u) / (p, A p), and (p_new, A p_new) = d + 2 b (A p, u) +
-    // b^2 (p, A p) from phase 2's exact A p.
+    // true residual's, so b = gamma / gamma_prev would be far too large; su
+    // and ps come from phase 2's exact A p.
     sc->cgf_rounds += 1;
-    bn = -(su / ps);
-    an = g / (d + df64(2.f) * bn * su + bn * bn * ps);
+    cgf_restart_steps(g, d, su, ps, &an, &bn);
   } else {
     const df64 g_prev = sc_get<df64>(&sc->cgf_gamma[0]), a_prev = sc_get<df64>(&sc->alpha);
     cgf_steps(g, d, g_prev, a_prev, rcp_of(g_prev), rcp_of(a_prev), &an, &bn);
