@@ -89,7 +89,7 @@ enum { MFEM_FORMULATION_MIXED_STRETCH = 0, MFEM_FORMULATION_STRETCH = 1 };
  * single-reduction form of the same PCG (Chronopoulos and Gear, 1989), one
  * launch per iteration; equal to the others in exact arithmetic, not bitwise.
  * AUTO: the batch picks the form: FUSED when its PCG tiles (256 rows each)
- * fill at least two per SM, or are at most four (but not for one FP64 scene),
+ * fill at least two per SM, or are at most four (not in FP64),
  * SPLIT in between.  A batch of PERSISTENT, or of AUTO where it picked SPLIT
  * or at most four tiles, runs each solve as one launch with the matrix
  * resident in shared memory if that fits (up to two tiles per SM; FP64 up to

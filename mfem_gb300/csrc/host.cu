@@ -2179,7 +2179,7 @@ int batch_build(mfem_scene* const* scenes, int n, mfem_batch** out) {
   }
   b->auto_form = b->pcg_kernel == MFEM_PCG_KERNEL_AUTO;
   if (b->pcg_kernel == MFEM_PCG_KERNEL_AUTO)
-    b->pcg_kernel = (b->ntiles[TB_CG] >= 2 * sms || (b->ntiles[TB_CG] <= 4 && !(b->fp64 && n == 1)))
+    b->pcg_kernel = (b->ntiles[TB_CG] >= 2 * sms || (b->ntiles[TB_CG] <= 4 && !b->fp64))
                         ? MFEM_PCG_KERNEL_FUSED
                         : MFEM_PCG_KERNEL_SPLIT;
   if (b->pcg_kernel == MFEM_PCG_KERNEL_PERSISTENT) {
