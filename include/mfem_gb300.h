@@ -89,13 +89,15 @@ enum { MFEM_FORMULATION_MIXED_STRETCH = 0, MFEM_FORMULATION_STRETCH = 1 };
  * single-reduction form of the same PCG (Chronopoulos and Gear, 1989), one
  * launch per iteration; equal to the others in exact arithmetic, not bitwise.
  * AUTO: the batch picks the form: FUSED when its PCG tiles (256 rows each)
- * fill at least two per SM, or are at most four (not in FP64),
- * SPLIT in between.  A batch of PERSISTENT, or of AUTO where it picked SPLIT
+ * fill at least two per SM, or are at most four (not in FP64), SPLIT in
+ * between.  A batch of PERSISTENT, or of AUTO where it picked SPLIT
  * or at most four tiles, runs each solve as one launch with the matrix
  * resident in shared memory if that fits (up to two tiles per SM; FP64 up to
  * 128 rows per SM), or, where AUTO picked FUSED, streamed through it (up to
  * six tiles per SM), with the results of the picked form's launches, bitwise;
- * mfem_gpu_batch_step_n runs FUSED batches that way too. */
+ * mfem_gpu_batch_step_n runs FUSED batches that way too.  Mixed batches that
+ * step at the same time and want several times the SMs together run the
+ * launches, which interleave, instead. */
 enum { MFEM_PCG_KERNEL_PERSISTENT = 0, MFEM_PCG_KERNEL_SPLIT = 1, MFEM_PCG_KERNEL_FUSED = 2,
        MFEM_PCG_KERNEL_AUTO = 3 };
 

@@ -518,14 +518,19 @@ struct mfem_batch {
   cudaGraphExec_t cg_graph = nullptr;   // one chunk of PCG iterations, captured once
   // the whole PCG loop as one graph: a WHILE node around a chunk of
   // iterations and the loop's condition kernel (the device decides when
-  // the solve has ended; no host round trip per chunk); cg_loop_len
+  // the solve has ended; no host round trip per chunk); len
   // iterations a body; loop_pending: a solve whose bodies the host has not
   // yet counted (read with the next counter sync)
-  cudaGraphExec_t cg_loop = nullptr;
+  struct Loop {
+    cudaGraphExec_t graph = nullptr;
+    int len = 8;
+    bool fused = true;
+    bool resident = false;  // the body starts with the resident solve
+  };
+  Loop cg_loop[2];  // by PcgMode
+  int loop_mode = 0;  // the loop that is pending
   bool cg_loop_on = true;
   bool loop_pending = false;
-  int cg_loop_len = 8;
-  bool loop_fused = true;
   cudaEvent_t ev_pipe[2] = {nullptr, nullptr};
   SceneScalars* h_sc = nullptr;     // pinned, one per scene
   int max_newton = 0, max_ls = 0, max_cg = 0;
@@ -550,8 +555,11 @@ struct mfem_batch {
   // graph of one tick (captured on first use, dropped when a kernel shape or
   // variant changes)
   unsigned long long* d_step_ns = nullptr;
-  cudaGraphExec_t tick_graph = nullptr;
-  cudaGraphExec_t tick_graph_c = nullptr;  // the same over compacted tables
+  struct Tick {
+    cudaGraphExec_t graph = nullptr;
+    bool resident = false;
+  };
+  Tick tick[2][2];  // over the full and the compacted tables, by PcgMode
   // PCG iterations in one tick: 16 measured best between the 64-scene mix's
   // total time (8 iterations: 8.6 s for 100 steps, 16: 8.0 s, 32: 7.7 s) and
   // the per-step latency of its light scenes
@@ -562,14 +570,16 @@ struct mfem_batch {
   int coop_grid = 0;  // blocks of the persistent PCG (all co-resident)
   bool auto_form = false;  // the scenes left the PCG form to the batch
   // the resident solve (k_resident.cu) of the batch's form, planned on first
-  // use: 0 not planned yet, 1 planned, -1 the batch does not fit
-  int cgr_state = 0;
+  // use: 0 not planned yet, 1 planned, -1 the batch does not fit; cgr_need: its
+  // blocks, known without the plan (0: not counted yet, -1: it does not fit)
+  int cgr_state = 0, cgr_need = 0;
+  bool cgr_streams = false;  // with cgr_need: the form that streams the matrix
+  int device = 0, sms = 0;
   char* cgr_mem = nullptr;
   CgrArgs cgr_args{};
   int cgr_blocks = 0, cgr_nthreads = 0;
   size_t cgr_smem_bytes = 0;
   bool cgr_wide = false;
-  bool loop_resident = false;  // the PCG loop graph's body starts with the resident solve
   int pstride = 0;  // tiles per partials quantity
   // instrumentation
   bool profiling = false;
@@ -814,12 +824,13 @@ int sync_counters(mfem_batch* b) {
     // a device-driven PCG loop has finished: its launches into the counts
     const int64_t bodies = b->h_ctr->cg_bodies;
     b->k_launches[MFEM_K_CG_LOOP] += 1 + bodies;  // k_cg_enter and one k_cg_continue a body
-    if (b->loop_fused) {
-      b->k_launches[MFEM_K_CGF_ITER] += bodies * b->cg_loop_len;
-      if (b->loop_resident) b->k_launches[MFEM_K_CG_SOLVE] += bodies;
+    const mfem_batch::Loop& l = b->cg_loop[b->loop_mode];
+    if (l.fused) {
+      b->k_launches[MFEM_K_CGF_ITER] += bodies * l.len;
+      if (l.resident) b->k_launches[MFEM_K_CG_SOLVE] += bodies;
     } else {
-      b->k_launches[MFEM_K_CG_SPMV] += bodies * b->cg_loop_len;
-      b->k_launches[MFEM_K_CG_UPDATE] += bodies * b->cg_loop_len;
+      b->k_launches[MFEM_K_CG_SPMV] += bodies * l.len;
+      b->k_launches[MFEM_K_CG_UPDATE] += bodies * l.len;
       if (!b->fp64) b->k_launches[MFEM_K_CG_REPLACE] += bodies;
     }
     b->loop_pending = false;
@@ -906,21 +917,25 @@ int worst_status(const SceneScalars& sc) {
 // fewest slices of 1, 2 and 4 for which every block has an SM of its own, for
 // a slice's product is 3400 cycles of its SM's FP64 pipe.  False: the batch
 // does not fit, or its form has no resident kernel.
-bool cgr_plan(mfem_batch* b) {
-  if (b->cgr_state != 0) return b->cgr_state > 0;
-  b->cgr_state = -1;
+struct CgrSplit {
+  std::vector<std::vector<int>> first;  // first slice of every block, per scene
+  int spb = 0;                          // slices a block, at most
+  bool wide = false;
+};
+bool cgr_split_blocks(const mfem_batch* b, CgrSplit* out) {
   const bool fused = b->pcg_kernel == MFEM_PCG_KERNEL_FUSED;
   const bool fp64 = b->fp64 != 0;
   if (b->minres || (fused && fp64)) return false;
-  int dev = 0, sms = 0, coop = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
-    return false;
+  for (const mfem_scene* s : b->scenes)
+    if (s->M.nf == 0) return false;
+  const int sms = b->sms;
+  int coop = 0;
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, b->device) != cudaSuccess || !coop) return false;
   const int n = (int)b->scenes.size();
-  // first slice of every block, per scene
-  std::vector<std::vector<int>> first(n);
-  int spb = fp64 ? 1 : kCgrTile;
+  std::vector<std::vector<int>>& first = out->first;
+  first.assign(n, {});
+  int& spb = out->spb;
+  spb = fp64 ? 1 : kCgrTile;
   long total = 0;
   for (;; spb *= 2) {
     total = 0;
@@ -931,7 +946,7 @@ bool cgr_plan(mfem_batch* b) {
     }
     if (!fp64 || total <= sms || spb >= kCgrMaxSpb64) break;
   }
-  const bool wide = fused && total > 2 * sms;
+  const bool wide = out->wide = fused && total > 2 * sms;
   if (wide) {
     // the fewest tiles a block for which every block has an SM
     for (spb = 3 * kCgrTile; spb <= kCgrWideSlices; spb += kCgrTile) {
@@ -972,6 +987,33 @@ bool cgr_plan(mfem_batch* b) {
     spb = 2 * kCgrTile;
     total = 1;
   }
+  return true;
+}
+
+// Blocks of the batch's resident solve, -1 where it has none.
+int cgr_blocks(mfem_batch* b) {
+  if (b->cgr_need == 0) {
+    CgrSplit p;
+    b->cgr_need = -1;
+    if (cgr_split_blocks(b, &p)) {
+      b->cgr_need = 0;
+      b->cgr_streams = p.wide;
+      for (const std::vector<int>& f : p.first) b->cgr_need += (int)f.size();
+    }
+  }
+  return b->cgr_need;
+}
+
+bool cgr_plan(mfem_batch* b) {
+  if (b->cgr_state != 0) return b->cgr_state > 0;
+  b->cgr_state = -1;
+  CgrSplit split;
+  if (!cgr_split_blocks(b, &split)) return false;
+  const bool fused = b->pcg_kernel == MFEM_PCG_KERNEL_FUSED;
+  const bool fp64 = b->fp64 != 0;
+  const int n = (int)b->scenes.size(), sms = b->sms, spb = split.spb;
+  const std::vector<std::vector<int>>& first = split.first;
+  const bool wide = split.wide;
   std::vector<CgrBlock> blocks;
   std::vector<int> h_col;
   std::vector<uint16_t> lidx;
@@ -980,7 +1022,6 @@ bool cgr_plan(mfem_batch* b) {
   int nrec = 0;
   for (int i = 0; i < n; ++i) {
     const HostMesh& M = b->scenes[i]->M;
-    if (M.nf == 0) return false;
     const int ns = (M.nf + 31) / 32, nblk = (int)first[i].size();
     const int ntile = (ns + kCgrTile - 1) / kCgrTile;
     if (ntile > (fp64 ? kCgrMaxTiles64 : wide ? kCgrWideTiles : INT_MAX)) return false;
@@ -1114,6 +1155,65 @@ bool cgr_plan(mfem_batch* b) {
   return true;
 }
 
+// SMs that the resident solves of the batches stepping on each device now want
+// (all of them for a batch without one): each call adds its batch's, and
+// mfem_gpu_batches_step_n all of its batches' before the first one steps.
+constexpr int kMaxDevices = 64;
+std::atomic<int> g_wanted[kMaxDevices];
+int sms_wanted(mfem_batch* b) { return cgr_blocks(b) > 0 ? cgr_blocks(b) : b->sms; }
+class Stepping {
+ public:
+  explicit Stepping(mfem_batch* b) : dev_(b->device), sms_(sms_wanted(b)) {
+    if (dev_ < kMaxDevices) g_wanted[dev_].fetch_add(sms_);
+  }
+  ~Stepping() { end(); }
+  void end() {
+    if (dev_ < kMaxDevices) g_wanted[dev_].fetch_sub(sms_);
+    sms_ = 0;
+  }
+  Stepping(const Stepping&) = delete;
+  Stepping& operator=(const Stepping&) = delete;
+
+ private:
+  int dev_, sms_;
+};
+
+// How a batch of the mixed path that left the form to the library, or steps
+// in ticks, runs its PCG now (the bits are the same).  A resident solve holds
+// an SM for each of its blocks until it ends, so batches that step side by side
+// and do not all fit solve in turns.  The launches of several batches interleave
+// instead (without programmatic dependent launches, whose early blocks hold SMs
+// that another batch's launch could use: the 64-scene mix in 4 lanes 1313
+// against 856 timesteps/s), an iteration of each at a time.  Turns of solves
+// that take a third or less of the time are the better until there are many,
+// so the line is drawn by how often the batches' blocks fill the SMs (three
+// steps of n equal batches in ms, resident / launches): two reductions, 6
+// times: 113 tiles, n = 2 / 4 / 8: 33 / 65, 65 / 79, 131 / 145; 263 tiles: 72 /
+// 112, 142 / 143, 284 / 266; several scenes 5 times (the 64-scene mix in 8
+// lanes: 838 timesteps/s, 6 times 803, resident 761); single reduction, 3.5
+// times: 113 tiles: 28 / 56,
+// 51 / 64, 103 / 90; sixteen scenes of 130 tiles: 36 / 56, 52 / 65, 98 / 86;
+// six of 215: 53 / 69, 103 / 89, 197 / 137.  The streamed form is faster than
+// its launches by a third at most and idles more with scenes of unlike solves:
+// never (16 scenes of 554 tiles, 135 / 115, 257 / 177; one of 334: 109 / 110,
+// 215 / 164) but for one scene that fills the SMs (873 tiles: 214 / 225, 439 /
+// 453).  FP64 launches take several times the resident solve: always resident.
+// A batch looks again before every solve or group of ticks.
+enum PcgMode { kPcgAlone = 0, kPcgBeside = 1 };
+PcgMode pcg_mode(mfem_batch* b) {
+  const int need = sms_wanted(b), wanted = b->device < kMaxDevices ? g_wanted[b->device].load() : 0;
+  if (b->fp64 || wanted <= std::max(need, b->sms)) return kPcgAlone;
+  if (cgr_blocks(b) <= 0) return kPcgBeside;
+  if (b->cgr_streams) return b->scenes.size() == 1 && 10 * need >= 9 * b->sms ? kPcgAlone : kPcgBeside;
+  const double turns = b->pcg_kernel == MFEM_PCG_KERNEL_FUSED ? 3.5 : b->scenes.size() == 1 ? 6.0 : 5.0;
+  return wanted <= turns * b->sms ? kPcgAlone : kPcgBeside;
+}
+CgfShape pcg_shape(const mfem_batch* b, PcgMode mode) {
+  CgfShape c = b->cgf_shape;
+  if (mode == kPcgBeside) c.pdl = 0;
+  return c;
+}
+
 cudaError_t cgr_launch(mfem_batch* b, int max_iters) {
   CgrArgs a = b->cgr_args;
   a.max_iters = max_iters;
@@ -1162,7 +1262,8 @@ int capture_cg_graph(mfem_batch* b, const Launch& Lcg, bool fused, cudaGraphExec
 // resident: the body is the resident solve, which ends when a stop of the
 // recursion is to be verified, and the three launches of k_cgf_iter that
 // verify it.
-int capture_cg_loop(mfem_batch* b, const Launch& Lcg, bool fused, bool resident, cudaGraphExec_t* out) {
+int capture_cg_loop(mfem_batch* b, const Launch& Lcg, bool fused, PcgMode mode, bool resident, mfem_batch::Loop* out) {
+  const CgfShape shape = pcg_shape(b, mode);
   const int len = resident ? 3 : fused ? 8 : kCgReplace;
   const int max_launch = b->max_cg + (fused && !b->fp64 ? 9 : 0);
   const int max_bodies = (max_launch + len - 1) / len + 1;
@@ -1204,7 +1305,7 @@ int capture_cg_loop(mfem_batch* b, const Launch& Lcg, bool fused, bool resident,
   if (resident) er = cgr_launch(b, 1 << 30);
   for (int k = 0; k < len; ++k) {
     if (fused) {
-      launch_cgf_iter(Lcg, b->cgf_shape);
+      launch_cgf_iter(Lcg, shape);
     } else {
       launch_cg_spmv(Lcg);
       launch_cg_update(Lcg);
@@ -1216,34 +1317,37 @@ int capture_cg_loop(mfem_batch* b, const Launch& Lcg, bool fused, bool resident,
   e = cudaStreamEndCapture(b->stream, &cap);
   if (e == cudaSuccess) e = er;
   if (e != cudaSuccess) return fail(e);
-  e = cudaGraphInstantiate(out, g, 0);
+  e = cudaGraphInstantiate(&out->graph, g, 0);
   cudaGraphDestroy(g);
   CUDA_OR(e, MFEM_ERR_CUDA);
-  b->cg_loop_len = len;
-  b->loop_fused = fused;
-  b->loop_resident = resident;
+  out->len = len;
+  out->fused = fused;
+  out->resident = resident;
   return MFEM_OK;
 }
 
 int run_pcg_graph(mfem_batch* b, const Launch& Lcg, bool fused) {
   const int len = fused ? 8 : kCgReplace;
-  if (b->cg_loop_on && !b->cg_loop) {
-    const bool resident = fused && b->auto_form && cgr_plan(b);
-    int rc = capture_cg_loop(b, Lcg, fused, resident, &b->cg_loop);
+  const PcgMode mode = fused ? pcg_mode(b) : kPcgAlone;  // (SPLIT: one launch form)
+  mfem_batch::Loop& loop = b->cg_loop[mode];
+  if (b->cg_loop_on && !loop.graph) {
+    const bool resident = fused && b->auto_form && mode == kPcgAlone && cgr_plan(b);
+    int rc = capture_cg_loop(b, Lcg, fused, mode, resident, &loop);
     if (rc != MFEM_OK && resident) {
       cudaGetLastError();
-      rc = capture_cg_loop(b, Lcg, fused, false, &b->cg_loop);
+      rc = capture_cg_loop(b, Lcg, fused, mode, false, &loop);
     }
     if (rc != MFEM_OK) {
       // conditional nodes unavailable: chunks with host checks instead
       cudaGetLastError();
-      b->cg_loop = nullptr;
+      loop.graph = nullptr;
       b->cg_loop_on = false;
     }
   }
-  if (b->cg_loop) {
+  if (loop.graph) {
     CUDA_OR(cudaMemsetAsync(&b->d_ctr->cg_bodies, 0, sizeof(int), b->stream), MFEM_ERR_CUDA);
-    CUDA_OR(cudaGraphLaunch(b->cg_loop, b->stream), MFEM_ERR_CUDA);
+    CUDA_OR(cudaGraphLaunch(loop.graph, b->stream), MFEM_ERR_CUDA);
+    b->loop_mode = mode;
     b->loop_pending = true;
     return MFEM_OK;
   }
@@ -1298,7 +1402,7 @@ int run_pcg(mfem_batch* b, const Launch& Lcg) {
   // a batch that chose its form itself runs that form's launches instead
   // (the same results), so that every kernel carries its own event pair.
   if ((b->pcg_kernel == MFEM_PCG_KERNEL_PERSISTENT ||
-       (b->pcg_kernel == MFEM_PCG_KERNEL_SPLIT && b->auto_form && !b->profiling)) &&
+       (b->pcg_kernel == MFEM_PCG_KERNEL_SPLIT && b->auto_form && !b->profiling && pcg_mode(b) == kPcgAlone)) &&
       cgr_plan(b)) {
     cudaError_t e;
     { KTimer t(b, MFEM_K_CG_SOLVE); e = cgr_launch(b, 1 << 30); }
@@ -1483,7 +1587,7 @@ constexpr int kTickResident = 128;
 // tables: every kernel of a Newton iteration once, each acting on the
 // scenes in its phase, with tick_pcg PCG iterations and one line-search
 // trial.
-int capture_tick_graph(mfem_batch* b, cudaGraphExec_t* out) {
+int capture_tick_graph(mfem_batch* b, PcgMode mode, mfem_batch::Tick* out) {
   Launch Lel = make_launch(b, TB_ELEM);
   Lel.variant = b->var_elem;
   const Launch Lev = make_launch(b, TB_EV);
@@ -1492,7 +1596,8 @@ int capture_tick_graph(mfem_batch* b, cudaGraphExec_t* out) {
   Lls.variant = b->var_ls;
   const Launch Lcg = make_launch(b, TB_CG);
   cudaGraph_t g = nullptr;
-  const bool resident = cgr_plan(b);
+  const bool resident = mode == kPcgAlone && cgr_plan(b);
+  const CgfShape shape = pcg_shape(b, mode);
   cudaError_t er = cudaSuccess;
   CUDA_OR(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), MFEM_ERR_CUDA);
   launch_elem_update(Lel, nullptr);
@@ -1500,7 +1605,7 @@ int capture_tick_graph(mfem_batch* b, cudaGraphExec_t* out) {
   launch_cgf_scale(Lcg);
   launch_cgf_init(Lcg);
   if (resident) er = cgr_launch(b, kTickResident);
-  for (int k = 0; k < (resident ? 3 : b->tick_pcg); ++k) launch_cgf_iter(Lcg, b->cgf_shape);
+  for (int k = 0; k < (resident ? 3 : b->tick_pcg); ++k) launch_cgf_iter(Lcg, shape);
   launch_local_solve(Llo);
   launch_ls_energy(Lls);
   launch_apply(Lev);
@@ -1511,10 +1616,27 @@ int capture_tick_graph(mfem_batch* b, cudaGraphExec_t* out) {
     if (g) cudaGraphDestroy(g);
     CUDA_OR(ec, MFEM_ERR_CUDA);
   }
-  const cudaError_t ei = cudaGraphInstantiate(out, g, 0);
+  const cudaError_t ei = cudaGraphInstantiate(&out->graph, g, 0);
   cudaGraphDestroy(g);
   CUDA_OR(ei, MFEM_ERR_CUDA);
+  out->resident = resident;
   return MFEM_OK;
+}
+
+// The graphs captured so far are dropped (the stream must be idle).
+void drop_ticks(mfem_batch::Tick (&t)[2]) {
+  for (mfem_batch::Tick& k : t) {
+    if (k.graph) cudaGraphExecDestroy(k.graph);
+    k = {};
+  }
+}
+void drop_loops(mfem_batch* b) {
+  if (b->cg_graph) cudaGraphExecDestroy(b->cg_graph);
+  b->cg_graph = nullptr;
+  for (mfem_batch::Loop& l : b->cg_loop) {
+    if (l.graph) cudaGraphExecDestroy(l.graph);
+    l = {};
+  }
 }
 
 // The kernels' tables become the tiles of the scenes with active[i] set
@@ -1539,9 +1661,8 @@ int compact_tables(mfem_batch* b, const std::vector<char>& active) {
   }
   int rc = upload_sds(b);
   if (rc) return rc;
-  if (b->tick_graph_c) cudaGraphExecDestroy(b->tick_graph_c);
-  b->tick_graph_c = nullptr;
-  return capture_tick_graph(b, &b->tick_graph_c);
+  drop_ticks(b->tick[1]);
+  return MFEM_OK;
 }
 
 // The full tables again.
@@ -1555,8 +1676,7 @@ int restore_tables(mfem_batch* b) {
       b->h_sds[i].tile_count[tb] = b->full_count[(size_t)i * TB_COUNT + tb];
     }
   }
-  if (b->tick_graph_c) cudaGraphExecDestroy(b->tick_graph_c);
-  b->tick_graph_c = nullptr;
+  drop_ticks(b->tick[1]);
   return upload_sds(b);
 }
 
@@ -1622,21 +1742,28 @@ int batch_step_n_impl(mfem_batch* b, int steps, mfem_step_stats* stats, double* 
     // trial; a scene goes as far through its iteration as the tick takes it
     // and never waits for another scene.  The host reads the batch's
     // counters after every few ticks, one check behind.
-    if (!b->tick_graph && (rc = capture_tick_graph(b, &b->tick_graph))) return rc;
     constexpr int kTicksPerCheck = 4;
     const long max_ticks = (long)steps * (b->max_newton + 2) * ((b->max_cg + 17) / b->tick_pcg + b->max_ls + 4);
     long ticks = 0;
     int nchunk = 0;
     bool finished = false;
     int table_scenes = n;  // scenes in the tables the ticks run over
-    cudaGraphExec_t tick = b->tick_graph;
+    bool compacted = false;
     while (ticks < max_ticks) {
+      const PcgMode mode = pcg_mode(b);
+      mfem_batch::Tick& tick = b->tick[compacted][mode];
+      if (!tick.graph && (rc = capture_tick_graph(b, mode, &tick))) {
+        if (compacted) restore_tables(b);
+        return rc;
+      }
       for (int r = 0; r < kTicksPerCheck; ++r, ++ticks) {
-        const cudaError_t e = cudaGraphLaunch(tick, b->stream);
+        const cudaError_t e = cudaGraphLaunch(tick.graph, b->stream);
         if (e != cudaSuccess) {
-          if (tick != b->tick_graph) restore_tables(b);
+          if (compacted) restore_tables(b);
           CUDA_OR(e, MFEM_ERR_CUDA);
         }
+        b->k_launches[MFEM_K_CG_SOLVE] += tick.resident;
+        b->k_launches[MFEM_K_CGF_ITER] += tick.resident ? 3 : b->tick_pcg;
       }
       const int slot = nchunk & 1;
       CUDA_OR(cudaMemcpyAsync(&b->h_ctr_pipe[slot], b->d_ctr, sizeof(BatchCounters), cudaMemcpyDeviceToHost,
@@ -1647,7 +1774,7 @@ int batch_step_n_impl(mfem_batch* b, int steps, mfem_step_stats* stats, double* 
         CUDA_OR(cudaEventSynchronize(b->ev_pipe[slot ^ 1]), MFEM_ERR_CUDA);
         const BatchCounters& c = b->h_ctr_pipe[slot ^ 1];
         if (c.error) {
-          if (tick != b->tick_graph) restore_tables(b);
+          if (compacted) restore_tables(b);
           return MFEM_ERR_TIMEOUT;
         }
         if (c.newton_active == 0) {
@@ -1674,7 +1801,7 @@ int batch_step_n_impl(mfem_batch* b, int steps, mfem_step_stats* stats, double* 
             restore_tables(b);
             return rc;
           }
-          tick = b->tick_graph_c;
+          compacted = true;
           table_scenes = na;
           nchunk = 0;
           continue;
@@ -1682,7 +1809,7 @@ int batch_step_n_impl(mfem_batch* b, int steps, mfem_step_stats* stats, double* 
       }
       ++nchunk;
     }
-    if (tick != b->tick_graph && (rc = restore_tables(b))) return rc;
+    if (compacted && (rc = restore_tables(b))) return rc;
     if (!finished) {
       if ((rc = sync_counters(b))) return rc;
       if (b->h_ctr->error) return MFEM_ERR_TIMEOUT;
@@ -2171,12 +2298,9 @@ int batch_build(mfem_scene* const* scenes, int n, mfem_batch** out) {
     if (scenes[i]->cfg.pcg_kernel != b->pcg_kernel || scenes[i]->dev.minres != b->minres ||
         scenes[i]->dev.fem != b->fem)
       return MFEM_ERR_INVALID;
-  int sms = 0;
-  {
-    int dev = 0;
-    CUDA_OR(cudaGetDevice(&dev), MFEM_ERR_CUDA);
-    CUDA_OR(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), MFEM_ERR_CUDA);
-  }
+  CUDA_OR(cudaGetDevice(&b->device), MFEM_ERR_CUDA);
+  CUDA_OR(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device), MFEM_ERR_CUDA);
+  const int sms = b->sms;
   b->auto_form = b->pcg_kernel == MFEM_PCG_KERNEL_AUTO;
   if (b->pcg_kernel == MFEM_PCG_KERNEL_AUTO)
     b->pcg_kernel = (b->ntiles[TB_CG] >= 2 * sms || (b->ntiles[TB_CG] <= 4 && !b->fp64))
@@ -2248,14 +2372,13 @@ void batch_free(mfem_batch* b) {
   if (b->cgr_mem) cudaFree(b->cgr_mem);
   if (b->h_ctr) cudaFreeHost(b->h_ctr);
   if (b->h_ctr_pipe) cudaFreeHost(b->h_ctr_pipe);
-  if (b->cg_graph) cudaGraphExecDestroy(b->cg_graph);
-  if (b->cg_loop) cudaGraphExecDestroy(b->cg_loop);
+  drop_loops(b);
+  drop_ticks(b->tick[0]);
+  drop_ticks(b->tick[1]);
   for (int k = 0; k < 2; ++k)
     if (b->ev_pipe[k]) cudaEventDestroy(b->ev_pipe[k]);
   if (b->h_sc) cudaFreeHost(b->h_sc);
   for (cudaEvent_t e : b->ev_pool) cudaEventDestroy(e);
-  if (b->tick_graph) cudaGraphExecDestroy(b->tick_graph);
-  if (b->tick_graph_c) cudaGraphExecDestroy(b->tick_graph_c);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -2636,6 +2759,7 @@ int mfem_gpu_scene_destroy(mfem_scene* scene) {
 int mfem_gpu_scene_step(mfem_scene* scene, mfem_step_stats* stats) {
   if (!scene) return MFEM_ERR_INVALID;
   mfem_step_stats st{};
+  Stepping now(scene->solo);
   int rc = batch_step_impl(scene->solo, &st);
   if (stats) *stats = st;
   return rc;
@@ -2976,17 +3100,10 @@ int mfem_gpu_batch_set_pcg_shape(mfem_batch* b, int32_t stages, int32_t keep, in
       b->cgf_shape.pdl == sh.pdl)
     return MFEM_OK;
   b->cgf_shape = sh;
-  if (b->cg_graph || b->cg_loop || b->tick_graph || b->tick_graph_c) {  // captured with the old shape
-    CUDA_OR(cudaStreamSynchronize(b->stream), MFEM_ERR_CUDA);
-    if (b->cg_graph) cudaGraphExecDestroy(b->cg_graph);
-    if (b->cg_loop) cudaGraphExecDestroy(b->cg_loop);
-    if (b->tick_graph) cudaGraphExecDestroy(b->tick_graph);
-    if (b->tick_graph_c) cudaGraphExecDestroy(b->tick_graph_c);
-    b->cg_graph = nullptr;
-    b->cg_loop = nullptr;
-    b->tick_graph = nullptr;
-    b->tick_graph_c = nullptr;
-  }
+  CUDA_OR(cudaStreamSynchronize(b->stream), MFEM_ERR_CUDA);
+  drop_loops(b);  // captured with the old shape
+  drop_ticks(b->tick[0]);
+  drop_ticks(b->tick[1]);
   return MFEM_OK;
 }
 
@@ -3007,11 +3124,9 @@ int mfem_gpu_batch_set_variants(mfem_batch* b, int32_t elem_update, int32_t loca
   b->var_elem = elem_update;
   b->var_local = local_solve;
   b->var_ls = ls_energy;
-  if (b->tick_graph) {  // captured with the old variants
-    CUDA_OR(cudaStreamSynchronize(b->stream), MFEM_ERR_CUDA);
-    cudaGraphExecDestroy(b->tick_graph);
-    b->tick_graph = nullptr;
-  }
+  CUDA_OR(cudaStreamSynchronize(b->stream), MFEM_ERR_CUDA);
+  drop_ticks(b->tick[0]);  // captured with the old variants
+  drop_ticks(b->tick[1]);
   return MFEM_OK;
 }
 
@@ -3054,11 +3169,13 @@ int mfem_gpu_batch_destroy(mfem_batch* batch) {
 
 int mfem_gpu_batch_step_n(mfem_batch* batch, int32_t steps, mfem_step_stats* stats, double* step_done_ms) {
   if (!batch || steps < 1 || steps > MFEM_BATCH_MAX_STEPS) return MFEM_ERR_INVALID;
+  Stepping now(batch);
   return batch_step_n_impl(batch, steps, stats, step_done_ms);
 }
 
 int mfem_gpu_batch_step(mfem_batch* batch, mfem_step_stats* stats) {
   if (!batch) return MFEM_ERR_INVALID;
+  Stepping now(batch);
   return batch_step_impl(batch, stats);
 }
 
@@ -3082,6 +3199,8 @@ int mfem_gpu_batches_step_n(mfem_batch* const* batches, int32_t nbatch, int32_t 
   // one host thread per batch, each driving its batch's stream; the GPU
   // runs the batches' launches side by side
   std::vector<int> rc(nbatch, MFEM_OK);
+  std::vector<std::unique_ptr<Stepping>> now(nbatch);  // all of them from the start
+  for (int k = 0; k < nbatch; ++k) now[k].reset(new Stepping(batches[k]));
   std::vector<std::thread> th;
   th.reserve(nbatch);
   for (int k = 0; k < nbatch; ++k)
@@ -3092,6 +3211,7 @@ int mfem_gpu_batches_step_n(mfem_batch* const* batches, int32_t nbatch, int32_t 
       }
       rc[k] = batch_step_n_impl(batches[k], steps, stats ? stats + first[k] : nullptr,
                                 step_done_ms ? step_done_ms + first[k] * (size_t)steps : nullptr);
+      now[k]->end();
     });
   for (std::thread& t : th) t.join();
   // the first failure of the call in batch order; a retired scene's
