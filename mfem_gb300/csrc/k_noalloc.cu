@@ -745,7 +745,7 @@ extern "C" int mfem_gpu_bsr_pcg_noalloc(int32_t n_block_rows, int32_t nnzb, cons
       return MFEM_ERR_CUDA;
     }
     // the resident form: its shared memory, and how many of its blocks fit
-    int sms = 0, per_sm = 0;
+    int sms = 0, per_sm = 0, coop = 0;
     const unsigned int first_tag = 1;  // the records start with tag 0
     if (cudaMemcpyAsync(static_cast<unsigned char*>(p) + kNaOffSeq, &first_tag, sizeof(first_tag),
                         cudaMemcpyHostToDevice, static_cast<cudaStream_t>(stream)) != cudaSuccess ||
@@ -757,6 +757,7 @@ extern "C" int mfem_gpu_bsr_pcg_noalloc(int32_t n_block_rows, int32_t nnzb, cons
              per_sm > 0;
     };
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
         ready((const void*)k_na_resident<kNaFewSlices>, kNaFewSlices) &&
         ready((const void*)k_na_resident<kNaMaxSlices>, kNaMaxSlices))
       g_na_sms[dev] = per_sm > 0 ? std::min(sms, kNaMaxBlocks) : 0;
@@ -782,10 +783,14 @@ extern "C" int mfem_gpu_bsr_pcg_noalloc(int32_t n_block_rows, int32_t nnzb, cons
                                                                           : (const void*)k_na_resident<kNaMaxSlices>,
                                                       dim3((slices + spb - 1) / spb),
                                                       dim3(96 * spb), args, kNaSmem, st);
-    if (e != cudaSuccess) return MFEM_ERR_CUDA;
-    if (cudaMemcpyAsync(&h, v.sc, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
+    // refused (a stream or process that is limited to a part of the SMs): h says
+    // not done, and the launches, which need no co-residency, take the system
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+    } else if (cudaMemcpyAsync(&h, v.sc, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+               cudaStreamSynchronize(st) != cudaSuccess) {
       return MFEM_ERR_CUDA;
+    }
     if (h.error) return MFEM_ERR_TIMEOUT;
     if (h.done) {
       if (iterations) *iterations = h.iter;

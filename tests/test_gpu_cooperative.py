@@ -1,0 +1,52 @@
+"""Cooperative launches that the runtime refuses (a stream or process limited to
+a part of the SMs): the forms that need no co-residency run instead.  Each test
+runs in a child process whose cooperative launches go through a stand-in."""
+import pytest
+
+import coop_calls
+
+pytestmark = pytest.mark.gpu
+
+SCENE = """
+from mfem_gb300 import abi, gpu
+from mfem_gb300.desc import SceneSpec
+from mfem_gb300.meshgen import cube_grid, enu_to_lame, face_mask
+def scene(dims, prec, kern, **kw):
+    V, T = cube_grid(*dims, 0.05)
+    lam, mu = enu_to_lame(2e5, 0.4)
+    return gpu.Scene(SceneSpec(V_rest=V, tets=T, mu=np.full(len(T), mu), lam=np.full(len(T), lam),
+                               is_fixed=face_mask(V, 0, "min"), dt=1 / 60, body_force=(0.0, -9.8, 0.0),
+                               max_newton_iterations=3, iterative_solver_tolerance=1e-6, precision=prec,
+                               max_iterative_solver_iters=400, pcg_kernel=kern, **kw))
+M, D = abi.PRECISION_MIXED, abi.PRECISION_FP64
+"""
+
+
+def test_allocation_free_solve(gpu_lib, tmp_path):
+    # (980 rows: 31 blocks; both solves to 1e-10, their sums in another order)
+    coop_calls.run(tmp_path, SCENE, """
+    import torch
+    from mfem_gb300._lib import load
+    sc = scene((20, 6, 6), D, abi.PCG_KERNEL_SPLIT, linear_solver=abi.SOLVER_GPU_PCG_BLOCK)
+    sc.step()
+    rp, col, val, rhs = sc.get_system()
+    dev = [torch.from_numpy(np.ascontiguousarray(a).ravel()).cuda() for a in (rp, col, val, rhs)]
+    x = torch.zeros(3 * sc.n_free, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    def solve():
+        it, err = C.c_int32(-1), C.c_double(-1)
+        x.zero_()
+        torch.cuda.synchronize()
+        rc = load().mfem_gpu_bsr_pcg_noalloc(sc.n_free, sc.nnzb, *[C.c_void_p(a.data_ptr()) for a in dev],
+                                             C.c_void_p(x.data_ptr()), 3000, C.c_double(1e-10), None, C.byref(it),
+                                             C.byref(err))
+        return rc, it.value, x.cpu().numpy()
+    rc, it, ref = solve()
+    assert rc == 0 and it > 0 and any("k_na_resident" in n for n in launched())
+    for on, runs in ((1, False), (1, False), (0, True)):
+        lib.coop_refuse(on)
+        rc, n, y = solve()
+        assert rc == 0 and abs(n - it) <= max(2, it // 50), (rc, n, it)
+        assert any("k_na_resident" in k for k in launched()) == runs
+        assert np.abs(y - ref).max() <= 1e-7 * np.abs(ref).max()
+    """)
