@@ -1214,6 +1214,13 @@ CgfShape pcg_shape(const mfem_batch* b, PcgMode mode) {
   return c;
 }
 
+// The runtime refused the resident launch (a process limited to a part of the
+// SMs, say): the batch runs its launches from now on.
+void cgr_refused(mfem_batch* b) {
+  cudaGetLastError();
+  b->cgr_state = -1;
+}
+
 cudaError_t cgr_launch(mfem_batch* b, int max_iters) {
   CgrArgs a = b->cgr_args;
   a.max_iters = max_iters;
@@ -1334,7 +1341,7 @@ int run_pcg_graph(mfem_batch* b, const Launch& Lcg, bool fused) {
     const bool resident = fused && b->auto_form && mode == kPcgAlone && cgr_plan(b);
     int rc = capture_cg_loop(b, Lcg, fused, mode, resident, &loop);
     if (rc != MFEM_OK && resident) {
-      cudaGetLastError();
+      cgr_refused(b);
       rc = capture_cg_loop(b, Lcg, fused, mode, false, &loop);
     }
     if (rc != MFEM_OK) {
@@ -1346,7 +1353,14 @@ int run_pcg_graph(mfem_batch* b, const Launch& Lcg, bool fused) {
   }
   if (loop.graph) {
     CUDA_OR(cudaMemsetAsync(&b->d_ctr->cg_bodies, 0, sizeof(int), b->stream), MFEM_ERR_CUDA);
-    CUDA_OR(cudaGraphLaunch(loop.graph, b->stream), MFEM_ERR_CUDA);
+    const cudaError_t e = cudaGraphLaunch(loop.graph, b->stream);
+    if (e != cudaSuccess && loop.resident) {
+      cgr_refused(b);
+      cudaGraphExecDestroy(loop.graph);
+      loop = {};
+      return run_pcg_graph(b, Lcg, fused);
+    }
+    CUDA_OR(e, MFEM_ERR_CUDA);
     b->loop_mode = mode;
     b->loop_pending = true;
     return MFEM_OK;
@@ -1406,8 +1420,9 @@ int run_pcg(mfem_batch* b, const Launch& Lcg) {
       cgr_plan(b)) {
     cudaError_t e;
     { KTimer t(b, MFEM_K_CG_SOLVE); e = cgr_launch(b, 1 << 30); }
-    CUDA_OR(e, MFEM_ERR_CUDA);
-    return MFEM_OK;
+    if (e == cudaSuccess) return MFEM_OK;
+    b->k_launches[MFEM_K_CG_SOLVE] -= 1;
+    cgr_refused(b);
   }
   if (b->pcg_kernel == MFEM_PCG_KERNEL_PERSISTENT) {
     cudaError_t e;
@@ -1612,13 +1627,16 @@ int capture_tick_graph(mfem_batch* b, PcgMode mode, mfem_batch::Tick* out) {
   launch_step_turn(Lev);
   cudaError_t ec = cudaStreamEndCapture(b->stream, &g);
   if (ec == cudaSuccess) ec = er;
+  if (ec == cudaSuccess) ec = cudaGraphInstantiate(&out->graph, g, 0);
+  if (g) cudaGraphDestroy(g);
   if (ec != cudaSuccess) {
-    if (g) cudaGraphDestroy(g);
+    out->graph = nullptr;
+    if (resident) {
+      cgr_refused(b);
+      return capture_tick_graph(b, mode, out);
+    }
     CUDA_OR(ec, MFEM_ERR_CUDA);
   }
-  const cudaError_t ei = cudaGraphInstantiate(&out->graph, g, 0);
-  cudaGraphDestroy(g);
-  CUDA_OR(ei, MFEM_ERR_CUDA);
   out->resident = resident;
   return MFEM_OK;
 }
@@ -1757,7 +1775,14 @@ int batch_step_n_impl(mfem_batch* b, int steps, mfem_step_stats* stats, double* 
         return rc;
       }
       for (int r = 0; r < kTicksPerCheck; ++r, ++ticks) {
-        const cudaError_t e = cudaGraphLaunch(tick.graph, b->stream);
+        cudaError_t e = cudaGraphLaunch(tick.graph, b->stream);
+        if (e != cudaSuccess && tick.resident) {
+          cgr_refused(b);
+          cudaGraphExecDestroy(tick.graph);
+          tick = {};
+          rc = capture_tick_graph(b, mode, &tick);
+          e = rc ? cudaErrorUnknown : cudaGraphLaunch(tick.graph, b->stream);
+        }
         if (e != cudaSuccess) {
           if (compacted) restore_tables(b);
           CUDA_OR(e, MFEM_ERR_CUDA);

@@ -50,3 +50,31 @@ def test_allocation_free_solve(gpu_lib, tmp_path):
         assert any("k_na_resident" in k for k in launched()) == runs
         assert np.abs(y - ref).max() <= 1e-7 * np.abs(ref).max()
     """)
+
+
+@pytest.mark.parametrize("form", ["split", "fused", "ticks"])
+def test_scenes_that_leave_the_form_to_the_library(gpu_lib, tmp_path, form):
+    """Six tiles: the two-reduction solve; one tile: the single-reduction loop;
+    a batch of those in ticks.  The launches take the same steps, bitwise."""
+    coop_calls.run(tmp_path, SCENE, f"""
+    form = {form!r}
+    def steps():
+        if form == "ticks":
+            s = [scene(d, M, abi.PCG_KERNEL_FUSED) for d in [(13, 9, 9), (7, 5, 5)]]
+            b = gpu.Batch(s)
+            b.step_n(2)
+            h = b.handle
+        else:
+            s = [scene((13, 9, 9) if form == "split" else (7, 5, 5), M, abi.PCG_KERNEL_AUTO)]
+            for _ in range(2):
+                s[0].step(raise_on_error=False)
+            h = s[0].solo_batch_handle()
+        return [x.positions() for x in s], gpu.kernel_stats(h)["k_cg_solve"][1], launched()
+    ref, n, names = steps()
+    kernel = dict(split="k_cgr_split", fused="k_cgr_fused", ticks="k_cgr_fused")[form]
+    assert n > 0 and any(kernel in k for k in names), names
+    lib.coop_refuse(1)
+    got, n, names = steps()
+    assert n == 0 and not names
+    assert all(np.array_equal(a, b) for a, b in zip(ref, got))
+    """)
