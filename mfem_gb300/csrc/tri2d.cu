@@ -1370,8 +1370,8 @@ struct mfem_tri2d {
   struct Pending { int kernel, a, b; };
   std::vector<Pending> ev_pending;
   size_t ev_used = 0;
-  // blocks of the grid PCG (t2_pcg_grid), 0: the resident one, of res_grid
-  // blocks (t2_pcg_res2 up to 1024 free rows, t2_pcg_res above)
+  // blocks of the resident PCG (t2_pcg_res2 up to 1024 free rows, t2_pcg_res
+  // above); 0: the grid PCG, of pcg_grid blocks (one is launched plainly)
   int pcg_grid = 0, res_grid = 0;
   size_t res_smem = 0;
   // configuration
@@ -1636,31 +1636,30 @@ int t2_step(mfem_tri2d& sc, mfem_step_stats* out) {
     st.residual = rn;
     if (sc.res_tol > 0 && ((i > 0 && rn <= sc.res_tol * st.residual0) || rn <= sc.res_tol * sc.load_norm))
       break;
-    if (sc.nf > 0 && sc.pcg_grid > 0) {
-      // a fresh barrier (arrivals, generation, error) for the cooperative launch
+    if (sc.nf > 0) {
+      T2 dd = sc.d;
+      int mi = sc.cg_iters;
+      double tl = sc.cg_tol;
+      void* args[] = {&dd, &mi, &tl};
+      // a fresh barrier (arrivals, generation, error)
       T2_CUDA(cudaMemsetAsync(sc.d.bar, 0, 4 * sizeof(unsigned int), sc.stream));
       cudaError_t e = cudaSuccess;
       launch(sc, MFEM_T2_K_PCG, [&] {
-        T2 dd = sc.d;
-        int mi = sc.cg_iters;
-        double tl = sc.cg_tol;
-        void* args[] = {&dd, &mi, &tl};
-        e = cudaLaunchCooperativeKernel((const void*)t2_pcg_grid, dim3(sc.pcg_grid), dim3(kGridThreads), args, 0,
-                                        sc.stream);
+        if (sc.res_grid > 0)
+          e = cudaLaunchCooperativeKernel(t2_res_kernel(sc.nf <= 1024), dim3(sc.res_grid), dim3(kResThreads), args,
+                                          sc.res_smem, sc.stream);
+        else if (sc.pcg_grid > 1)
+          e = cudaLaunchCooperativeKernel((const void*)t2_pcg_grid, dim3(sc.pcg_grid), dim3(kGridThreads), args, 0,
+                                          sc.stream);
+        if (e != cudaSuccess) {
+          // refused (a process limited to a part of the SMs, say): one block
+          // needs no other from now on
+          cudaGetLastError();
+          sc.res_grid = 0;
+          sc.pcg_grid = 1;
+        }
+        if (sc.res_grid == 0 && sc.pcg_grid == 1) t2_pcg_grid<<<1, kGridThreads, 0, sc.stream>>>(dd, mi, tl);
       });
-      T2_CUDA(e);
-    } else if (sc.nf > 0) {
-      T2_CUDA(cudaMemsetAsync(sc.d.bar, 0, 4 * sizeof(unsigned int), sc.stream));
-      cudaError_t e = cudaSuccess;
-      launch(sc, MFEM_T2_K_PCG, [&] {
-        T2 dd = sc.d;
-        int mi = sc.cg_iters;
-        double tl = sc.cg_tol;
-        void* args[] = {&dd, &mi, &tl};
-        e = cudaLaunchCooperativeKernel(t2_res_kernel(sc.nf <= 1024), dim3(sc.res_grid), dim3(kResThreads), args,
-                                        sc.res_smem, sc.stream);
-      });
-      T2_CUDA(e);
     }
     launch(sc, MFEM_T2_K_LOCAL, [&] { t2_local<<<grid_of(sc.nt), kThreads, 0, sc.stream>>>(sc.d); });
     if (launch_status() != MFEM_OK) return MFEM_ERR_CUDA;

@@ -78,3 +78,34 @@ def test_scenes_that_leave_the_form_to_the_library(gpu_lib, tmp_path, form):
     assert n == 0 and not names
     assert all(np.array_equal(a, b) for a, b in zip(ref, got))
     """)
+
+
+@pytest.mark.parametrize("nx,ny,kernel", [(12, 8, "t2_pcg_res2"), (64, 20, "t2_pcg_res")])  # 99 and 1,302 free rows
+def test_sheets(gpu_lib, tmp_path, nx, ny, kernel):
+    # (Newton's converged states of forms that add in another order: 1e-9 of
+    # the sheet apart; the bound is the one on parity, 1e-6)
+    coop_calls.run(tmp_path, "", f"""
+    from mfem_gb300 import abi
+    from mfem_gb300.desc import Tri2dSpec
+    from mfem_gb300.meshgen import enu_to_lame, square_grid
+    from mfem_gb300.tri2d import Tri2dScene
+    def steps():
+        V, T = square_grid({nx}, {ny}, 1.0 / {nx})
+        lam, mu = enu_to_lame(1e5, 0.45)
+        sc = Tri2dScene(Tri2dSpec(V_rest=V, tris=T, mu=np.full(len(T), float(mu)), lam=np.full(len(T), float(lam)),
+                                  density_const=1000.0, bc_type=abi.BC_HANGENDS, bc_ratio=0.01, bc_axis=0, dt=0.0333,
+                                  body_force=(0.0, -9.8, 0.0), max_newton_iterations=10,
+                                  max_linesearch_iterations=20, max_iterative_solver_iters=10000,
+                                  iterative_solver_tolerance=1e-10))
+        st = [sc.step() for _ in range(2)]
+        x = sc.get_state()["x"]
+        n = sc.n_free
+        sc.close()
+        return np.array(x), n, launched()
+    ref, n, names = steps()
+    assert any({kernel!r} in k for k in names), (n, names)
+    lib.coop_refuse(1)
+    got, n, names = steps()
+    assert not names
+    assert np.abs(got - ref).max() <= 1e-6, np.abs(got - ref).max()
+    """)
