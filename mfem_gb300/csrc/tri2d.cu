@@ -109,9 +109,7 @@ struct T2 {
   double* A;     // 4 nnzb row-major blocks
   double* rhs;   // 2 nf
   double* dinv;  // 2 nf
-  double* r;     // PCG vectors, 2 nf
-  double* p;
-  double* q;
+  double* p;     // the grid PCG's p, 2 nf
   double* sr;     // the grid PCG's r, w, s by iteration parity: 6 x 2 nf (r0 r1 w0 w1 s0 s1)
   double* part;   // the grid PCG's block partials: 3 x kT2MaxGrid
   unsigned int* bar;  // the grid PCG's barrier: arrivals, generation, error flag
@@ -453,8 +451,8 @@ __global__ void __launch_bounds__(kBlock) t2_norm(T2 d) {
 }
 
 // ----------------------------------------------------- grid PCG ---
-// The Jacobi-PCG of sheets too large for t2_pcg_res.  One cooperative launch of G blocks of kGridThreads, each
-// owning a contiguous range of free rows; a reduction is each block's
+// The Jacobi-PCG of sheets that t2_pcg_res does not fit.  One cooperative
+// launch of G blocks of kGridThreads, each owning a contiguous range of free rows; a reduction is each block's
 // fixed-order partial, a bounded grid barrier, and the G partials summed in
 // the same fixed order by every block (so every block takes the same
 // branches).  The iteration is the single-reduction form of the same PCG
@@ -2021,8 +2019,7 @@ int mfem_gpu_tri2d_create(const mfem_tri2d_desc* dsc, mfem_tri2d** out) {
                o_A = L.take<double>(4 * size_t(std::max(nnzb, 1))),
                o_rhs = L.take<double>(2 * size_t(std::max(nf, 1))),
                o_dinv = L.take<double>(2 * size_t(std::max(nf, 1))),
-               o_r = L.take<double>(2 * size_t(std::max(nf, 1))), o_p = L.take<double>(2 * size_t(std::max(nf, 1))),
-               o_q = L.take<double>(2 * size_t(std::max(nf, 1))),
+               o_p = L.take<double>(2 * size_t(std::max(nf, 1))),
                o_sr = L.take<double>(12 * size_t(std::max(nf, 1))), o_part = L.take<double>(3 * kT2MaxGrid),
                o_bar = L.take<unsigned int>(4),
                o_rslot = L.take<int>(res_slot.size()), o_rhp = L.take<int>(res_hptr.size()),
@@ -2099,9 +2096,7 @@ int mfem_gpu_tri2d_create(const mfem_tri2d_desc* dsc, mfem_tri2d** out) {
   d.A = dp(o_A);
   d.rhs = dp(o_rhs);
   d.dinv = dp(o_dinv);
-  d.r = dp(o_r);
   d.p = dp(o_p);
-  d.q = dp(o_q);
   d.sr = dp(o_sr);
   d.part = dp(o_part);
   d.bar = reinterpret_cast<unsigned int*>(base + o_bar);
