@@ -1004,6 +1004,31 @@ int cgr_blocks(mfem_batch* b) {
   return b->cgr_need;
 }
 
+// What a scene adds to its batch's plan in device memory at most (0: no plan
+// takes it).  The halos are those of the smallest blocks there are: a block
+// made of two has no more than both.
+size_t cgr_bytes(const mfem_scene_desc& cfg, const HostMesh& M, bool fp64) {
+  const int ns = (M.nf + 31) / 32, ntile = (ns + kCgrTile - 1) / kCgrTile;
+  if (M.nf == 0 || cfg.linear_solver == MFEM_SOLVER_MINRES_ID || cfg.pcg_kernel == MFEM_PCG_KERNEL_SPLIT ||
+      (fp64 && cfg.pcg_kernel == MFEM_PCG_KERNEL_FUSED) || ntile > (fp64 ? kCgrMaxTiles64 : kCgrWideTiles))
+    return 0;
+  const int spb = fp64 ? 1 : kCgrTile;
+  std::vector<int> seen(M.nf, -1);
+  size_t halo = 0, blocks = 0;
+  for (int s0 = 0; s0 < ns; s0 += spb, ++blocks) {
+    const int s1 = std::min(ns, s0 + spb), r0 = 32 * s0, r1 = std::min(M.nf, 32 * s1);
+    for (int q = M.slice_off[s0]; q < M.slice_off[s1]; ++q) {
+      const int c = M.ell_col[q];
+      if ((c >= r0 && c < r1) || seen[c] == s0) continue;
+      seen[c] = s0;
+      ++halo;
+    }
+  }
+  return blocks * (sizeof(CgrBlock) + kCgrWideSlices) + 4 * halo + 2 * M.ell_col.size() +
+         2 * kMaxCopies * 3 * sizeof(uint4) * (size_t)(fp64 ? ns : ntile) +
+         2 * sizeof(uint4) * (size_t)M.nf * (fp64 ? 3 : 1) + sizeof(unsigned int) + 7 * 256;
+}
+
 bool cgr_plan(mfem_batch* b) {
   if (b->cgr_state != 0) return b->cgr_state > 0;
   b->cgr_state = -1;
@@ -2736,10 +2761,12 @@ int mfem_gpu_scene_footprint(const mfem_scene_desc* desc, int64_t* bytes) {
   if (rc) return rc;
   size_t b = 0;
   scene_layout_bytes(s.get(), &b);
-  // plus the single-scene batch (tile tables, partials)
+  // plus the single-scene batch (tile tables, partials, step times) and its plan
   const size_t tiles = (size_t)(s->M.nt / kElemTile + 1) * 2 + s->M.nf / kRowTile + s->M.nf / kCgRows +
                        s->M.nv / kVertTile + 8;  // tile tables of the single-scene batch
-  *bytes = (int64_t)(b + tiles * (sizeof(Tile) + kNumPartials * sizeof(double)) + 4096);
+  *bytes = (int64_t)(b + tiles * (2 * sizeof(Tile) + kNumPartials * sizeof(double)) + sizeof(SceneDev) +
+                     (kMaxCallSteps + 1) * sizeof(unsigned long long) + 4096 +
+                     cgr_bytes(s->cfg, s->M, s->fp64 != 0));
   return MFEM_OK;
 }
 

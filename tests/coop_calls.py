@@ -1,7 +1,7 @@
 """A stand-in for cudaLaunchCooperativeKernel, compiled and preloaded into a child
 process: it counts the launches by kernel name and, on request, refuses them as
 the runtime refuses a grid that cannot be co-resident, or leaves out the last
-block of the grid."""
+block of the grid.  Beside it one for cudaMalloc that adds up the bytes."""
 import os
 import subprocess
 import sys
@@ -17,6 +17,14 @@ typedef struct { unsigned x, y, z; } dim;
 typedef int (*launch_t)(const void*, dim, dim, void**, unsigned long, void*);
 typedef int (*name_t)(const char**, const void*);
 static int refuse_, drop_;
+static unsigned long bytes_;
+unsigned long malloc_bytes(void) { return bytes_; }
+int cudaMalloc(void** p, unsigned long n) {
+  static int (*next)(void**, unsigned long);
+  if (!next) next = (int (*)(void**, unsigned long))dlsym(dlopen("libcudart.so.13", RTLD_LAZY), "cudaMalloc");
+  bytes_ += n;
+  return next(p, n);
+}
 static char names_[1 << 20];
 void coop_refuse(int on) { refuse_ = on; }
 void coop_drop(int on) { drop_ = on; }
@@ -48,6 +56,7 @@ sys.path.insert(0, {root!r})
 import numpy as np
 lib = C.CDLL({so!r})
 lib.coop_names.restype = C.c_char_p
+lib.malloc_bytes.restype = C.c_ulong
 def launched():
     names = lib.coop_names().decode().split()
     lib.coop_clear()
