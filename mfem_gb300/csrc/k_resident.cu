@@ -82,7 +82,8 @@ struct CgrShared {
 // one or two tiles, a scene of one block nothing.  `ahead` runs once the
 // other blocks' sums have come in, before the last of the adding: loads issued
 // there are under way meanwhile; `during` before, while the sums travel.
-// False: a wait ran out.
+// False: a wait ran out; of up to 32 records for the warps whose wait it was,
+// of more for the whole block.
 template <typename E, int NQ, typename F, typename G>
 __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B, CgrShared& S, bool lead, int sl,
                                             unsigned seq, E (&v)[NQ], const F& ahead, const G& during) {
@@ -151,10 +152,11 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
   E s[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) s[q] = E(0);
+  bool ok = true;
   if (warp < 8) {
-    for (int i0 = 32 * warp; i0 < n; i0 += 256) {
+    for (int i0 = 32 * warp; i0 < n && ok; i0 += 256) {
       E a[NQ];
-      if (!fetch(i0 + lane, a)) return false;
+      ok = fetch(i0 + lane, a);
 #pragma unroll
       for (int q = 0; q < NQ; ++q) s[q] = radd(s[q], a[q]);
     }
@@ -163,7 +165,8 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
 #pragma unroll
       for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.red[par][q][warp], s[q]);
   }
-  __syncthreads();
+  // (the warps wait for different records: all of them leave or none)
+  if (!__syncthreads_and(ok)) return false;
   ahead();
 #pragma unroll
   for (int q = 0; q < NQ; ++q) v[q] = lane < 8 ? Slot<E>::sget(&S.red[par][q][lane]) : E(0);
@@ -1051,22 +1054,27 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
         }
       }
     }
-    if (!scene_total<df64, 3>(A, B, S, roww, sl, seq, d, [&]() {
+    const bool got = scene_total<df64, 3>(A, B, S, roww, sl, seq, d, [&]() {
 #pragma unroll
           for (int j = 0; j < kHaloRegs; ++j)
             if (hw[j]) hv[j] = ld_rec(A.pub + (size_t)(seq & 1) * A.pub_stride + B.row0 + hc[j]);
-        }, [&]() { if (!kOne || threadIdx.x == 0) q.prepare(); })) {
-      cgr_abort(A, B);
-      return;
-    }
+        }, [&]() { if (!kOne || threadIdx.x == 0) q.prepare(); });
     wtag = seq;
     ++seq;
     if (kOne) {
-      if (threadIdx.x == 0) leave = q.step(sd, d) || n + 1 >= A.max_iters;
-      __syncthreads();
+      // (thread 0's step ends the loop for all: no warp goes on without it)
+      if (got && threadIdx.x == 0) leave = q.step(sd, d) || n + 1 >= A.max_iters;
+      if (!__syncthreads_and(got)) {
+        cgr_abort(A, B);
+        return;
+      }
       if (leave) break;
-    } else if (q.step(sd, d) || n + 1 >= A.max_iters) {
-      break;
+    } else {
+      if (!got) {
+        cgr_abort(A, B);
+        return;
+      }
+      if (q.step(sd, d) || n + 1 >= A.max_iters) break;
     }
   }
   // ---- the vectors as k_cgf_iter leaves them after iteration `last`

@@ -1,6 +1,7 @@
 """Cooperative launches that the runtime refuses (a stream or process limited to
-a part of the SMs): the forms that need no co-residency run instead.  Each test
-runs in a child process whose cooperative launches go through a stand-in."""
+a part of the SMs): the forms that need no co-residency run instead.  And waits
+between their blocks that run out.  Each test runs in a child process whose
+cooperative launches go through a stand-in."""
 import pytest
 
 import coop_calls
@@ -49,6 +50,12 @@ def test_allocation_free_solve(gpu_lib, tmp_path):
         assert rc == 0 and abs(n - it) <= max(2, it // 50), (rc, n, it)
         assert any("k_na_resident" in k for k in launched()) == runs
         assert np.abs(y - ref).max() <= 1e-7 * np.abs(ref).max()
+    # rows that nobody sends: the wait runs out, the next solve is as ever
+    lib.coop_drop(1)
+    assert solve()[0] == abi.ERR_TIMEOUT
+    lib.coop_drop(0)
+    rc, n, y = solve()
+    assert rc == 0 and n == it and np.array_equal(y, ref)
     """)
 
 
@@ -108,4 +115,49 @@ def test_sheets(gpu_lib, tmp_path, nx, ny, kernel):
     got, n, names = steps()
     assert not names
     assert np.abs(got - ref).max() <= 1e-6, np.abs(got - ref).max()
+    """)
+
+
+# k_cgr_split (6, 33 and 263 tiles), k_cgr_split64, k_cgr_wide; in ticks k_cgr_fused of 8 and of 16 warps
+@pytest.mark.parametrize("dims,prec,kern,n", [
+    ((13, 9, 9), "M", "PERSISTENT", 1), ((16, 21, 23), "M", "PERSISTENT", 1), ((40, 40, 40), "M", "PERSISTENT", 1),
+    ((13, 9, 9), "D", "PERSISTENT", 1), ((57, 32, 45), "M", "AUTO", 1), ((13, 9, 9), "M", "FUSED", 3),
+    ((20, 17, 23), "M", "FUSED", 5)])
+def test_a_wait_that_runs_out(gpu_lib, tmp_path, dims, prec, kern, n):
+    """The last block is left out of the grid, so that the others wait for sums
+    nobody sends until their limit of two seconds, then leave: the step reports
+    the timeout, and the next solves, on this scene and others, are as ever."""
+    coop_calls.run(tmp_path, SCENE, f"""
+    import time
+    from mfem_gb300._lib import MfemError
+    gpu.set_tuning(0)
+    def make():
+        s = [scene({dims}, {prec}, abi.PCG_KERNEL_{kern}) for _ in range({n})]
+        return s, gpu.Batch(s)
+    def step(b):
+        return b.step_n(1) if {n} > 1 else b.step()
+    s, b = make()
+    snap = [x.snapshot() for x in s]
+    step(b)
+    assert any("k_cgr" in k for k in launched())
+    ref = [x.positions() for x in s]
+    lib.coop_drop(1)
+    t, u = make()
+    t0 = time.perf_counter()
+    try:
+        step(u)
+        assert False, "no timeout"
+    except MfemError as e:
+        assert e.status == abi.ERR_TIMEOUT, e.status
+    waited = time.perf_counter() - t0
+    assert 1.9 < waited < 20, waited
+    lib.coop_drop(0)
+    direct = {kern!r} == "PERSISTENT"  # (graphs keep the grid they were captured with)
+    for x, q in zip(t if direct else s, snap):
+        x.restore(q)
+    step(u if direct else b)
+    assert all(np.array_equal(x.positions(), r) for x, r in zip(t if direct else s, ref))
+    v, c = make()
+    step(c)
+    assert all(np.array_equal(x.positions(), r) for x, r in zip(v, ref))
     """)
