@@ -66,7 +66,7 @@ constexpr double kDsvdTol = 1e-4;  // dsvd.cpp:153
 __constant__ double kSym2[3] = {1, 1, 2};
 __constant__ double kSymInv2[3] = {1, 1, 0.5};
 
-enum { SC_RN2 = 0, SC_E = 1, SC_DEC = 2, SC_CG_IT = 3, SC_CG_RN2 = 4, SC_CG_B2 = 5, SC_COUNT = 8 };
+enum { SC_RN2 = 0, SC_E = 1, SC_DEC = 2, SC_CG_IT = 3, SC_CG_RN2 = 4, SC_CG_B2 = 5, SC_STATUS = 6, SC_COUNT = 8 };
 
 // Device pointers of one 2-D scene (kernel argument, by value).
 struct T2 {
@@ -1278,7 +1278,10 @@ __global__ void __launch_bounds__(kBlock) t2_esum(T2 d, double h2, int slot, int
   const double sp = block_sum(a, sh);
   const double sq = block_sum(b, sh);
   const double sm = block_sum(c, sh);
-  if (t == 0) d.scal[slot] = 0.5 * sm + h2 * sp - sq;
+  if (t == 0) {
+    d.scal[slot] = 0.5 * sm + h2 * sp - sq;
+    d.scal[SC_STATUS] = *d.status;  // what the PCG before it left
+  }
   if (with_dec) {
     double m = 0;
     for (int i = t; i < 2 * d.nf; i += kBlock) m = fmax(m, fabs(d.dx[i]));
@@ -1662,6 +1665,12 @@ int t2_step(mfem_tri2d& sc, mfem_step_stats* out) {
     launch(sc, MFEM_T2_K_LOCAL, [&] { t2_local<<<grid_of(sc.nt), kThreads, 0, sc.stream>>>(sc.d); });
     if (launch_status() != MFEM_OK) return MFEM_ERR_CUDA;
     if (t2_energy_at(sc, 0.0, 1, scal) != MFEM_OK) return MFEM_ERR_CUDA;
+    if (scal[SC_STATUS] == MFEM_ERR_TIMEOUT) {  // a wait of the PCG ran out: it has no solution
+      collect_events(sc);
+      st.status = MFEM_ERR_TIMEOUT;
+      if (out) *out = st;
+      return MFEM_ERR_TIMEOUT;
+    }
     const int iters = sc.nf > 0 ? int(scal[SC_CG_IT]) : 0;
     const double b2 = sc.nf > 0 ? scal[SC_CG_B2] : 0.0;
     if (sc.nf > 0 && iters >= sc.cg_iters && status == MFEM_OK) status = MFEM_ERR_CG_MAXITER;

@@ -104,15 +104,23 @@ def test_sheets(gpu_lib, tmp_path, nx, ny, kernel):
                                   body_force=(0.0, -9.8, 0.0), max_newton_iterations=10,
                                   max_linesearch_iterations=20, max_iterative_solver_iters=10000,
                                   iterative_solver_tolerance=1e-10))
-        st = [sc.step() for _ in range(2)]
+        st = [sc.step().status for _ in range(steps_)]
         x = sc.get_state()["x"]
-        n = sc.n_free
         sc.close()
-        return np.array(x), n, launched()
-    ref, n, names = steps()
-    assert any({kernel!r} in k for k in names), (n, names)
+        return np.array(x), st, launched()
+    steps_ = 2
+    ref, st, names = steps()
+    assert any({kernel!r} in k for k in names), names
+    # rows that nobody sends: the wait runs out, the next sheet is as ever
+    lib.coop_drop(1)
+    steps_ = 1
+    assert steps()[1] == [abi.ERR_TIMEOUT]
+    lib.coop_drop(0)
+    steps_ = 2
+    again, st, names = steps()
+    assert abi.ERR_TIMEOUT not in st and np.array_equal(again, ref)
     lib.coop_refuse(1)
-    got, n, names = steps()
+    got, st, names = steps()
     assert not names
     assert np.abs(got - ref).max() <= 1e-6, np.abs(got - ref).max()
     """)
@@ -160,4 +168,41 @@ def test_a_wait_that_runs_out(gpu_lib, tmp_path, dims, prec, kern, n):
     v, c = make()
     step(c)
     assert all(np.array_equal(x.positions(), r) for x, r in zip(v, ref))
+    """)
+
+
+def test_which_resident_kernel_runs(gpu_lib, tmp_path):
+    """The kernels behind the comparisons with the launches in
+    test_gpu_resident.py: that the resident ones ran, at each of their sizes."""
+    coop_calls.run(tmp_path, SCENE, """
+    gpu.set_tuning(0)
+    A, P, F = abi.PCG_KERNEL_AUTO, abi.PCG_KERNEL_PERSISTENT, abi.PCG_KERNEL_FUSED
+    block = dict(linear_solver=abi.SOLVER_GPU_PCG_BLOCK)
+    # (mangled template arguments: Lb = scaled or not, Li = threads)
+    for dims, prec, kern, kw, name in [
+            ((7, 5, 5), M, A, {}, "k_cgr_fusedILb1ELi256E"), ((7, 5, 5), M, A, block, "k_cgr_fusedILb0ELi256E"),
+            ((11, 3, 5), M, A, {}, "k_cgr_fusedILb1ELi512E"), ((13, 9, 9), M, A, {}, "k_cgr_splitILi256E"),
+            ((13, 9, 9), M, A, block, "k_cgr_splitILi256E"), ((60, 27, 25), M, A, {}, "k_cgr_splitILi512E"),
+            ((57, 32, 45), M, A, {}, "k_cgr_wideILb1E"), ((57, 32, 45), M, A, block, "k_cgr_wideILb0E"),
+            ((59, 60, 61), M, A, {}, "k_cgr_wideILb1E"), ((2, 3, 3), M, P, {}, "k_cgr_splitILi256E"),
+            ((7, 5, 5), D, A, {}, "k_cgr_split64"), ((19, 15, 15), D, P, {}, "k_cgr_split64"),
+            ((26, 26, 24), D, P, {}, "k_cgr_split64")]:
+        s = scene(dims, prec, kern, **kw)
+        launched()
+        s.step(raise_on_error=False)
+        names = launched()
+        assert names and all(name in k for k in names), (dims, kern, kw, names)
+        assert gpu.kernel_stats(s.solo_batch_handle())["k_cg_solve"][1] > 0
+        s.close()
+    # the batch of 18 scenes on more than two tiles an SM, and lanes of small ones
+    s = [scene(d, M, F) for d in [(20, 20, 20)] * 10 + [(7, 5, 5), (13, 9, 9), (4, 2, 2), (16, 21, 23)] * 2]
+    b = gpu.Batch(s)
+    b.step_n(1)
+    assert all("k_cgr_wide" in k for k in launched()) and gpu.kernel_stats(b.handle)["k_cg_solve"][1] > 0
+    b.close()
+    lanes = gpu.Lanes(s[10:], lanes=3)
+    lanes.step_n(1)
+    assert {"k_cgr_fused" in k for k in launched()} == {True}
+    assert all(gpu.kernel_stats(x.handle)["k_cg_solve"][1] > 0 for x in lanes.batches)
+    lanes.close()
     """)
