@@ -82,9 +82,10 @@ struct CgrShared {
 // one or two tiles, a scene of one block nothing.  `ahead` runs once the
 // other blocks' sums have come in, before the last of the adding: loads issued
 // there are under way meanwhile; `during` before, while the sums travel.
-// False: a wait ran out; of up to 32 records for the warps whose wait it was,
+// kLead: only the first warp wants the sums (the others have them of more than
+// 32 records).  False: a wait ran out; of up to 32 records for the warps whose wait it was,
 // of more for the whole block.
-template <typename E, int NQ, typename F, typename G>
+template <typename E, int NQ, bool kLead = false, typename F, typename G>
 __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B, CgrShared& S, bool lead, int sl,
                                             unsigned seq, E (&v)[NQ], const F& ahead, const G& during) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -103,6 +104,7 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
     for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.part[par][q][sl], v[q]);
   __syncthreads();
   const int nt = (B.nsl + kCgrTile - 1) / kCgrTile;  // 1 or 2
+  if (B.nblk == 1 && kLead && warp > 0) return true;
   if (B.nblk == 1) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) v[q] = lane < B.nsl ? Slot<E>::sget(&S.part[par][q][lane]) : E(0);
@@ -141,6 +143,10 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
   };
   if (n <= 32) {
     // every warp for itself, no block barrier
+    if (kLead && warp > 0) {
+      ahead();
+      return true;
+    }
     E a[NQ];
     if (!fetch(lane, a)) return false;
     ahead();
@@ -390,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) d1[0] = acc_prod(d1[0], p[c], acc[c]);
     }
-    if (!scene_total<E, 1>(A, B, S, roww, sl, seq, d1, nothing, [&]() { rz_rcp = rcp_of(rz); })) {
+    if (!scene_total<E, 1>(A, B, S, roww, sl, seq, d1, nothing, [&]() { rz_rcp = E(1.f) / rz; })) {
       cgr_abort(A, B);
       return;
     }
@@ -428,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
     if (cg_meets(sd, thr, rr, rr0)) {
       stop = true;
     } else {
-      betaE = by_rcp(d2[1], rz, rz_rcp);
+      betaE = by_rcp_step(d2[1], rz, rz_rcp);
       rz_prev = rz;
       rz = d2[1];
       it = it + 1;
@@ -490,7 +496,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
         it = it - 1;  // as in Eigen, the iteration that meets the threshold is not counted
         break;
       }
-      betaE = by_rcp(d3[1], rz_prev, rz_rcp);
+      betaE = by_rcp_step(d3[1], rz_prev, rz_rcp);
       rz = d3[1];
     }
     beta = to_step(betaE);
@@ -835,7 +841,8 @@ __global__ void __launch_bounds__(kThreads64, 1) k_cgr_split64(const CgrArgs A) 
 // the next launches of k_cgf_iter verify), or max_iters iterations.  The
 // exchanged vector is w; each block keeps r and s at its halo.
 struct CgfScalars {
-  df64 gamma, alphaE, betaE, rr0, rr, rg, ra;
+  df64 gamma, alphaE, betaE, rr0, rr;
+  df_rcp rg, ra;  // of gamma and alphaE
   float2 thr;
   float a, b;
   int it, rounds, phase, status, cg_status;
@@ -852,6 +859,24 @@ struct CgfScalars {
   }
   // After an iteration's sums, as cgf_verify_step in phase 0: whether the launch ends.
   __device__ __forceinline__ bool step(const SceneDev& sd, const df64 (&d)[3]) {
+    return advance(sd, d, [&](df64 g, df64* b, df64* ga) {
+      *b = by_rcp(g, gamma, rg);
+      *ga = by_rcp(g, alphaE, ra);
+    });
+  }
+  // The same by a whole warp, whose even lanes take the quotients by gamma and
+  // whose odd ones those by alpha, in the time of one.
+  __device__ __forceinline__ df64 den() const { return threadIdx.x & 1 ? alphaE : gamma; }
+  __device__ __forceinline__ void prepare_warp() { rg = rcp_of(den()); }
+  __device__ __forceinline__ bool step_warp(const SceneDev& sd, const df64 (&d)[3]) {
+    return advance(sd, d, [&](df64 g, df64* b, df64* ga) {
+      const df64 v = by_rcp(g, den(), rg);
+      *b = shfl_to(v, 0);
+      *ga = shfl_to(v, 1);
+    });
+  }
+  template <typename F>
+  __device__ __forceinline__ bool advance(const SceneDev& sd, const df64 (&d)[3], const F& quotients) {
     rr = d[0];
     if (is_nan(rr)) {
       status = 4;
@@ -863,7 +888,9 @@ struct CgfScalars {
       swapped = true;
       return true;
     }
-    cgf_steps(d[1], d[2], gamma, alphaE, rg, ra, &alphaE, &betaE);
+    df64 ga;
+    quotients(d[1], &betaE, &ga);
+    alphaE = cgf_alpha(d[1], d[2], betaE, ga);
     gamma = d[1];
     a = to_step(alphaE);
     b = to_step(betaE);
@@ -875,6 +902,8 @@ struct CgfScalars {
     }
     return false;
   }
+  // the last iteration done
+  __device__ __forceinline__ int last() const { return swapped ? it : it - 1; }
   __device__ __forceinline__ void store(SceneScalars* sc) const {
     sc->cg_err = cg_rel(rr, rr0);
     sc_put(&sc->beta, betaE);
@@ -893,25 +922,19 @@ template <bool kScaled, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
   extern __shared__ __align__(16) unsigned char cgr_smem_raw[];
   __shared__ CgrShared S;
-  // The scalars, some 400 instructions an iteration: with 16 warps they are
-  // thread 0's, with a barrier more (two steps of 350 rows: 3.10 ms, against
-  // 3.24 ms with every warp for itself), with 8 every warp's own (three steps
-  // of 16 scenes: 26.4 ms against 26.9)
-  constexpr bool kOne = kThreads > 256;
-  __shared__ __align__(8) unsigned char q_raw[sizeof(CgfScalars)];
-  __shared__ int leave;
+  // The sums and the scalars, some 800 instructions an iteration, are warp 0's;
+  // the others wait for the halo meanwhile.  (Every warp for itself: three
+  // steps of 16 scenes in blocks of two tiles 27.0 ms, against 19.7, of six
+  // scenes in blocks of one 14.4 against 13.8.)
+  __shared__ float steps[2];  // warp 0's alpha and beta for the others
+  __shared__ int leave, done;
   const CgrBlock B = A.blocks[blockIdx.x];
   const SceneDev& sd = A.sds[B.scene];
   SceneScalars* sc = sd.sc;
   if (!sc->cg_active || sc->cgf_phase) return;
   unsigned seq = __ldcg(A.seq + B.scene);
   const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
-  CgfScalars q_own(sc);
-  CgfScalars& q = kOne ? *reinterpret_cast<CgfScalars*>(q_raw) : q_own;
-  if (kOne) {
-    if (threadIdx.x == 0) new (&q) CgfScalars(sc);
-    __syncthreads();
-  }
+  CgfScalars q(sc);
   const bool roww = sl < B.nsl;
   const int row = 32 * (B.slice0 + sl) + lane;
   const bool live = roww && row < sd.nf;
@@ -1054,31 +1077,36 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
         }
       }
     }
-    const bool got = scene_total<df64, 3>(A, B, S, roww, sl, seq, d, [&]() {
+    bool got = scene_total<df64, 3, true>(A, B, S, roww, sl, seq, d, [&]() {
 #pragma unroll
           for (int j = 0; j < kHaloRegs; ++j)
             if (hw[j]) hv[j] = ld_rec(A.pub + (size_t)(seq & 1) * A.pub_stride + B.row0 + hc[j]);
-        }, [&]() { if (!kOne || threadIdx.x == 0) q.prepare(); });
+        }, [&]() { if (sl == 0) q.prepare_warp(); });
     wtag = seq;
     ++seq;
-    if (kOne) {
-      // (thread 0's step ends the loop for all: no warp goes on without it)
-      if (got && threadIdx.x == 0) leave = q.step(sd, d) || n + 1 >= A.max_iters;
-      if (!__syncthreads_and(got)) {
-        cgr_abort(A, B);
-        return;
+    if (sl > 0)
+      got = poll_recs<kHaloRegs>(hv, [&](int j) { return A.pub + (size_t)(wtag & 1) * A.pub_stride + B.row0 + hc[j]; },
+                                 hw, wtag, &A.ctrs->error) && got;
+    if (got && sl == 0) {
+      const bool stop = q.step_warp(sd, d) || n + 1 >= A.max_iters;
+      if (lane == 0) {
+        leave = stop;
+        done = q.last();
+        steps[0] = q.a;
+        steps[1] = q.b;
       }
-      if (leave) break;
-    } else {
-      if (!got) {
-        cgr_abort(A, B);
-        return;
-      }
-      if (q.step(sd, d) || n + 1 >= A.max_iters) break;
     }
+    // (no warp goes on without warp 0, whose step ends the loop)
+    if (!__syncthreads_and(got)) {
+      cgr_abort(A, B);
+      return;
+    }
+    if (leave) break;
+    q.a = steps[0];
+    q.b = steps[1];
   }
+  const int last = done;
   // ---- the vectors as k_cgf_iter leaves them after iteration `last`
-  const int last = q.swapped ? q.it : q.it - 1;
   if (live) {
     st3(static_cast<float*>(sd.cgf_r[(last + 1) & 1]) + k4, r);
     st3(static_cast<float*>(sd.cgf_w[(last + 1) & 1]) + k4, w);
@@ -1481,7 +1509,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_cgr_wide(const CgrArgs A) {
   }
   drain();
   // ---- the vectors as k_cgf_iter leaves them after iteration `last`
-  const int last = q.swapped ? q.it : q.it - 1;
+  const int last = q.last();
 #pragma unroll
   for (int j = 0; j < kWideSlices; ++j)
     if (live[j]) {

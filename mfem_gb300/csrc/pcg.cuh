@@ -234,8 +234,6 @@ __device__ __forceinline__ bool is_nan(df64 v) { return v.hi != v.hi; }
 __device__ __forceinline__ bool is_nan(double v) { return v != v; }
 __device__ __forceinline__ bool is_zero(df64 v) { return v.hi == 0.f; }
 __device__ __forceinline__ bool is_zero(double v) { return v == 0.0; }
-// A step length as every thread uses it.
-__device__ __forceinline__ float to_step(df64 v) { return __fadd_rn(v.hi, v.lo); }
 __device__ __forceinline__ double to_step(double v) { return v; }
 
 // The stopping test |r|^2 < max(tol^2 |b|^2, DBL_MIN).  The mixed path forms

@@ -74,6 +74,16 @@ int main() {
     beta.add(q(bn), -q(su) / q(ps));
   }
   beta.put();
+  // step lengths: the same float as the quotient, also beside the middle of two
+  long differ = 0;
+  for (int i = 0; i < 400000; ++i) {
+    const df64 d = draw();
+    const float f = draw().hi, up = std::nextafterf(f, 2 * f);
+    const double mid = 0.5 * ((double)f + up) * (1 + (i % 41 - 20) * std::exp2(-47 + i % 7));
+    const df64 n = i % 2 ? df64(mid) * d : draw();
+    differ += to_step(by_rcp_step(n, d, df64(1.f) / d)) != to_step(by_rcp(n, d, rcp_of(d)));
+  }
+  std::printf("%ld 0\n", differ);
   // dens whose reciprocal leaves FP32's range are divided by
   for (double den : {1e-38, 1e-31, 1e31, 1e38}) {
     const df64 d(den), n = df64(3.0) * d;
@@ -96,5 +106,6 @@ def test_scalar_errors_are_those_of_fp64_products_between_divisions(tmp_path):
     for ref, now in zip(rows[0:10:2], rows[1:10:2]):
         assert now[0] <= ref[0] and now[1] <= ref[1], (ref, now)
     assert rows[10][0] <= 2.0 ** -46.5
+    assert rows[11][0] == 0
     # (near the ends of the range the low parts are subnormal: FP32's accuracy)
-    assert all(r[0] <= 2.0 ** -23 for r in rows[11:])
+    assert all(r[0] <= 2.0 ** -23 for r in rows[12:])
