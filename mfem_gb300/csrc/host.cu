@@ -1438,8 +1438,10 @@ int run_pcg(mfem_batch* b, const Launch& Lcg) {
     }
   }
   // the whole solve in one launch where the batch fits.  With profiling on,
-  // a batch that chose its form itself runs that form's launches instead
-  // (the same results), so that every kernel carries its own event pair.
+  // a batch that chose the two-reduction form itself runs that form's launches
+  // instead (the same results), so that every kernel carries its own event
+  // pair; one that chose the single-reduction form what its loop runs, a
+  // launch at a time.
   if ((b->pcg_kernel == MFEM_PCG_KERNEL_PERSISTENT ||
        (b->pcg_kernel == MFEM_PCG_KERNEL_SPLIT && b->auto_form && !b->profiling && pcg_mode(b) == kPcgAlone)) &&
       cgr_plan(b)) {
@@ -1454,6 +1456,24 @@ int run_pcg(mfem_batch* b, const Launch& Lcg) {
     { KTimer t(b, MFEM_K_CG_SOLVE); e = launch_cg_solve(Lcg, b->coop_grid, b->max_cg + 1); }
     CUDA_OR(e, MFEM_ERR_CUDA);
     return MFEM_OK;
+  }
+  if (b->profiling && fused && b->auto_form && pcg_mode(b) == kPcgAlone && cgr_plan(b)) {
+    for (int k = 0; k < (b->max_cg + 11) / 3 + 1; ++k) {  // as capture_cg_loop's bodies
+      cudaError_t e;
+      { KTimer t(b, MFEM_K_CG_SOLVE); e = cgr_launch(b, 1 << 30); }
+      if (e != cudaSuccess) {
+        b->k_launches[MFEM_K_CG_SOLVE] -= 1;
+        cgr_refused(b);
+        break;
+      }
+      for (int j = 0; j < 3; ++j) {
+        KTimer t(b, MFEM_K_CGF_ITER);
+        launch_cgf_iter(Lcg, b->cgf_shape);
+      }
+      const int rc = sync_counters(b);
+      if (rc) return rc;
+      if (b->h_ctr->cg_active == 0) return MFEM_OK;
+    }
   }
   // Chunks of iterations with the convergence check one chunk behind: after
   // each chunk the counters are copied to a pinned slot and an event is
