@@ -1132,6 +1132,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
 // takes 20 bytes of shared memory a column, and the iteration waits twice, for
 // the neighbours' rows and for the sums.
 //
+// (A later build, by events: 16.6 us at 85k rows, 26.4 at 223k.)
 // An iteration at 85k / 130k / 148k / 223k rows: 17.9 / 21.3 / 21.6 / 32.0 us,
 // against 25.4 / 28.1 / 30.2 / 37.9 us in launches (block Jacobi: 18.3 / 21.9 /
 // 22.3 / 33.7 against 32.3 / 35.3 / 37.0 / 50.9).  Of the 62,000 cycles at 223k

@@ -451,11 +451,12 @@ __global__ void __launch_bounds__(kBlock) t2_norm(T2 d) {
 }
 
 // ----------------------------------------------------- grid PCG ---
-// The Jacobi-PCG of sheets that t2_pcg_res does not fit.  One cooperative
-// launch of G blocks of kGridThreads, each owning a contiguous range of free rows; a reduction is each block's
-// fixed-order partial, a bounded grid barrier, and the G partials summed in
-// the same fixed order by every block (so every block takes the same
-// branches).  The iteration is the single-reduction form of the same PCG
+// The Jacobi-PCG of sheets that t2_pcg_res does not fit, and, with one block
+// launched plainly, of any sheet whose cooperative launch the runtime refuses.
+// G blocks of kGridThreads, each owning a contiguous range of free rows; a
+// reduction is each block's fixed-order partial, a bounded grid barrier, and
+// the G partials summed in the same fixed order by every block (so every block
+// takes the same branches).  The iteration is the single-reduction form of the same PCG
 // (Chronopoulos & Gear 1989; equal to Eigen's iteration in exact
 // arithmetic): with u = D^-1 r, w = A u, s = A p, each iteration needs one
 // reduction of (r, u), (w, u) and |r|^2 -- one grid barrier.  A
