@@ -1272,6 +1272,7 @@ __global__ void __launch_bounds__(kThreads) t2_energy(T2 d, double alpha) {
 __global__ void __launch_bounds__(kBlock) t2_esum(T2 d, double h2, int slot, int with_dec) {
   __shared__ double sh[kBlock];
   const int t = threadIdx.x;
+  const int status = with_dec && t == 0 ? *d.status : 0;  // what the PCG before it left
   double a = 0, b = 0, c = 0;
   for (int i = t; i < d.nt; i += kBlock) a += d.epart[i];
   for (int i = t; i < d.nt; i += kBlock) b += d.epart[d.nt + i];
@@ -1279,16 +1280,16 @@ __global__ void __launch_bounds__(kBlock) t2_esum(T2 d, double h2, int slot, int
   const double sp = block_sum(a, sh);
   const double sq = block_sum(b, sh);
   const double sm = block_sum(c, sh);
-  if (t == 0) {
-    d.scal[slot] = 0.5 * sm + h2 * sp - sq;
-    d.scal[SC_STATUS] = *d.status;  // what the PCG before it left
-  }
+  if (t == 0) d.scal[slot] = 0.5 * sm + h2 * sp - sq;
   if (with_dec) {
     double m = 0;
     for (int i = t; i < 2 * d.nf; i += kBlock) m = fmax(m, fabs(d.dx[i]));
     for (int i = t; i < 3 * d.nt; i += kBlock) m = fmax(m, fabs(d.ds[i]));
     const double mx = block_max(m, sh);
-    if (t == 0) d.scal[SC_DEC] = mx;
+    if (t == 0) {
+      d.scal[SC_DEC] = mx;
+      d.scal[SC_STATUS] = status;
+    }
   }
 }
 
