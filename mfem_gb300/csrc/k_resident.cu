@@ -71,6 +71,7 @@ __device__ __forceinline__ void tree(E (&v)[NQ]) {
 struct CgrShared {
   double part[2][3][kCgrMaxSlices];  // the block's slice sums
   double red[2][3][8];               // warp sums of the tiles
+  int late;                          // a wait of scene_total ran out (cleared by the kernel)
 };
 
 // Sums over the scene's rows, the same in every thread of every block.  v
@@ -166,20 +167,26 @@ __device__ __forceinline__ bool scene_total(const CgrArgs& A, const CgrBlock& B,
 #pragma unroll
       for (int q = 0; q < NQ; ++q) s[q] = radd(s[q], a[q]);
     }
+    // (the warps wait for different records: a wait that ran out shows in the
+    // sums, so that all warps leave or none; __syncthreads_and took 1% of a step)
+    if (!ok) {
+      S.late = 1;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) s[q] = E(__int_as_float(0x7fffffff));
+    }
     tree<E, NQ, 16>(s);
     if (lane == 0)
 #pragma unroll
       for (int q = 0; q < NQ; ++q) Slot<E>::put(&S.red[par][q][warp], s[q]);
   }
-  // (the warps wait for different records: all of them leave or none)
-  if (!__syncthreads_and(ok)) return false;
+  __syncthreads();
   ahead();
 #pragma unroll
   for (int q = 0; q < NQ; ++q) v[q] = lane < 8 ? Slot<E>::sget(&S.red[par][q][lane]) : E(0);
   tree<E, NQ, 4>(v);
 #pragma unroll
   for (int q = 0; q < NQ; ++q) v[q] = shfl_to(v[q], 0);
-  return true;
+  return !(is_nan(v[0]) && S.late);
 }
 
 // The block's slices in shared memory: nine planes (row-major 3x3 entries) of
@@ -284,6 +291,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_split(const CgrArgs A) {
   if (!sc->cg_active) return;
   unsigned seq = __ldcg(A.seq + B.scene);
   const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+  if (threadIdx.x == 0) S.late = 0;
   const bool roww = sl < B.nsl;
   const int row = 32 * (B.slice0 + sl) + lane;
   const bool live = roww && row < sd.nf;
@@ -934,6 +942,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cgr_fused(const CgrArgs A) {
   if (!sc->cg_active || sc->cgf_phase) return;
   unsigned seq = __ldcg(A.seq + B.scene);
   const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+  if (threadIdx.x == 0) S.late = 0;
   CgfScalars q(sc);
   const bool roww = sl < B.nsl;
   const int row = 32 * (B.slice0 + sl) + lane;
