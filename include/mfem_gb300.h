@@ -183,7 +183,8 @@ int mfem_gpu_scene_create(const mfem_scene_desc* desc, mfem_scene** out);
 int mfem_gpu_scene_destroy(mfem_scene* scene);
 /* One timestep: NewtonOptimizer<3>::step, src/optimizers/newton_optimizer.cpp:11-89. */
 int mfem_gpu_scene_step(mfem_scene* scene, mfem_step_stats* stats);
-/* Bytes of device memory the scene holds (admission control). */
+/* Bytes of device memory the scene holds at most, its single-scene batch and
+ * the resident solve's plan included (admission control). */
 int mfem_gpu_scene_footprint(const mfem_scene_desc* desc, int64_t* bytes);
 int mfem_gpu_scene_sizes(const mfem_scene* scene, int32_t* n_vertices,
                          int32_t* n_tets, int32_t* n_free);
